@@ -900,7 +900,7 @@ extern "C" int lda_max_topic(lda_trainer* t) {
             dev::StatsArgs as = a;
             as.recip = t->recip;
             as.order = t->order;
-            dev::k_sparse_order<<<1, 256, 0, t->stream>>>(as, t->order);
+            dev::k_sparse_order<<<(t->K + 31) / 32, 256, 0, t->stream>>>(as, t->order);
             CUDA_TRY(cudaGetLastError());
             const int64_t ns = a.V - std::max(t->Vd, a.wlo);
             const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(t->grid_stats_sparse, (ns + kLargeWarps - 1) / kLargeWarps));
