@@ -38,9 +38,23 @@ constexpr int kTilesPerWarp = LDA_TILES_PER_WARP;
 #ifndef LDA_DENSE_TILE
 #define LDA_DENSE_TILE 8192
 #endif
-constexpr int kDenseTileLarge = LDA_DENSE_TILE;  // dense-word tiles above kLargeK topics (one CTA per tile)
+constexpr int kDenseTileLarge = LDA_DENSE_TILE;  // most tokens per dense-word tile above kLargeK topics (one CTA per tile)
+#ifndef LDA_DENSE_TILE_MIN
+#define LDA_DENSE_TILE_MIN 512
+#endif
+constexpr int kDenseTileLargeMin = LDA_DENSE_TILE_MIN;
+#ifndef LDA_DENSE_TILES_PER_CTA
+#define LDA_DENSE_TILES_PER_CTA 4
+#endif
 constexpr int kLargeWarps = 8;                // warps per CTA of the large-K sampler kernels
-constexpr int kWtTile = 16384;     // tokens per dense word-topic tile
+// Tokens per dense word-topic tile: the corpus' tokens over twice the warps that fill the
+// GPU, within these bounds.  The upper one alone (16,384) left the rebuild waiting for the
+// one warp that walks the most frequent word's tile, 128 tokens per round of loads.
+constexpr int kWtTileMax = 16384;
+#ifndef LDA_WT_TILE_MIN
+#define LDA_WT_TILE_MIN 2048
+#endif
+constexpr int kWtTileMin = LDA_WT_TILE_MIN;
 constexpr int kCounters = 16;
 
 struct EventPair {
@@ -402,7 +416,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     }
     T.smem_stats = (size_t)(T.warps + 1) * row;
     // the rebuilds' warp-private histograms hold 16-bit counts, two per word: a dense
-    // word-topic tile has kWtTile tokens, a sparse word fewer than 65,536 and a doc at most
+    // word-topic tile has at most kWtTileMax tokens, a sparse word fewer than 65,536 and a doc at most
     // 65,535 (the corpus layout's limit), so every count fits.  Each rebuild takes as many
     // warps per CTA (up to 8) as its shared memory allows.
     const size_t bitw = (size_t)(T.K + 31) / 32;
@@ -442,7 +456,13 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     // sparse-word tiles, each largest first).  For K <= kLargeK a chunk's tile size is
     // its tokens / (kTilesPerWarp x the sampler's resident warps), rounded up to 32 and
     // kept within [kSampleTileMin, kSampleTile].
-    int64_t resident_warps = 0;
+    int64_t resident_warps = 0, resident_dense = 0;
+    if (T.large) {
+        CUDA_TRY(raise_smem_limit(dense_large_kernel(false), T.smem_dense));
+        int g = 0, orc = occupancy_grid(dense_large_kernel(false), 32 * kLargeWarps, T.smem_dense, T.num_sms, &g);
+        if (orc) return orc;
+        resident_dense = g;
+    }
     if (!T.large) {
         CUDA_TRY(raise_smem_limit(sample_kernel(false, T.K), T.smem_sample));
         int g = 0, orc = occupancy_grid(sample_kernel(false, T.K), 32 * T.swarps, T.smem_sample, T.num_sms, &g);
@@ -455,7 +475,17 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     auto by_size = [](const int4& a, const int4& b) { return a.z > b.z; };
     for (int ch = 0; ch < T.C; ++ch) {
         std::vector<int4> ct, cs;
-        int64_t tile_ch = kSampleTile;
+        int64_t tile_ch = kSampleTile, tile_dense = kDenseTileLarge;
+        if (T.large) {
+            // dense-word tiles: the chunk's dense tokens over kDenseTilesPerCta tiles per
+            // resident CTA.  A chunk of a smaller corpus would otherwise wait for the one
+            // CTA that holds the most frequent word's 8,192 tokens.
+            int64_t nd = 0;
+            for (int64_t w = 0; w < T.Vd; ++w) nd += c->seg_cnt[(size_t)ch * V + w];
+            const int64_t per = LDA_DENSE_TILES_PER_CTA * std::max<int64_t>(resident_dense, 1);
+            tile_dense = std::min<int64_t>(kDenseTileLarge,
+                                           std::max<int64_t>(kDenseTileLargeMin, ((nd + per - 1) / per + 255) / 256 * 256));
+        }
         if (!T.large) {
             const int64_t per = kTilesPerWarp * std::max<int64_t>(resident_warps, 1);
             const int64_t want = ((T.chunk_tok[ch + 1] - T.chunk_tok[ch] + per - 1) / per + 31) / 32 * 32;
@@ -464,7 +494,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
         for (int64_t w = 0; w < V; ++w) {
             const int64_t n = c->seg_cnt[(size_t)ch * V + w], o = c->seg_off[(size_t)ch * V + w];
             const bool dense = w < T.Vd;
-            const int64_t tile = T.large && dense ? kDenseTileLarge : tile_ch;
+            const int64_t tile = T.large && dense ? tile_dense : tile_ch;
             for (int64_t p = 0; p < n; p += tile) {
                 const int4 v = make_int4((int)w, (int)(o + p), (int)std::min<int64_t>(tile, n - p), dense);
                 (T.large && !dense ? cs : ct).push_back(v);
@@ -478,13 +508,15 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
         T.s_tile_base[ch + 1] = (int)st.size();
     }
     // word-topic tiles: dense segments of every chunk, and one tile per sparse word
+    const int64_t wt_tile = std::min<int64_t>(
+        kWtTileMax, std::max<int64_t>(kWtTileMin, (N / (2 * 64 * (int64_t)T.num_sms) + 127) / 128 * 128));
     std::vector<int4> wt;
     for (int64_t w = 0; w < V; ++w) {
         if (w < T.Vd) {
             for (int ch = 0; ch < T.C; ++ch) {
                 const int64_t n = c->seg_cnt[(size_t)ch * V + w], o = c->seg_off[(size_t)ch * V + w];
-                for (int64_t p = 0; p < n; p += kWtTile)
-                    wt.push_back(make_int4((int)w, (int)(o + p), (int)std::min<int64_t>(kWtTile, n - p), 1));
+                for (int64_t p = 0; p < n; p += wt_tile)
+                    wt.push_back(make_int4((int)w, (int)(o + p), (int)std::min<int64_t>(wt_tile, n - p), 1));
             }
         } else if (c->word_count[w] > 0) {
             wt.push_back(make_int4((int)w, 0, (int)c->word_count[w], 0));
