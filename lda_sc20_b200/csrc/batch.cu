@@ -42,8 +42,9 @@ struct BatchArgs {
     const uint2* sm_work;  // {model, sampler tile}
     int n_sm;
     unsigned* counters;    // [4] work counters of the stages, zeroed at the start of a sweep
-    const uint32_t* sweeps_done;  // sweeps this batch has run, added to each model's base iteration
+    const uint32_t* sweeps_done;  // sweeps this batch has begun: with a model's base iteration, its iteration
     int Kmax;
+    int nslots;            // row slots per warp of the sampler
 };
 
 __device__ __forceinline__ int grab(unsigned* counter, int lane) {
@@ -79,29 +80,29 @@ __global__ void __launch_bounds__(256) kb_wt(BatchArgs b) {
     }
 }
 
-// 1 / ((float)n_k + V*beta) of one model into a warp-private table.
-__device__ __forceinline__ void warp_recip(float* r, const int* n_k, int K, float Vbeta, int lane) {
-    __syncwarp();
-    for (int k = lane; k < K; k += 32) r[k] = __fdiv_rn(1.0f, fadd(__int2float_rn(n_k[k]), Vbeta));
-    __syncwarp();
+// Every model's reciprocals r_k = 1 / ((float)n_k + V*beta) and beta * r_k in the sampler's
+// column layout: block per model.  (The statistics and the sampler each formed them per
+// warp whenever the warp's next item was another model's.)  Also counts the sweep.
+__global__ void __launch_bounds__(256) kb_recip(const StatsArgs* st, uint32_t* sweeps_done) {
+    const StatsArgs& a = st[blockIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *sweeps_done += 1u;
+    for (int k = threadIdx.x; k < a.K; k += blockDim.x) {
+        const float r = __fdiv_rn(1.0f, fadd(__int2float_rn(a.n_k[k]), a.Vbeta));
+        a.recip_out[k] = r;
+        a.base_out[col_skew(k)] = fmul(a.beta, r);
+    }
 }
 
 __global__ void __launch_bounds__(256) kb_stats(BatchArgs b) {
     extern __shared__ float smf[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* r = smf + (size_t)b.Kmax * 2 * wid;
-    float* col = r + b.Kmax;
-    int cur = -1;
+    float* col = smf + (size_t)b.Kmax * wid;
     for (;;) {
         const int i = grab(b.counters + 1, lane);
         if (i >= b.n_st) break;
         const uint4 u = b.st_work[i];
         const StatsArgs& a = b.st[u.x];
-        if ((int)u.x != cur) {
-            cur = (int)u.x;
-            warp_recip(r, a.n_k, a.K, a.Vbeta, lane);
-        }
-        for (uint32_t w = u.y; w < u.y + u.z; ++w) word_stats_word(a, (int)w, r, col, lane);
+        for (uint32_t w = u.y; w < u.y + u.z; ++w) word_stats_word(a, (int)w, a.recip, col, lane);
     }
 }
 
@@ -123,21 +124,22 @@ __global__ void __launch_bounds__(256) kb_dt(BatchArgs b) {
 }
 
 template <bool LL, int QB>
-__global__ void __launch_bounds__(256) kb_sample(BatchArgs b) {
+__global__ void __launch_bounds__(256, 3) kb_sample(BatchArgs b) {
     extern __shared__ float smf[];
-    const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int per = b.Kmax + col_words(b.Kmax);
-    float* r = smf + (size_t)per * wid;
-    float* col = r + b.Kmax;
-    uint32_t* ctr = reinterpret_cast<uint32_t*>(smf + (size_t)per * warps) + C_NUM * wid;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* col = smf + (size_t)sample_warp_words(b.Kmax, b.nslots) * wid;
+    float* slots = col + col_words(b.Kmax);
+    uint32_t* ctr = reinterpret_cast<uint32_t*>(slots + ((row_state_words(b.nslots) + 3) & ~3));
     if (lane < C_NUM) ctr[lane] = 0u;
     __syncwarp();
-    const uint32_t done = *b.sweeps_done;
+    const uint32_t done = *b.sweeps_done - 1u;  // sweeps before this one
     int cur = -1;
+    bool clean = false;
     const SampleArgs* ca = nullptr;
-    for (;;) {
-        const int i = grab(b.counters + 3, lane);
-        if (i >= b.n_sm) break;
+    int i = grab(b.counters + 3, lane);
+    while (i < b.n_sm) {
+        int next = 0;
+        if (lane == 0) next = (int)atomicAdd(b.counters + 3, 1u);
         const uint2 w = b.sm_work[i];
         if ((int)w.x != cur) {
             __syncwarp();
@@ -146,10 +148,11 @@ __global__ void __launch_bounds__(256) kb_sample(BatchArgs b) {
             if (lane < C_NUM) ctr[lane] = 0u;
             cur = (int)w.x;
             ca = b.sm + cur;
-            warp_recip(r, ca->n_k, ca->K, ca->Vbeta, lane);
+            clean = false;
         }
         const SampleArgs& a = *ca;
-        sample_tile<LL, QB>(a, (int)w.y, a.tiles[w.y], a.iter + done, r, col, ctr, lane);
+        sample_tile<LL, QB>(a, (int)w.y, a.tiles[w.y], a.iter + done, col, slots, clean, ctr, lane);
+        i = __shfl_sync(FULL, next, 0);
     }
     __syncwarp();
     if (ca && lane < C_NUM && ctr[lane]) atomicAdd(ca->ctr + lane, (unsigned long long)ctr[lane]);
@@ -169,8 +172,6 @@ __global__ void __launch_bounds__(1024) kb_ll(const SampleArgs* sm, double* out)
     }
     if (threadIdx.x == 0) out[blockIdx.x] = s[0];
 }
-
-__global__ void kb_advance(uint32_t* sweeps_done) { *sweeps_done += 1u; }
 
 // ORs the models' device error flags into one and clears them.
 __global__ void kb_errors(int* const* errs, int n, int* out) {
@@ -245,6 +246,7 @@ struct lda_batch {
     uint32_t host_sweeps = 0;
     // launch shapes
     size_t smem_hist = 0, smem_stats = 0, smem_sample = 0, smem_dt = 0;
+    int nslots = 1;
     int grid_wt = 0, grid_stats = 0, grid_dt = 0, grid_sample = 0, grid_sample_ll = 0;
     // cached graph of (sweeps, ll)
     cudaGraphExec_t graph = nullptr;
@@ -286,6 +288,7 @@ static int batch_build(lda_batch* b) {
     std::vector<dev::StatsArgs> stt(M);
     std::vector<dev::DtArgs> dt(M);
     std::vector<dev::SampleArgs> sm(M);
+    const int nslots = b->Kmax <= 512 ? 32 : 16;
     std::vector<dev::ZeroSeg> zero;
     std::vector<int*> errs;
     std::vector<int4> sub;
@@ -306,11 +309,15 @@ static int batch_build(lda_batch* b) {
         const TrainerView& v = b->views[m];
         wt[m] = v.wt;
         stt[m] = v.st;
+        stt[m].recip = v.sm.recip;
+        stt[m].recip_out = const_cast<float*>(v.sm.recip);
+        stt[m].base_out = const_cast<float*>(v.sm.base);
         dt[m] = v.dt;
         sm[m] = v.sm;
         sm[m].tiles = b->sub_tiles.p + sub_base[m];
         sm[m].ntiles = (int)(sub_base[m + 1] - sub_base[m]);
         sm[m].tile_ll = b->sub_ll.p + sub_base[m];
+        sm[m].nslots = nslots;
         zero.push_back({v.n_k, (long long)v.K});
         if (v.dwt_count > 0) zero.push_back({v.dwt, (long long)v.dwt_count});
         errs.push_back(v.wt.err);
@@ -352,8 +359,9 @@ static int batch_build(lda_batch* b) {
     // launch shapes
     const int threads = 32 * tu.warps;
     b->smem_hist = (size_t)tu.warps * (b->Kmax + (b->Kmax + 31) / 32) * 4;
-    b->smem_stats = (size_t)tu.warps * b->Kmax * 8;
-    b->smem_sample = (size_t)tu.warps * ((b->Kmax + dev::col_words(b->Kmax)) * 4 + dev::C_NUM * 4);
+    b->smem_stats = (size_t)tu.warps * b->Kmax * 4;
+    b->smem_sample = (size_t)tu.warps * dev::sample_warp_words(b->Kmax, nslots) * 4;
+    b->nslots = nslots;
     b->smem_dt = (size_t)tu.warps * (b->Kmax + (b->Kmax + 31) / 32) * 4;
     if ((rc = occupancy((const void*)dev::kb_wt, threads, b->smem_hist, b->num_sms, &b->grid_wt)) ||
         (rc = occupancy((const void*)dev::kb_stats, threads, b->smem_stats, b->num_sms, &b->grid_stats)) ||
@@ -379,6 +387,7 @@ static dev::BatchArgs batch_args(const lda_batch* b) {
     a.counters = b->counters;
     a.sweeps_done = b->sweeps_done;
     a.Kmax = b->Kmax;
+    a.nslots = b->nslots;
     return a;
 }
 
@@ -395,6 +404,7 @@ static int enqueue_sweeps(lda_batch* b, int sweeps, int ll) {
         const bool last_ll = ll && s == sweeps - 1;
         dev::kb_zero<<<std::min<int>((int)b->zero.n, 4 * b->num_sms), 256, 0, b->st>>>(b->zero.p, (int)b->zero.n, b->counters);
         dev::kb_wt<<<grid_for(b->grid_wt, a.n_wt, W), threads, b->smem_hist, b->st>>>(a);
+        dev::kb_recip<<<M, 256, 0, b->st>>>(b->stt.p, b->sweeps_done);
         dev::kb_stats<<<grid_for(b->grid_stats, a.n_st, W), threads, b->smem_stats, b->st>>>(a);
         dev::kb_dt<<<grid_for(b->grid_dt, a.n_dt, W), threads, b->smem_dt, b->st>>>(a);
         const int gs = last_ll ? grid_for(b->grid_sample_ll, a.n_sm, W) : grid_for(b->grid_sample, a.n_sm, W);
@@ -406,7 +416,6 @@ static int enqueue_sweeps(lda_batch* b, int sweeps, int ll) {
             else dev::kb_sample<false, 1><<<gs, threads, b->smem_sample, b->st>>>(a);
         }
         if (last_ll) dev::kb_ll<<<M, 1024, 0, b->st>>>(b->sm.p, b->ll_dev);
-        dev::kb_advance<<<1, 1, 0, b->st>>>(b->sweeps_done);
         CUDA_TRY(cudaGetLastError());
         b->kernel_launches += last_ll ? 8 : 7;
     }

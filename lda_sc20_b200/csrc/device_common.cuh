@@ -150,28 +150,24 @@ __host__ __device__ __forceinline__ int col_skew(int k) { return k + (k >> 5); }
 __host__ __device__ __forceinline__ int col_words(int K) { return (K + (K >> 5) + 4) & ~3; }
 
 // phi_k = ((float)n_wk + beta) * r_k into a warp-private shared row (EZLDA builds the
-// same column as WTHead, utility.cu:1257-1269 sparse, :1698-1702 dense); SKEW selects the
-// sampler's layout.
-template <bool SKEW = false>
+// same column as WTHead, utility.cu:1257-1269 sparse, :1698-1702 dense).
 __device__ __forceinline__ void build_column(float* col, const float* r, int w, int Vd, int K, float beta,
                                              const int* __restrict__ dwt, const uint32_t* __restrict__ swt_off,
                                              const uint32_t* __restrict__ swt_nnz,
-                                             const uint32_t* __restrict__ swt_ent, int lane, uint32_t* nnz_read) {
+                                             const uint32_t* __restrict__ swt_ent, int lane) {
     if (w < Vd) {
         const int* row = dwt + (size_t)w * K;
-        for (int k = lane; k < K; k += 32)
-            col[SKEW ? col_skew(k) : k] = fmul(fadd(__int2float_rn(__ldg(row + k)), beta), r[k]);
+        for (int k = lane; k < K; k += 32) col[k] = fmul(fadd(__int2float_rn(__ldg(row + k)), beta), r[k]);
     } else {
-        for (int k = lane; k < K; k += 32) col[SKEW ? col_skew(k) : k] = fmul(beta, r[k]);
+        for (int k = lane; k < K; k += 32) col[k] = fmul(beta, r[k]);
         __syncwarp();
         const int s = w - Vd;
         const uint32_t off = __ldg(swt_off + s), nnz = __ldg(swt_nnz + s);
         for (uint32_t e = lane; e < nnz; e += 32) {
             const uint32_t en = __ldg(swt_ent + off + e);
             const uint32_t k = en >> 16;
-            col[SKEW ? col_skew((int)k) : (int)k] = fmul(fadd(u2f(en & 0xffffu), beta), r[k]);
+            col[k] = fmul(fadd(u2f(en & 0xffffu), beta), r[k]);
         }
-        if (nnz_read && lane == 0) *nnz_read += nnz;
     }
     __syncwarp();
 }
@@ -315,22 +311,34 @@ __device__ __forceinline__ int warp_level2_table(uint32_t n, float t2, int lane,
 }
 
 // Doc-row entries are (key << 16) | count.  Up to kLargeK topics the trainer's rows carry
-// the word column's slot index col_skew(k) as the key, so a lookup needs no index
-// arithmetic; above kLargeK, and in rows a caller supplies, the key is the topic k.
-// col_skew is k + k/32, so k = s - s/33 inverts it (s = 33a + b with b < 32).
+// the byte offset of the topic's word-column slot, 4 col_skew(k) (at most 8,440), as the
+// key, so that a lookup's address is one instruction from the entry; above kLargeK, and in
+// rows a caller supplies, the key is the topic k.  col_skew is k + k/32, so k = s - s/33
+// inverts it (s = 33a + b with b < 32).
 __host__ __device__ __forceinline__ int col_unskew(int s) { return s - s / 33; }
+__host__ __device__ __forceinline__ uint32_t row_key(int K, uint32_t k) {
+    return K <= kLargeK ? 4u * (uint32_t)col_skew((int)k) : k;
+}
+__host__ __device__ __forceinline__ uint32_t row_topic(int K, uint32_t key) {
+    return K <= kLargeK ? (uint32_t)col_unskew((int)(key >> 2)) : key;
+}
 
 // The sampler's view of the tile's word column: colz(k) = phi_k of the word with its max
 // topic zeroed; row(key) the same for a doc-row key and topic(key) the key's topic.
 // ColSharedT reads a column built in shared memory (skewed layout, with the max topic's
-// slot already zeroed); SKEWKEYS: the rows' keys are slot indices.
-template <bool SKEWKEYS>
+// slot already zeroed); SLOTKEYS: the rows' keys are slot byte offsets.
+template <bool SLOTKEYS>
 struct ColSharedT {
     using Entry = uint32_t;  // a doc-row entry: (key << 16) | count
     const float* col;
     __device__ __forceinline__ float operator()(int k) const { return col[col_skew(k)]; }
-    __device__ __forceinline__ float row(uint32_t key) const { return col[SKEWKEYS ? (int)key : col_skew((int)key)]; }
-    __device__ __forceinline__ int topic(uint32_t key) const { return SKEWKEYS ? col_unskew((int)key) : (int)key; }
+    __device__ __forceinline__ float row(uint32_t key) const {
+        return SLOTKEYS ? *reinterpret_cast<const float*>(reinterpret_cast<const char*>(col) + key)
+                        : col[col_skew((int)key)];
+    }
+    __device__ __forceinline__ int topic(uint32_t key) const {
+        return SLOTKEYS ? col_unskew((int)(key >> 2)) : (int)key;
+    }
     __device__ __forceinline__ uint32_t key(uint32_t e) const { return e >> 16; }
     __device__ __forceinline__ float cnt(uint32_t e) const { return u2f(e & 0xffffu); }
 };
@@ -348,58 +356,40 @@ __device__ __forceinline__ int ldg_hint(const int* p, uint64_t pol) {
     return v;
 }
 
+// N steps of lane_mass: the loads of all steps, then the fmaf chain.  MASKED: only the lanes
+// below `left` have an entry in the last step; the others add an entry of count 0, and
+// fmaf(0, phi, acc) is acc.
+template <int N, bool MASKED, class View>
+__device__ __forceinline__ float lane_steps(const typename View::Entry* __restrict__ p, uint32_t lane, uint32_t left,
+                                            const View& colz, float acc) {
+    using E = typename View::Entry;
+    E e[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) e[j] = (!MASKED || j < N - 1 || lane < left) ? __ldg(p + 32 * j) : E{};
+#pragma unroll
+    for (int j = 0; j < N; ++j) acc = ffma(colz.cnt(e[j]), colz.row(colz.key(e[j])), acc);
+    return acc;
+}
+
 // Serial per-lane sum over the lane's entries l, l + 32, l + 64, ... of a doc row of nnz
 // entries (one fmaf chain).  A warp's loads of one step then read 32 consecutive entries,
 // one or two 128-byte lines, where contiguous per-lane blocks would touch one line per
-// lane block.
-// ROWM 1: the loads of four steps at a time are issued before their use (rows that often
-// miss L2, at large K); ROWM 0: two steps at a time.
-template <int ROWM = 0, class View>
+// lane block.  Every branch is uniform across the warp: whole batches of four steps, then
+// the one of four straight-line tails that the row's remaining steps ask for.  A row's sum
+// is the sampler's inner loop, and the sampler is bound by the instructions it issues:
+// loops with predicated ends took 100 warp instructions per row of 122 entries.
+template <class View>
 __device__ __forceinline__ float lane_mass(const typename View::Entry* __restrict__ row, uint32_t lane, uint32_t nnz,
-                                           const View& colz, float acc = 0.0f) {
-    using E = typename View::Entry;
-    // Loop bounds are warp-uniform: `full` steps in which every lane has an entry, taken in
-    // batches, then the lane's last steps together with the partial step.  Bounds per lane
-    // would send the lanes of one warp through different batches, and the warp would issue
-    // each of them (K=1024 corpus: sampler 10.38 -> 9.93 ms per sweep, the same sums).
-    const uint32_t full = nnz >> 5;
-    const E* __restrict__ p = row + lane;
-    uint32_t s = 0;
-    if (ROWM == 1) {
-        for (; s + 4u <= full; s += 4u) {
-            const E e0 = __ldg(p + 32u * s), e1 = __ldg(p + 32u * s + 32u), e2 = __ldg(p + 32u * s + 64u),
-                    e3 = __ldg(p + 32u * s + 96u);
-            acc = ffma(colz.cnt(e0), colz.row(colz.key(e0)), acc);
-            acc = ffma(colz.cnt(e1), colz.row(colz.key(e1)), acc);
-            acc = ffma(colz.cnt(e2), colz.row(colz.key(e2)), acc);
-            acc = ffma(colz.cnt(e3), colz.row(colz.key(e3)), acc);
-        }
-        // the lane's last steps (up to three full ones and the partial one): their loads
-        // issued together, so that a row of up to 256 entries costs two rounds of loads
-        const uint32_t nl = full + (lane < (nnz & 31u) ? 1u : 0u);
-        if (s < full + ((nnz & 31u) ? 1u : 0u)) {
-            E e[4];
-#pragma unroll
-            for (uint32_t j = 0; j < 4u; ++j) e[j] = s + j < nl ? __ldg(p + 32u * (s + j)) : E{};
-#pragma unroll
-            for (uint32_t j = 0; j < 4u; ++j)
-                if (s + j < nl) acc = ffma(colz.cnt(e[j]), colz.row(colz.key(e[j])), acc);
-        }
-        return acc;
+                                           const View& colz) {
+    const typename View::Entry* __restrict__ p = row + lane;
+    float acc = 0.0f;
+    for (; nnz > 128u; nnz -= 128u, p += 128) acc = lane_steps<4, false>(p, lane, 0u, colz, acc);
+    if (nnz > 64u) {
+        if (nnz > 96u) return lane_steps<4, true>(p, lane, nnz - 96u, colz, acc);
+        return lane_steps<3, true>(p, lane, nnz - 64u, colz, acc);
     }
-    for (; s + 2u <= full; s += 2u) {
-        const E e0 = __ldg(p + 32u * s), e1 = __ldg(p + 32u * s + 32u);
-        acc = ffma(colz.cnt(e0), colz.row(colz.key(e0)), acc);
-        acc = ffma(colz.cnt(e1), colz.row(colz.key(e1)), acc);
-    }
-    // the last full step (if any) and the lanes of the partial step, loads issued together
-    const bool one = s < full, tail = lane < (nnz & 31u);
-    E e0{}, e1{};
-    if (one) e0 = __ldg(p + 32u * s);
-    if (tail) e1 = __ldg(p + 32u * full);
-    if (one) acc = ffma(colz.cnt(e0), colz.row(colz.key(e0)), acc);
-    if (tail) acc = ffma(colz.cnt(e1), colz.row(colz.key(e1)), acc);
-    return acc;
+    if (nnz > 32u) return lane_steps<2, true>(p, lane, nnz - 32u, colz, acc);
+    return lane_steps<1, true>(p, lane, nnz, colz, acc);
 }
 
 // The S-bucket draw among lane ls's entries ls, ls + 32, ... of the row: their serial

@@ -539,7 +539,8 @@ __global__ void __launch_bounds__(256, LDA_DT_SMALL_MIN_BLOCKS) k_dt_build_small
     }
 }
 
-// Word statistics: warp per word.
+// Word statistics: warp per word.  CTA 0 also leaves the reciprocals and the column of a
+// word without tokens for the sampler.
 __global__ void __launch_bounds__(256) k_word_stats(StatsArgs a) {
     extern __shared__ float smf[];
     const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -547,6 +548,12 @@ __global__ void __launch_bounds__(256) k_word_stats(StatsArgs a) {
     float* col = smf + (size_t)a.K * (1 + wid);
     fill_recip(r, a.n_k, a.K, a.Vbeta);
     __syncthreads();
+    if (blockIdx.x == 0 && a.recip_out) {
+        for (int k = threadIdx.x; k < a.K; k += blockDim.x) {
+            a.recip_out[k] = r[k];
+            a.base_out[col_skew(k)] = fmul(a.beta, r[k]);
+        }
+    }
     for (int w = a.wlo + blockIdx.x * warps + wid; w < a.V; w += gridDim.x * warps) {
         word_stats_word(a, w, r, col, lane);
     }
@@ -586,27 +593,30 @@ __global__ void __launch_bounds__(256) k_dt_build(DtArgs a) {
     }
 }
 
-// Sampler: warp per tile, tiles taken from an atomic counter.  SKEWKEYS: the doc rows'
-// keys are word-column slot indices (the trainer's rows up to kLargeK topics).
+// Sampler: warp per tile, tiles taken from an atomic counter (the next one is claimed when a
+// tile starts, so that the claim's round trip overlaps the tile's work).  SKEWKEYS: the doc
+// rows' keys are word-column slot indices and a.recip / a.base are there (the trainer's rows
+// and tables up to kLargeK topics).
 template <bool LL, int QB = 1, bool SKEWKEYS = true>
-__global__ void __launch_bounds__(32 * kSampleWarps, LL ? LDA_SAMPLE_LL_MIN_BLOCKS
-                                                       : (QB == 1 ? LDA_SAMPLE_MIN_BLOCKS : LDA_SAMPLE_QB_MIN_BLOCKS))
+__global__ void __launch_bounds__(32 * kSampleWarps, QB > 1 ? LDA_SAMPLE_QB_MIN_BLOCKS
+                                                       : (LL ? LDA_SAMPLE_LL_MIN_BLOCKS : LDA_SAMPLE_MIN_BLOCKS))
 k_sample_t(SampleArgs a) {
     extern __shared__ float smf[];
-    const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* r = smf;
-    float* col = smf + a.K + (size_t)col_words(a.K) * wid;
-    uint32_t* ctr = reinterpret_cast<uint32_t*>(smf + a.K + (size_t)col_words(a.K) * warps) + C_NUM * wid;
-    fill_recip(r, a.n_k, a.K, a.Vbeta);
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* col = smf + (size_t)sample_warp_words(a.K, a.nslots) * wid;
+    float* slots = col + col_words(a.K);
+    uint32_t* ctr = reinterpret_cast<uint32_t*>(slots + ((row_state_words(a.nslots) + 3) & ~3));
     if (lane < C_NUM) ctr[lane] = 0u;
-    __syncthreads();
-    for (;;) {
-        int tile = 0;
-        if (lane == 0) tile = (int)atomicAdd(a.tile_counter, 1u);
-        tile = __shfl_sync(FULL, tile, 0);
-        if (tile >= a.ntiles) break;
-        const int4 t = a.tiles[tile];
-        sample_tile<LL, QB, SKEWKEYS>(a, tile, t, a.iter, r, col, ctr, lane);
+    __syncwarp();
+    bool clean = false;
+    int tile = 0;
+    if (lane == 0) tile = (int)atomicAdd(a.tile_counter, 1u);
+    tile = __shfl_sync(FULL, tile, 0);
+    while (tile < a.ntiles) {
+        int next = 0;
+        if (lane == 0) next = (int)atomicAdd(a.tile_counter, 1u);
+        sample_tile<LL, QB, SKEWKEYS>(a, tile, a.tiles[tile], a.iter, col, slots, clean, ctr, lane);
+        tile = __shfl_sync(FULL, next, 0);
     }
     __syncwarp();
     if (lane < C_NUM && ctr[lane]) atomicAdd(a.ctr + lane, (unsigned long long)ctr[lane]);
@@ -656,8 +666,9 @@ __host__ __device__ __forceinline__ int large_pre_words(int K) { return ((K + 31
 // (col_words(K) floats: a Q round's 32 topics k, k + 32, ... then sit in 32 banks), then
 // per warp the bitmap, then per warp the prefix counts (uint16, an even number per warp),
 // then per warp the counter row.
-__host__ __device__ __forceinline__ size_t sparse_large_smem(int K, int warps) {
-    return (size_t)col_words(K) * 4 + (size_t)warps * (large_bit_words(K) * 4 + large_pre_words(K) * 2 + C_NUM * 4);
+__host__ __device__ __forceinline__ size_t sparse_large_smem(int K, int warps, int nslots) {
+    return (size_t)col_words(K) * 4 +
+           (size_t)warps * (large_bit_words(K) * 4 + large_pre_words(K) * 2 + C_NUM * 4 + row_state_words(nslots) * 4) + 8;
 }
 
 // Shared memory of the dense-word kernel: the shared column, the warps' counter rows and
@@ -667,20 +678,13 @@ __host__ __device__ __forceinline__ size_t sparse_large_smem(int K, int warps) {
 #endif
 // Shared memory of the dense-word sampler: the word column, the warps' counter rows, their
 // LL partials and (when qtab_rounds(K) > 0) the Q-round table of 32 x R float2.
-__host__ __device__ __forceinline__ size_t dense_large_smem(int K, int warps) {
+__host__ __device__ __forceinline__ size_t dense_large_smem(int K, int warps, int nslots) {
     return (((size_t)col_words(K) * 4 + (size_t)warps * C_NUM * 4 + 7) & ~(size_t)7) + (size_t)warps * 8 +
-           (LDA_QTAB ? (size_t)32 * qtab_rounds(K) * sizeof(float2) : 0);
+           (LDA_QTAB ? (size_t)32 * qtab_rounds(K) * sizeof(float2) : 0) + (size_t)warps * row_state_words(nslots) * 4;
 }
 
 #ifndef LDA_DENSE_LARGE_MIN_BLOCKS
 #define LDA_DENSE_LARGE_MIN_BLOCKS 4
-#endif
-
-// How the large-K samplers issue a doc row's loads (lane_mass ROWM): four steps together,
-// since at large K a third of the rows' bytes miss L2 (K=10,000 corpus: 148.3 -> 133.6
-// ms of sampling per sweep; at K=1024 the same batching loses).
-#ifndef LDA_LARGE_ROW_MODE
-#define LDA_LARGE_ROW_MODE 1
 #endif
 
 // The sparse-word sampler keeps each word's Qw rounds' table in registers (lane r: round
@@ -699,6 +703,9 @@ __global__ void __launch_bounds__(256, LDA_SPARSE_LARGE_MIN_BLOCKS) k_sample_spa
                                                                             (size_t)bw * warps) +
                                                 (size_t)pw * warps) +
                     C_NUM * wid;
+    float* slots = reinterpret_cast<float*>(
+                       (reinterpret_cast<uintptr_t>(ctr + C_NUM * (warps - wid)) + 7) & ~(uintptr_t)7) +
+                   (size_t)row_state_words(a.nslots) * wid;
     for (int k = threadIdx.x; k < a.K; k += blockDim.x)
         r[col_skew(k)] = __fdiv_rn(1.0f, fadd(__int2float_rn(a.n_k[k]), a.Vbeta));
     for (int i = lane; i < bw; i += 32) bits[i] = 0u;
@@ -741,9 +748,9 @@ __global__ void __launch_bounds__(256, LDA_SPARSE_LARGE_MIN_BLOCKS) k_sample_spa
         const ColBits view{bits, pre, ent, r, a.beta, maxK};
         SplitQ sq{ent, nnz_w, __shfl_sync(FULL, QL, 0), a.smooth, r, true};
         split_q_table(sq, maxK, a.alpha, lane);
-        double ll = sample_groups<LL, QB, true, LDA_LARGE_ROW_MODE>(a, (uint32_t)t.y, (uint32_t)t.z, 0u, 32u, a.iter,
-                                                                    maxK, ph, QL, QP, Q, view, ctr, lane, nullptr, 0,
-                                                                    &sq);
+        double ll = sample_groups<LL, QB, true>(a, (uint32_t)t.y, (uint32_t)t.z, 0u, 32u, a.iter,
+                                                                    maxK, ph, QL, QP, Q, view, ctr, lane, slots,
+                                                                    nullptr, 0, &sq);
         if (LL) {
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) ll += __shfl_xor_sync(FULL, ll, off);
@@ -771,6 +778,7 @@ __global__ void __launch_bounds__(256, LDA_DENSE_LARGE_MIN_BLOCKS) k_sample_dens
         (reinterpret_cast<uintptr_t>(ctr_all + C_NUM * warps) + 7) & ~(uintptr_t)7);
     const int qr = LDA_QTAB ? qtab_rounds(a.K) : 0;
     float2* qtab = reinterpret_cast<float2*>(wll + warps);
+    float* slots = reinterpret_cast<float*>(qtab + 32 * qr) + (size_t)row_state_words(a.nslots) * wid;
     if (lane < C_NUM) ctr[lane] = 0u;
     __syncthreads();
     for (;;) {
@@ -838,10 +846,11 @@ __global__ void __launch_bounds__(256, LDA_DENSE_LARGE_MIN_BLOCKS) k_sample_dens
         const float QL = __ldg(a.st_ql + (size_t)w * 32 + lane);
         const float QP = warp_ks_scan(QL, lane);
         const float Q = __shfl_sync(FULL, QP, 31);
-        double ll = sample_groups<LL, QB, false, LDA_LARGE_ROW_MODE>(a, (uint32_t)t.y, (uint32_t)t.z, 32u * wid,
+        double ll = sample_groups<LL, QB, false>(a, (uint32_t)t.y, (uint32_t)t.z, 32u * wid,
                                                                      32u * warps, a.iter, maxK, ph, QL, QP, Q,
-                                                                     ColShared{col}, ctr, lane, qr ? qtab : nullptr, qr,
-                                                                     nullptr, LL ? nullptr : &s_group);
+                                                                     ColShared{col}, ctr, lane, slots,
+                                                                     qr ? qtab : nullptr, qr, nullptr,
+                                                                     LL ? nullptr : &s_group);
         if (LL) {
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) ll += __shfl_xor_sync(FULL, ll, off);

@@ -134,7 +134,9 @@ struct StatsArgs {
     float* st_ql;       // [V*32]
     const float* smooth = nullptr;  // K > kLargeK: the smoothing table (k_smooth_table)
     int wlo = 0;                    // the words [wlo, V) get statistics (a word range)
-    const float* recip = nullptr;   // K > kLargeK: r_k as fill_recip forms it (k_recip)
+    const float* recip = nullptr;   // r_k as fill_recip forms it
+    float* recip_out = nullptr;     // K <= kLargeK: where the statistics leave r_k ...
+    float* base_out = nullptr;      // ... and beta * r_k in the skewed column layout
     const int* order = nullptr;     // K > kLargeK: the sparse words' topic order (k_sparse_order)
     // K > kLargeK: the dense words' Q-round tables (32 lane slots x qrounds float2 per word,
     // the table k_sample_dense_large would build per tile), or null
@@ -163,7 +165,7 @@ template <class Phi>
 __device__ __forceinline__ int word_stats_from(const StatsArgs& a, int w, const Phi& phi, int lane);
 
 __device__ __forceinline__ void word_stats_word(const StatsArgs& a, int w, const float* r, float* col, int lane) {
-    build_column(col, r, w, a.Vd, a.K, a.beta, a.dwt, a.swt_off, a.swt_nnz, a.swt_ent, lane, nullptr);
+    build_column(col, r, w, a.Vd, a.K, a.beta, a.dwt, a.swt_off, a.swt_nnz, a.swt_ent, lane);
     word_stats_from(a, w, ColumnPhi{col}, lane);
 }
 
@@ -355,8 +357,7 @@ __device__ __forceinline__ void dt_doc(const DtArgs& a, uint32_t d, const H& his
         while (m) {
             const uint32_t k = (uint32_t)wi * 32u + (uint32_t)(__ffs(m) - 1);
             m &= m - 1u;
-            const uint32_t key = a.K <= kLargeK ? (uint32_t)col_skew((int)k) : k;
-            out[p++] = (key << 16) | hist.get(k);
+            out[p++] = (row_key(a.K, k) << 16) | hist.get(k);
             hist.clear(k);
         }
     }
@@ -409,9 +410,17 @@ struct SampleArgs {
     // tok_doc / meta hold tokens [tok_base, ...) and dt_ent the doc-row entries
     // [dt_base, ...) (non-zero when the chunk is streamed into a slot buffer)
     uint32_t tok_base, dt_base;
-    // r_k = 1 / ((float)n_k + V*beta) for k < K, formed once per sweep (the K > kLargeK
-    // dense-word sampler reads it instead of dividing for every tile's column)
+    // r_k = 1 / ((float)n_k + V*beta) for k < K, formed once per sweep with the word
+    // statistics, or null (then a column's r_k are formed from n_k)
     const float* recip = nullptr;
+    // K <= kLargeK: beta * r_k in the skewed column layout, the column of a word without
+    // tokens (col_words(K) floats, formed with recip)
+    const float* base = nullptr;
+    int nslots = 1;  // row slots per warp (sample_groups)
+    template <bool TABLE>
+    __device__ __forceinline__ float rk(int k) const {
+        return TABLE ? __ldg(recip + k) : __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta));
+    }
     // K > kLargeK: the smoothing table of the split Q bucket (k_smooth_table)
     const float* smooth = nullptr;
     // K > kLargeK: the dense words' Q-round tables (word_qtab), or null
@@ -425,13 +434,17 @@ struct SplitQ {
     uint32_t nnz;
     float Qw;
     const float* T;       // the smoothing table (K entries, non-decreasing)
-    const float* r;       // r_k, at col_skew(k) when skew
+    const float* r;       // r_k, at col_skew(k) when skew; null: formed from n_k
     bool skew;
     // the Qw rounds' table, lane r holding round r's (carry before it, carry + its largest
     // KS prefix); rounds = 0 when not built (more than 32 rounds, or not wanted)
     int rounds = 0;
     float qcarry = 0.0f, qthr = 0.0f;
-    __device__ __forceinline__ float rk(int k) const { return r[skew ? col_skew(k) : k]; }
+    const int* n_k = nullptr;
+    float Vbeta = 0.0f;
+    __device__ __forceinline__ float rk(int k) const {
+        return r ? r[skew ? col_skew(k) : k] : __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta));
+    }
     // round slot i of the Qw search: alpha * (n_wk * r_k), the max topic's term 0
     __device__ __forceinline__ void slot(uint32_t i, int maxK, float alpha, int& key, float& term, bool& ok) const {
         const uint32_t en = __ldg(ent + i);
@@ -525,28 +538,90 @@ enum { BR_NONE = 0, BR_MAX = 1, BR_S = 2, BR_Q = 3 };
 #endif
 constexpr int kSampleWarps = LDA_SAMPLE_WARPS;
 #ifndef LDA_SAMPLE_MIN_BLOCKS
-#define LDA_SAMPLE_MIN_BLOCKS 5
+#define LDA_SAMPLE_MIN_BLOCKS 4
 #endif
 #ifndef LDA_SAMPLE_QB_MIN_BLOCKS
-#define LDA_SAMPLE_QB_MIN_BLOCKS 4
+#define LDA_SAMPLE_QB_MIN_BLOCKS 3
 #endif
 #ifndef LDA_SAMPLE_LL_MIN_BLOCKS
-#define LDA_SAMPLE_LL_MIN_BLOCKS 5
+#define LDA_SAMPLE_LL_MIN_BLOCKS 4
 #endif
 #ifndef LDA_SPARSE_LARGE_MIN_BLOCKS
 #define LDA_SPARSE_LARGE_MIN_BLOCKS 4
 #endif
 
+// The slots in which a warp keeps doc rows' lane sums: row slot s holds the 32 sums of one
+// row at [33 s, 33 s + 32), so that 32 threads reading element i of 32 different rows touch
+// 32 banks.
+constexpr int kSlotWords = 33;
+// Words of a warp's row slots, even (the rows' list, 32 x {offset, length}, follows them).
+__host__ __device__ __forceinline__ int slot_words(int nslots) { return (kSlotWords * nslots + 1) & ~1; }
+__host__ __device__ __forceinline__ int row_state_words(int nslots) { return slot_words(nslots) + 64; }
+
+// A warp's search for the S bucket's lane, for one token (the whole warp works on it): the
+// first lane whose prefix exceeds tt and whose sum is positive, else the last lane with a
+// positive sum.
+__device__ __forceinline__ int warp_s_lane(float SL, float tt, int lane, float& prev) {
+    const float SP = warp_ks_scan(SL, lane);
+    const unsigned cand = __ballot_sync(FULL, tt < SP && SL > 0.0f), pos = __ballot_sync(FULL, SL > 0.0f);
+    const int ls = cand ? __ffs(cand) - 1 : 31 - __clz(pos);
+    prev = __shfl_sync(FULL, SP, ls > 0 ? ls - 1 : 0);
+    return ls;
+}
+
+// The Kogge-Stone scan of 32 values held by one thread: element l adds element l - off at
+// each step off = 1, 2, ..., 16, the additions of warp_ks_scan.
+__device__ __forceinline__ void thread_ks_scan(float (&v)[32]) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+        for (int l = 31; l >= off; --l) v[l] = fadd(v[l], v[l - off]);
+    }
+}
+
+// The crossing of t in 32 Kogge-Stone prefixes of non-negative terms held by one thread: a
+// binary search with the prefixes halved in registers.  idx is a place with
+// v[idx - 1] <= t (prev) and, when any prefix exceeds t, t < v[idx] (at).  Rounding can leave
+// the prefixes out of order by a few units in the last place: a prefix is within (1 + 2^-24)^5
+// of its exact sum and the exact sums ascend, so when t >= prev (1 + 2^-19) no earlier prefix
+// exceeds t, and idx is the first place that does.  `sure` says so (false also when no
+// prefix exceeds t).
+__device__ __forceinline__ void thread_crossing(const float (&v)[32], float t, int& idx, float& prev, bool& sure) {
+    float w[16];
+    prev = 0.0f;
+    bool up = !(t < v[15]);
+    idx = up ? 16 : 0;
+    if (up) prev = v[15];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) w[i] = up ? v[16 + i] : v[i];
+#pragma unroll
+    for (int h = 8; h >= 1; h >>= 1) {
+        up = !(t < w[h - 1]);
+        idx += up ? h : 0;
+        if (up) prev = w[h - 1];
+#pragma unroll
+        for (int i = 0; i < h; ++i) w[i] = up ? w[h + i] : w[i];
+    }
+    sure = t < w[0] && !(t < fmul(prev, 1.0f + 0x1p-19f));
+}
+
 // The 32-token groups g0, g0 + gstep, ... of the token range [start, start + cnt) of one
 // word (column view colz, max topic maxK, phi4 ph, Q partials QL / QP / Q of the word), or,
 // with a shared group counter gq, the groups the warp claims from it (32 tokens at a time,
-// so that the warps sharing a tile finish it together).  Returns the lane's LL partial (LL
-// mode).
-template <bool LL, int QB, bool SPLIT = false, int ROWM = 0, class View>
+// so that the warps sharing a tile finish it together).  `slots` holds the warp's a.nslots
+// row slots and its list of a group's rows (row_state_words).  Returns the lane's LL partial (LL mode).
+//
+// A group runs in three parts: its tokens are screened thread-per-token; the doc rows that
+// the unsettled tokens need are summed one after another by the whole warp into the slots
+// (consecutive tokens of one doc share a row, also across groups); then each token's thread
+// scans its row's 32 lane sums, forms S and picks bucket and lane by itself.  Deciding each
+// token with the whole warp (a scan by shuffles, ballots and broadcasts per token) took
+// about half of the kernel's instructions, and the kernel is bound by their issue.
+template <bool LL, int QB, bool SPLIT = false, class View>
 __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t start, uint32_t cnt, uint32_t g0,
                                                 uint32_t gstep, uint32_t iter, int maxK, const float4 ph, float QL,
                                                 float QP, float Q, const View& colz, uint32_t* ctr, int lane,
-                                                const float2* qtab = nullptr, int qrounds = 0,
+                                                float* slots, const float2* qtab = nullptr, int qrounds = 0,
                                                 const SplitQ* sq = nullptr, uint32_t* gq = nullptr) {
     auto claim = [&]() {
         uint32_t v = 0;
@@ -560,10 +635,10 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
     int ll_n = 0;
     using E = typename View::Entry;
     const E* rows = reinterpret_cast<const E*>(a.dt_ent);
-    uint32_t cur = 0xffffffffu, nnz = 0;
-    const E* row = rows;
-    float SL = 0.0f, SP = 0.0f, S = 0.0f;
-    unsigned spos = 0u;  // lanes of the current row with a positive sum
+    const int nslots = a.nslots;
+    uint2* list = reinterpret_cast<uint2*>(slots + slot_words(nslots));
+    uint32_t cur = 0xffffffffu;  // the doc of the last row summed, in slot cslot
+    int cslot = 0;
     for (uint32_t g = gq ? claim() : g0; g < cnt; g = gq ? claim() : g + gstep) {
         const bool valid = g + lane < cnt;
         const uint32_t tok = start + g + lane;
@@ -584,77 +659,124 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
             ea = fmul(u, bound) < pmax;
         }
         int znew = maxK;
-        // per-lane record of this token's evaluation, for the deferred draw and counters
         uint32_t my_ls = 0;
-        float my_t2 = 0.0f, my_total = 0.0f;
+        float my_t = 0.0f, my_total = 0.0f;
         int kind = BR_NONE;
-        bool evaluated = false;
         const unsigned vmask = __ballot_sync(FULL, valid);
         const unsigned emask = __ballot_sync(FULL, ea);
-        const unsigned need0 = LL ? vmask : (vmask & ~emask);
-        unsigned need = need0;
-        while (need) {
-            const int j = __ffs(need) - 1;
-            need &= need - 1u;
-            const uint32_t dj = __shfl_sync(FULL, d, j);
-            if (dj != cur) {
-                cur = dj;
-                nnz = __shfl_sync(FULL, my_nnz, j);
-                row = rows + __shfl_sync(FULL, my_off, j);
-                SL = lane_mass<ROWM>(row, (uint32_t)lane, nnz, colz);
-                SP = warp_ks_scan(SL, lane);
-                S = __shfl_sync(FULL, SP, 31);
-                spos = __ballot_sync(FULL, SL > 0.0f);
-                evaluated |= (lane == j);
-            }
-            const float pmj = __shfl_sync(FULL, pmax, j);
-            const float uj = __shfl_sync(FULL, u, j);
-            const float pS = fadd(pmj, S);
-            const float total = fadd(pS, Q);
-            if (LL && lane == j) my_total = total;
-            if (LL && ((emask >> j) & 1u)) continue;
-            const float target = fmul(uj, total);
-            if (target < pmj) {
-                if (lane == j) kind = BR_MAX;
-            } else if (target < pS) {
-                const float tt = fsub(target, pmj);
-                const unsigned cand = __ballot_sync(FULL, tt < SP && SL > 0.0f);
-                const int ls = cand ? __ffs(cand) - 1 : 31 - __clz(spos);
-                const float prev = __shfl_sync(FULL, SP, ls > 0 ? ls - 1 : 0);
-                if (lane == j) {
-                    kind = BR_S;
-                    my_ls = (uint32_t)ls;
-                    my_t2 = ls > 0 ? fsub(tt, prev) : tt;
+        const unsigned need = LL ? vmask : (vmask & ~emask);
+        const bool mine = (need >> lane) & 1u;
+        // the tokens that start a new row: those whose doc differs from the previous
+        // evaluated token's (the last group's last row for the first)
+        const unsigned below = need & ((1u << lane) - 1u);
+        uint32_t dp = __shfl_sync(FULL, d, below ? 31 - __clz(below) : lane);
+        if (!below) dp = cur;
+        const bool lead = mine && d != dp;
+        const unsigned leaders = __ballot_sync(FULL, lead);
+        if (need) {
+            // the group's rows in order: row 0 is the carried one when its first token's doc
+            // was the last one summed (its sums move to the first slot); rows r0 + i of a
+            // part sit in slot i.  The rows' places and lengths wait in `list`.
+            const bool carried = !(leaders & need & (0u - need));
+            const int c1 = carried ? 1 : 0;
+            const int nrows = __popc(leaders) + c1;
+            const int ri = __popc(leaders & ((2u << lane) - 1u)) - 1 + c1;
+            if (lead) list[ri] = make_uint2(my_off, my_nnz);
+            if (carried) slots[lane] = slots[kSlotWords * cslot + lane];
+            __syncwarp();
+            for (int r0 = 0; r0 < nrows; r0 += nslots) {
+                const int n = min(nrows - r0, nslots);
+                float* out = slots + lane;
+                int i = 0;
+                if (r0 == 0) {
+                    i = c1;
+                    out += kSlotWords * c1;
                 }
+                for (; i < n; ++i, out += kSlotWords) {
+                    const uint2 q = list[r0 + i];
+                    *out = lane_mass(rows + q.x, (uint32_t)lane, q.y, colz);
+                }
+                __syncwarp();
+                // the tokens of these rows, thread per token
+                const bool act = mine && (unsigned)(ri - r0) < (unsigned)n;
+                const int my_s = act ? ri - r0 : 0;
+                const float* p = slots + kSlotWords * my_s;
+                float tt;
+                bool slow = false;
+                {
+                    float v[32];
+#pragma unroll
+                    for (int l = 0; l < 32; ++l) v[l] = p[l];
+                    thread_ks_scan(v);
+                    const float pS = fadd(pmax, v[31]);
+                    const float total = fadd(pS, Q);
+                    const float target = fmul(u, total);
+                    tt = fsub(target, pmax);
+                    int ls;
+                    float prev;
+                    bool sure;
+                    thread_crossing(v, tt, ls, prev, sure);
+                    if (act) {
+                        if (LL) my_total = total;
+                        if (!LL || !ea) {
+                            if (target < pmax) {
+                                kind = BR_MAX;
+                            } else if (target < pS) {
+                                kind = BR_S;
+                                my_ls = (uint32_t)ls;
+                                my_t = ls > 0 ? fsub(tt, prev) : tt;
+                                slow = !sure || !(p[ls] > 0.0f);
+                            } else {
+                                kind = BR_Q;
+                                my_t = fsub(target, pS);
+                            }
+                        }
+                    }
+                }
+                // a token whose lane the search could not be sure of: with the whole warp
+                for (unsigned b = __ballot_sync(FULL, slow); b; b &= b - 1u) {
+                    const int j = __ffs(b) - 1;
+                    const float SL = slots[kSlotWords * __shfl_sync(FULL, my_s, j) + lane];
+                    const float ttj = __shfl_sync(FULL, tt, j);
+                    float prev;
+                    const int ls = warp_s_lane(SL, ttj, lane, prev);
+                    if (lane == j) {
+                        my_ls = (uint32_t)ls;
+                        my_t = ls > 0 ? fsub(ttj, prev) : ttj;
+                    }
+                }
+                __syncwarp();  // the slots may be overwritten
+            }
+            cslot = (nrows - 1) % nslots;
+            cur = __shfl_sync(FULL, d, 31 - __clz(need));
+        }
+        const unsigned qm = __ballot_sync(FULL, kind == BR_Q);
+        for (unsigned b = qm; b; b &= b - 1u) {
+            const int j = __ffs(b) - 1;
+            const float tt = __shfl_sync(FULL, my_t, j);
+            int zq;
+            if (SPLIT) {
+                zq = split_q_draw(*sq, tt, maxK, a.K, a.alpha, a.beta, lane);
             } else {
-                const float tt = fsub(target, pS);
-                int zq;
-                if (SPLIT) {
-                    zq = split_q_draw(*sq, tt, maxK, a.K, a.alpha, a.beta, lane);
-                } else {
-                    const unsigned cand = __ballot_sync(FULL, tt < QP && QL > 0.0f);
-                    const unsigned pos = __ballot_sync(FULL, QL > 0.0f);
-                    const int ls = cand ? __ffs(cand) - 1 : (pos ? 31 - __clz(pos) : 0);
-                    const float prev = __shfl_sync(FULL, QP, ls > 0 ? ls - 1 : 0);
-                    const float t2 = ls > 0 ? fsub(tt, prev) : tt;
-                    const int K = a.K;
-                    const float alpha = a.alpha;
-                    const uint32_t n = (uint32_t)((K - ls + 31) / 32);
-                    auto slot = [&](uint32_t i, int& key, float& term, bool& ok) {
-                        const int k = ls + 32 * (int)i;
-                        const float cz = colz(k);
-                        key = k;
-                        term = fmul(alpha, cz);
-                        ok = cz > 0.0f;
-                    };
-                    zq = qtab ? warp_level2_table(n, t2, lane, slot, qtab + ls * qrounds) : -1;
-                    if (zq < 0) zq = warp_level2_rounds<QB>(n, t2, maxK, lane, slot);
-                }
-                if (lane == j) {
-                    kind = BR_Q;
-                    znew = zq;
-                }
+                const unsigned cand = __ballot_sync(FULL, tt < QP && QL > 0.0f);
+                const unsigned pos = __ballot_sync(FULL, QL > 0.0f);
+                const int ls = cand ? __ffs(cand) - 1 : (pos ? 31 - __clz(pos) : 0);
+                const float prev = __shfl_sync(FULL, QP, ls > 0 ? ls - 1 : 0);
+                const float t2 = ls > 0 ? fsub(tt, prev) : tt;
+                const int K = a.K;
+                const float alpha = a.alpha;
+                const uint32_t n = (uint32_t)((K - ls + 31) / 32);
+                auto slot = [&](uint32_t i, int& key, float& term, bool& ok) {
+                    const int k = ls + 32 * (int)i;
+                    const float cz = colz(k);
+                    key = k;
+                    term = fmul(alpha, cz);
+                    ok = cz > 0.0f;
+                };
+                zq = qtab ? warp_level2_table(n, t2, lane, slot, qtab + ls * qrounds) : -1;
+                if (zq < 0) zq = warp_level2_rounds<QB>(n, t2, maxK, lane, slot);
             }
+            if (lane == j) znew = zq;
         }
         // each lane's own token's log-likelihood factors, all lanes at once (every lane
         // accumulates only its own tokens, in group order)
@@ -668,23 +790,21 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
             }
         }
         // an S-bucket token's row is its own doc's: the lane holds its offset and length
-        if (kind == BR_S) znew = lane_draw(rows + my_off, my_ls, my_nnz, colz, my_t2, maxK);
+        if (kind == BR_S) znew = lane_draw(rows + my_off, my_ls, my_nnz, colz, my_t, maxK);
         if (valid) a.z[tok] = (uint16_t)znew;
         // counters of the group: ballots and warp sums instead of per-token updates
-        const bool in_need = (need0 >> lane) & 1u;
-        const unsigned sm = __ballot_sync(FULL, kind == BR_S), qm = __ballot_sync(FULL, kind == BR_Q);
-        const unsigned xm = __ballot_sync(FULL, kind == BR_MAX), rm = __ballot_sync(FULL, evaluated);
-        const uint32_t nnz_full = __reduce_add_sync(FULL, in_need ? my_nnz : 0u);
-        const uint32_t nnz_rows = __reduce_add_sync(FULL, evaluated ? my_nnz : 0u);
+        const unsigned sm = __ballot_sync(FULL, kind == BR_S), xm = __ballot_sync(FULL, kind == BR_MAX);
+        const uint32_t nnz_full = __reduce_add_sync(FULL, mine ? my_nnz : 0u);
+        const uint32_t nnz_rows = __reduce_add_sync(FULL, lead ? my_nnz : 0u);
         if (lane == 0) {
             ctr[C_TOK] += __popc(vmask);
             ctr[C_EA] += __popc(emask);
-            ctr[C_FULL] += __popc(need0);
+            ctr[C_FULL] += __popc(need);
             ctr[C_NNZ] += nnz_full;
             ctr[C_MAX] += __popc(xm) + __popc(emask);
             ctr[C_S] += __popc(sm);
             ctr[C_Q] += __popc(qm);
-            ctr[C_ROWS] += __popc(rm);
+            ctr[C_ROWS] += __popc(leaders);
             ctr[C_RENT] += nnz_rows;
         }
     }
@@ -692,49 +812,94 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
     return ll;
 }
 
+// Words of shared memory that a warp of the column samplers uses: its word column, its row
+// slots and its counter row, a multiple of 4 (the columns are 16-byte aligned).
+__host__ __device__ __forceinline__ int sample_warp_words(int K, int nslots) {
+    return col_words(K) + ((row_state_words(nslots) + 3) & ~3) + ((C_NUM + 3) & ~3);
+}
+
 // One sampler tile (tile index `tile` of a.tiles, content t) with the word column in the
-// warp's shared `col` (col_words(K) floats, skewed layout), the reciprocal table `r` and
-// the warp's shared counter row `ctr`.  QB: Q-bucket rounds decided per batch (1 for
-// K <= 1024, where a lane has one round of topics).
+// warp's shared `col` (col_words(K) floats, skewed layout), its row slots and its shared
+// counter row `ctr`.  QB: Q-bucket rounds decided per batch (1 for K <= 1024, where a lane
+// has one round of topics).  `clean`: whether `col` holds the column of a word without
+// tokens (a.base); a sparse word's column is that with the word's own topics written over
+// it, and a word with few of them puts the base values back when the tile is done, so that
+// the next sparse word costs its own entries instead of K.  (Forming every tile's column
+// anew cost 160 warp instructions at K=1024, where an average tile has 31 tokens on a
+// corpus of 14M tokens.)  Without a.base the column is formed in full from n_k.
 template <bool LL, int QB = 1, bool SKEWKEYS = true>
-__device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const int4 t, uint32_t iter,
-                                            const float* r, float* col, uint32_t* ctr, int lane) {
+__device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const int4 t, uint32_t iter, float* col,
+                                            float* slots, bool& clean, uint32_t* ctr, int lane) {
     using View = ColSharedT<SKEWKEYS>;
     const int w = t.x;
     const uint32_t start = (uint32_t)t.y, cnt = (uint32_t)t.z;
-    __syncwarp();
-    uint32_t wnnz = 0;
-    build_column<true>(col, r, w, a.Vd, a.K, a.beta, a.dwt, a.swt_off, a.swt_nnz, a.swt_ent, lane, &wnnz);
-    if (lane == 0) {
-        ctr[C_WNNZ] += wnnz;
-        ctr[w < a.Vd ? C_TDENSE : C_TSPARSE] += 1u;
-    }
+    const bool sparse = w >= a.Vd;
     const int maxK = (int)(__ldg(a.st_top2 + w) & 0xffffu);
     const float4 ph = __ldg(a.st_phi + w);
     const float QL = __ldg(a.st_ql + (size_t)w * 32 + lane);
+    const uint32_t* ent = a.swt_ent;
+    uint32_t nnz = 0;
+    if (sparse) {
+        ent += __ldg(a.swt_off + (w - a.Vd));
+        nnz = __ldg(a.swt_nnz + (w - a.Vd));
+    }
+    __syncwarp();
+    if (!sparse) {
+        const int* row = a.dwt + (size_t)w * a.K;
+        for (int k = lane; k < a.K; k += 32)
+            col[col_skew(k)] = fmul(fadd(__int2float_rn(__ldg(row + k)), a.beta), a.rk<SKEWKEYS>(k));
+        clean = false;
+    } else {
+        if (SKEWKEYS) {
+            if (!clean) {
+                const float4* src = reinterpret_cast<const float4*>(a.base);
+                for (int i = lane; i < col_words(a.K) / 4; i += 32) reinterpret_cast<float4*>(col)[i] = __ldg(src + i);
+            }
+        } else {
+            for (int k = lane; k < a.K; k += 32) col[col_skew(k)] = fmul(a.beta, a.rk<SKEWKEYS>(k));
+        }
+        __syncwarp();
+        for (uint32_t e = lane; e < nnz; e += 32) {
+            const uint32_t en = __ldg(ent + e);
+            const int k = (int)(en >> 16);
+            col[col_skew(k)] = fmul(fadd(u2f(en & 0xffffu), a.beta), a.rk<SKEWKEYS>(k));
+        }
+        clean = SKEWKEYS && nnz <= (uint32_t)a.K >> 3;
+    }
+    __syncwarp();
+    if (lane == 0) {
+        ctr[C_WNNZ] += nnz;
+        ctr[sparse ? C_TSPARSE : C_TDENSE] += 1u;
+        col[col_skew(maxK)] = 0.0f;
+    }
     const float QP = warp_ks_scan(QL, lane);
     const float Q = __shfl_sync(FULL, QP, 31);
-    if (lane == 0) col[col_skew(maxK)] = 0.0f;
     __syncwarp();
     double ll;
-    if constexpr (QB > 1) {
-        if (a.K > kLargeK && w >= a.Vd) {
-            // a sparse word above kLargeK topics: the split Q bucket
-            const int s = w - a.Vd;
-            const SplitQ sq{a.swt_ent + __ldg(a.swt_off + s), __ldg(a.swt_nnz + s), __shfl_sync(FULL, QL, 0),
-                            a.smooth, r, false};
-            ll = sample_groups<LL, QB, true>(a, start, cnt, 0u, 32u, iter, maxK, ph, QL, QP, Q, View{col}, ctr,
-                                             lane, nullptr, 0, &sq);
-        } else {
-            ll = sample_groups<LL, QB>(a, start, cnt, 0u, 32u, iter, maxK, ph, QL, QP, Q, View{col}, ctr, lane);
+    bool split = false;
+    if constexpr (QB > 1) split = a.K > kLargeK && sparse;
+    if (split) {
+        // a sparse word above kLargeK topics: the split Q bucket
+        if constexpr (QB > 1) {
+            const SplitQ sq{ent, nnz, __shfl_sync(FULL, QL, 0), a.smooth, a.recip, false, 0, 0.0f, 0.0f, a.n_k, a.Vbeta};
+            ll = sample_groups<LL, QB, true>(a, start, cnt, 0u, 32u, iter, maxK, ph, QL, QP, Q, View{col}, ctr, lane,
+                                             slots, nullptr, 0, &sq);
         }
     } else {
-        ll = sample_groups<LL, QB>(a, start, cnt, 0u, 32u, iter, maxK, ph, QL, QP, Q, View{col}, ctr, lane);
+        ll = sample_groups<LL, QB>(a, start, cnt, 0u, 32u, iter, maxK, ph, QL, QP, Q, View{col}, ctr, lane, slots);
     }
     if (LL) {
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) ll += __shfl_xor_sync(FULL, ll, off);
         if (lane == 0) a.tile_ll[tile] = ll;
+    }
+    if (clean) {
+        __syncwarp();
+        for (uint32_t e = lane; e < nnz; e += 32) {
+            const int i = col_skew((int)(__ldg(ent + e) >> 16));
+            col[i] = __ldg(a.base + i);
+        }
+        if (lane == 0) col[col_skew(maxK)] = __ldg(a.base + col_skew(maxK));
     }
 }
 

@@ -69,7 +69,11 @@ struct lda_trainer {
     cudaStream_t own_stream = nullptr, stream = nullptr;
     int K = 0, Vd = 0, C = 0, warps = 8, num_sms = 0;
     int swarps = 8;  // warps per CTA of the K <= 2048 sampler
-    float* recip = nullptr;  // [K] per-sweep reciprocals (K > kLargeK)
+    int dwarps = 8, pwarps = 8;  // warps per CTA of the large-K dense-word and sparse-word samplers
+    // row slots per warp of the K <= 2048 sampler (plain, LL) and of the large-K ones
+    int slots_sample = 1, slots_sample_ll = 1, slots_dense = 1, slots_sparse = 1;
+    float* recip = nullptr;  // [K] per-sweep reciprocals
+    float* base = nullptr;   // K <= kLargeK: the column of a word without tokens (SampleArgs::base)
     float* smooth = nullptr; // [K] per-sweep smoothing table of the split Q bucket (K > kLargeK)
     int* order = nullptr;    // [dev::kOrderList] per-sweep topic order of the sparse-word statistics (K > kLargeK)
     // K > kLargeK: the dense words' Q-round tables, [Vd][32 * qrounds] float2, built by the
@@ -108,7 +112,7 @@ struct lda_trainer {
     double* ll_host = nullptr;            // pinned
 
     int64_t dt_cap = 0, swt_cap = 0;
-    size_t smem_wt = 0, smem_stats = 0, smem_dt = 0, smem_sample = 0, smem_dense = 0, smem_sparse = 0;
+    size_t smem_wt = 0, smem_stats = 0, smem_dt = 0, smem_sample = 0, smem_sample_ll = 0, smem_dense = 0, smem_sparse = 0;
     size_t smem_stats_sparse = 0;
     int grid_wt_cta = 0, grid_dt_cta = 0, grid_totals = 0;  // K > kLargeK: the CTA-per-unit rebuilds
     int grid_stats_dense = 0;                                // K > kLargeK: dense-word statistics
@@ -357,6 +361,31 @@ static void launch_sample(bool ll, int K, int grid, int threads, size_t smem, cu
     }
 }
 
+// The row slots per warp of a sampler whose CTA takes bytes(slots) of shared memory: as many,
+// up to a group's 32, as leave the CTAs per SM that kMinRowSlots leave (a group whose rows do
+// not fit is taken in parts, each with a whole per-token part); fewer only where the shared
+// memory of one CTA asks for it.
+constexpr int kMinRowSlots = 8;
+template <class Bytes>
+static int pick_slots(const void* fn, int threads, int max_smem, const Bytes& bytes, int* slots, size_t* smem) {
+    int least = kMinRowSlots;
+    while (least > 1 && bytes(least) > (size_t)max_smem) --least;
+    if (bytes(least) > (size_t)max_smem)
+        return fail(LDA_ERR_ARG, "a sampler CTA needs %zu bytes of shared memory (max %d)", bytes(least), max_smem);
+    int most = 32;
+    while (most > least && bytes(most) > (size_t)max_smem) --most;
+    CUDA_TRY(raise_smem_limit(fn, bytes(most)));
+    int ctas = 0, n = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, fn, threads, bytes(least)));
+    for (; most > least; --most) {
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, bytes(most)));
+        if (n == ctas) break;
+    }
+    *slots = most;
+    *smem = bytes(most);
+    return LDA_OK;
+}
+
 extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* cfg, lda_trainer** out) {
     if (!c || !cfg || !out) return fail(LDA_ERR_ARG, "null argument");
     *out = nullptr;
@@ -400,19 +429,27 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     const int64_t row = (int64_t)T.K * 4;
     T.warps = (int)std::min<int64_t>(8, ((int64_t)max_smem - 2048) / (row + 256) - 1);
     if (T.warps < 1) return fail(LDA_ERR_ARG, "K=%d needs %lld bytes of shared memory per warp (max %d)", T.K, (long long)(2 * row), max_smem);
-    auto sample_bytes = [&](int w) { return (size_t)T.K * 4 + (size_t)w * (dev::col_words(T.K) * 4 + 16 * sizeof(uint32_t)); };
     T.large = T.K > dev::kLargeK;
+    int orc;
     if (!T.large) {
+        auto bytes = [&](int ns) { return (size_t)T.swarps * dev::sample_warp_words(T.K, ns) * 4; };
         T.swarps = dev::kSampleWarps;
-        while (T.swarps > 1 && sample_bytes(T.swarps) > (size_t)max_smem) --T.swarps;
-        if (sample_bytes(T.swarps) > (size_t)max_smem) return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory", T.K);
-        T.smem_sample = sample_bytes(T.swarps);
+        while (T.swarps > 1 && bytes(1) > (size_t)max_smem) --T.swarps;
+        if ((orc = pick_slots(sample_kernel(false, T.K), 32 * T.swarps, max_smem, bytes, &T.slots_sample, &T.smem_sample)) ||
+            (orc = pick_slots(sample_kernel(true, T.K), 32 * T.swarps, max_smem, bytes, &T.slots_sample_ll, &T.smem_sample_ll)))
+            return orc;
     } else {
-        T.smem_dense = dev::dense_large_smem(T.K, kLargeWarps);
-        T.smem_sparse = dev::sparse_large_smem(T.K, kLargeWarps);
-        if (T.smem_dense > (size_t)max_smem || T.smem_sparse > (size_t)max_smem)
+        auto dense_bytes = [&](int ns) { return dev::dense_large_smem(T.K, T.dwarps, ns); };
+        auto sparse_bytes = [&](int ns) { return dev::sparse_large_smem(T.K, T.pwarps, ns); };
+        T.dwarps = T.pwarps = kLargeWarps;
+        while (T.dwarps > 1 && dense_bytes(1) > (size_t)max_smem) --T.dwarps;
+        while (T.pwarps > 1 && sparse_bytes(1) > (size_t)max_smem) --T.pwarps;
+        if (dense_bytes(1) > (size_t)max_smem || sparse_bytes(1) > (size_t)max_smem)
             return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory (the dense-word sampler needs %zu bytes)", T.K,
-                        T.smem_dense);
+                        dense_bytes(1));
+        if ((orc = pick_slots(dense_large_kernel(false), 32 * T.dwarps, max_smem, dense_bytes, &T.slots_dense, &T.smem_dense)) ||
+            (orc = pick_slots(sparse_large_kernel(false), 32 * T.pwarps, max_smem, sparse_bytes, &T.slots_sparse, &T.smem_sparse)))
+            return orc;
     }
     T.smem_stats = (size_t)(T.warps + 1) * row;
     // the rebuilds' warp-private histograms hold 16-bit counts, two per word: a dense
@@ -458,15 +495,13 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     // kept within [kSampleTileMin, kSampleTile].
     int64_t resident_warps = 0, resident_dense = 0;
     if (T.large) {
-        CUDA_TRY(raise_smem_limit(dense_large_kernel(false), T.smem_dense));
-        int g = 0, orc = occupancy_grid(dense_large_kernel(false), 32 * kLargeWarps, T.smem_dense, T.num_sms, &g);
-        if (orc) return orc;
+        int g = 0;
+        if ((orc = occupancy_grid(dense_large_kernel(false), 32 * T.dwarps, T.smem_dense, T.num_sms, &g))) return orc;
         resident_dense = g;
     }
     if (!T.large) {
-        CUDA_TRY(raise_smem_limit(sample_kernel(false, T.K), T.smem_sample));
-        int g = 0, orc = occupancy_grid(sample_kernel(false, T.K), 32 * T.swarps, T.smem_sample, T.num_sms, &g);
-        if (orc) return orc;
+        int g = 0;
+        if ((orc = occupancy_grid(sample_kernel(false, T.K), 32 * T.swarps, T.smem_sample, T.num_sms, &g))) return orc;
         resident_warps = (int64_t)g * T.swarps;
     }
     std::vector<int4> st;
@@ -550,7 +585,8 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
         const int64_t resident = 4 * nb(N, 4) + nb(T.dt_cap, 4) + nb(N, 2) + nb(D + 1, 4) + 3 * nb(D, 4) +
                                  nb((int64_t)T.Vd * T.K, 4) + 2 * nb(std::max<int64_t>(Vs, 1), 4) + nb(T.swt_cap, 4) +
                                  nb(T.K, 4) + 2 * nb(V, 4) + nb(V, 16) + nb(V * 32, 4) + 2 * nb((int64_t)T.C * V, 4) +
-                                 nb(ns, 16) + nb(nw, 16) + nb(ns, 8) + nb(1, 8) + nb(3 + 2 * T.C, 4) + nb(kCounters, 8) + (T.large ? 2 * nb(T.K, 4) + nb(dev::kOrderList, 4) : 0) +
+                                 nb(ns, 16) + nb(nw, 16) + nb(ns, 8) + nb(1, 8) + nb(3 + 2 * T.C, 4) + nb(kCounters, 8) + nb(T.K, 4) +
+                                 (T.large ? nb(T.K, 4) + nb(dev::kOrderList, 4) : nb(dev::col_words(T.K), 4)) +
                                  (T.large && dev::qtab_rounds(T.K) > 0 && T.Vd > 0 ? nb((int64_t)T.Vd * 32 * dev::qtab_rounds(T.K), 8) : 0) +
                                  nb(1, 4);
         T.streaming = cfg->stream_mode == 2 || (cfg->stream_mode == 0 && T.budget > 0 && resident > T.budget);
@@ -598,7 +634,9 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     ALLOC(T.s_tiles, (int64_t)st.size()); ALLOC(T.w_tiles, (int64_t)wt.size());
     ALLOC(T.tile_ll, (int64_t)st.size()); ALLOC(T.ll_dev, 1);
     ALLOC(T.tile_ctr, 3 + 2 * T.C); ALLOC(T.ctr, kCounters); ALLOC(T.err, 1);
-    if (T.large) { ALLOC(T.recip, T.K); ALLOC(T.smooth, T.K); ALLOC(T.order, dev::kOrderList); }
+    ALLOC(T.recip, T.K);
+    if (T.large) { ALLOC(T.smooth, T.K); ALLOC(T.order, dev::kOrderList); }
+    else { ALLOC(T.base, dev::col_words(T.K)); }
     if (T.large && dev::qtab_rounds(T.K) > 0 && T.Vd > 0) {
         T.qrounds = dev::qtab_rounds(T.K);
         ALLOC(T.qtab_g, (int64_t)T.Vd * 32 * T.qrounds);
@@ -633,6 +671,8 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     CUDA_TRY(cudaMemset(T.st_phi, 0, sizeof(float4) * (size_t)V));
     CUDA_TRY(cudaMemset(T.st_ql, 0, sizeof(float) * 32 * (size_t)V));
     CUDA_TRY(cudaMemset(T.n_k, 0, sizeof(int) * (size_t)T.K));
+    CUDA_TRY(cudaMemset(T.recip, 0, sizeof(float) * (size_t)T.K));
+    if (T.base) CUDA_TRY(cudaMemset(T.base, 0, sizeof(float) * (size_t)dev::col_words(T.K)));
     CUDA_TRY(cudaMemset(T.err, 0, sizeof(int)));
     CUDA_TRY(cudaMemset(T.ctr, 0, sizeof(unsigned long long) * kCounters));
     CUDA_TRY(cudaMemset(T.tile_ll, 0, sizeof(double) * std::max<size_t>(st.size(), 1)));
@@ -688,21 +728,20 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
             return rc;
     }
     if (!T.large) {
-        for (bool ll : {false, true}) CUDA_TRY(raise_smem_limit(sample_kernel(ll, T.K), T.smem_sample));
         const int st = 32 * T.swarps;
         if ((rc = occupancy_grid(sample_kernel(false, T.K), st, T.smem_sample, T.num_sms, &T.grid_sample))) return rc;
-        if ((rc = occupancy_grid(sample_kernel(true, T.K), st, T.smem_sample, T.num_sms, &T.grid_sample_ll))) return rc;
+        if ((rc = occupancy_grid(sample_kernel(true, T.K), st, T.smem_sample_ll, T.num_sms, &T.grid_sample_ll))) return rc;
     } else {
-        const int lt = 32 * kLargeWarps;
+        const int lt = 32 * kLargeWarps, td = 32 * T.dwarps, tp = 32 * T.pwarps;
         int g0 = 0, g1 = 0, g2 = 0, g3 = 0;
         for (bool ll : {false, true}) {
             CUDA_TRY(raise_smem_limit(dense_large_kernel(ll), T.smem_dense));
             CUDA_TRY(raise_smem_limit(sparse_large_kernel(ll), T.smem_sparse));
         }
-        if ((rc = occupancy_grid(dense_large_kernel(false), lt, T.smem_dense, T.num_sms, &g0)) ||
-            (rc = occupancy_grid(dense_large_kernel(true), lt, T.smem_dense, T.num_sms, &g1)) ||
-            (rc = occupancy_grid(sparse_large_kernel(false), lt, T.smem_sparse, T.num_sms, &g2)) ||
-            (rc = occupancy_grid(sparse_large_kernel(true), lt, T.smem_sparse, T.num_sms, &g3)))
+        if ((rc = occupancy_grid(dense_large_kernel(false), td, T.smem_dense, T.num_sms, &g0)) ||
+            (rc = occupancy_grid(dense_large_kernel(true), td, T.smem_dense, T.num_sms, &g1)) ||
+            (rc = occupancy_grid(sparse_large_kernel(false), tp, T.smem_sparse, T.num_sms, &g2)) ||
+            (rc = occupancy_grid(sparse_large_kernel(true), tp, T.smem_sparse, T.num_sms, &g3)))
             return rc;
         T.grid_dense = std::min(g0, g1);
         T.grid_sparse = std::min(g2, g3);
@@ -905,11 +944,12 @@ extern "C" int lda_max_topic(lda_trainer* t) {
         a.V = t->wt_hi;
     }
     if (!t->large) {
-        if (a.V > a.wlo) {
-            const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(t->grid_stats, (a.V - a.wlo + t->warps - 1) / t->warps));
-            dev::k_word_stats<<<grid, 32 * t->warps, t->smem_stats, t->stream>>>(a);
-            CUDA_TRY(cudaGetLastError());
-        }
+        // (an empty word range still leaves the sampler its tables)
+        a.recip_out = t->recip;
+        a.base_out = t->base;
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(t->grid_stats, (a.V - a.wlo + t->warps - 1) / t->warps));
+        dev::k_word_stats<<<grid, 32 * t->warps, t->smem_stats, t->stream>>>(a);
+        CUDA_TRY(cudaGetLastError());
     } else {
         // the sweep's reciprocals (the sparse-word statistics and the dense-word sampler's
         // column builds read them), the smoothing table of the sparse words' split Q bucket,
@@ -1040,6 +1080,8 @@ static dev::SampleArgs sample_args(const lda_trainer* t, int chunk, int slot, in
     a.tok_base = b.tok_base;
     a.dt_base = b.dt_base;
     a.recip = t->recip;
+    a.base = t->base;
+    a.nslots = ll_mode ? t->slots_sample_ll : t->slots_sample;
     return a;
 }
 
@@ -1057,6 +1099,8 @@ static int sample_launch(lda_trainer* t, int chunk, int slot, int ll_mode, cudaS
         as.tile_counter = t->tile_ctr + 1 + t->C + chunk;
         CUDA_TRY(cudaMemsetAsync(ad.tile_counter, 0, sizeof(unsigned), q));
         CUDA_TRY(cudaMemsetAsync(as.tile_counter, 0, sizeof(unsigned), q));
+        ad.nslots = t->slots_dense;
+        as.nslots = t->slots_sparse;
         const bool ll = ll_mode != 0;
         // the sparse-word sampler on the side stream of q, so that its CTAs start as the
         // dense-word kernel's CTAs run out of tiles (both read only this chunk's doc rows)
@@ -1079,14 +1123,14 @@ static int sample_launch(lda_trainer* t, int chunk, int slot, int ll_mode, cudaS
         const cudaStream_t qs = side ? side->stream : q;
         if (nd > 0) {
             const int grid = std::max(1, std::min(t->grid_dense, nd));
-            if (ll) dev::k_sample_dense_large<true, 4><<<grid, 32 * kLargeWarps, t->smem_dense, q>>>(ad);
-            else dev::k_sample_dense_large<false, 4><<<grid, 32 * kLargeWarps, t->smem_dense, q>>>(ad);
+            if (ll) dev::k_sample_dense_large<true, 4><<<grid, 32 * t->dwarps, t->smem_dense, q>>>(ad);
+            else dev::k_sample_dense_large<false, 4><<<grid, 32 * t->dwarps, t->smem_dense, q>>>(ad);
             CUDA_TRY(cudaGetLastError());
         }
         if (ns > 0) {
-            const int grid = std::max(1, std::min(t->grid_sparse, (ns + kLargeWarps - 1) / kLargeWarps));
-            if (ll) dev::k_sample_sparse_large<true, 4><<<grid, 32 * kLargeWarps, t->smem_sparse, qs>>>(as);
-            else dev::k_sample_sparse_large<false, 4><<<grid, 32 * kLargeWarps, t->smem_sparse, qs>>>(as);
+            const int grid = std::max(1, std::min(t->grid_sparse, (ns + t->pwarps - 1) / t->pwarps));
+            if (ll) dev::k_sample_sparse_large<true, 4><<<grid, 32 * t->pwarps, t->smem_sparse, qs>>>(as);
+            else dev::k_sample_sparse_large<false, 4><<<grid, 32 * t->pwarps, t->smem_sparse, qs>>>(as);
             CUDA_TRY(cudaGetLastError());
         }
         if (side) {
@@ -1100,7 +1144,8 @@ static int sample_launch(lda_trainer* t, int chunk, int slot, int ll_mode, cudaS
     if (n > 0) {
         const int cap = a.ll_mode ? t->grid_sample_ll : t->grid_sample;
         const int grid = std::max(1, std::min(cap, (n + t->swarps - 1) / t->swarps));
-        launch_sample(a.ll_mode != 0, t->K, grid, 32 * t->swarps, t->smem_sample, q, a);
+        launch_sample(a.ll_mode != 0, t->K, grid, 32 * t->swarps,
+                      a.ll_mode ? t->smem_sample_ll : t->smem_sample, q, a);
         CUDA_TRY(cudaGetLastError());
     }
     t->chunk_sampled_ll[chunk] = ll_mode != 0;
@@ -1128,7 +1173,8 @@ static int sample_launch_group(lda_trainer* t, int c0, int c1, int ll_mode, cuda
     if (a.ntiles > 0) {
         const int cap = a.ll_mode ? t->grid_sample_ll : t->grid_sample;
         const int grid = std::max(1, std::min(cap, (a.ntiles + t->swarps - 1) / t->swarps));
-        launch_sample(a.ll_mode != 0, t->K, grid, 32 * t->swarps, t->smem_sample, q, a);
+        launch_sample(a.ll_mode != 0, t->K, grid, 32 * t->swarps,
+                      a.ll_mode ? t->smem_sample_ll : t->smem_sample, q, a);
         CUDA_TRY(cudaGetLastError());
     }
     for (int ch = c0; ch < c1; ++ch) t->chunk_sampled_ll[ch] = ll_mode != 0;
@@ -1777,9 +1823,8 @@ extern "C" int64_t lda_get_doc_rows(lda_trainer* t, int64_t* off, uint32_t* ent,
             if (n + hnnz[d] > cap) return fail(LDA_ERR_ARG, "doc-row buffer too small");
             const uint32_t* src = hent.data() + hoff[d];
             for (uint32_t j = 0; j < hnnz[d]; ++j) {
-                // up to kLargeK topics the device rows carry word-column slot indices
-                const uint32_t key = src[j] >> 16;
-                const uint32_t k = t->K <= dev::kLargeK ? (uint32_t)dev::col_unskew((int)key) : key;
+                // up to kLargeK topics the device rows carry word-column slot offsets
+                const uint32_t k = dev::row_topic(t->K, src[j] >> 16);
                 ent[n + j] = (k << 16) | (src[j] & 0xffffu);
             }
         }
@@ -1946,12 +1991,14 @@ extern "C" int lda_sample_chunk_noalloc(const lda_sample_io* io, int32_t device,
     const int64_t row = (int64_t)io->K * 4;
     const int warps = (int)std::min<int64_t>(std::min(8, dev::kSampleWarps), ((int64_t)max_smem - 2048) / (row + 256) - 1);
     if (warps < 1) return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory", io->K);
-    const size_t smem = (size_t)io->K * 4 + (size_t)warps * (dev::col_words(io->K) * 4 + 16 * sizeof(uint32_t));
-    if (warps < 1 || smem > (size_t)max_smem) return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory", io->K);
     const void* kfn = sample_kernel(io->ll_mode != 0, io->K, false);
-    CUDA_TRY(raise_smem_limit(kfn, smem));
-    int grid = 0;
-    if ((rc = occupancy_grid(kfn, 32 * warps, smem, num_sms, &grid))) return rc;
+    auto bytes = [&](int ns) { return (size_t)warps * dev::sample_warp_words(io->K, ns) * 4; };
+    if (bytes(1) > (size_t)max_smem) return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory", io->K);
+    int grid = 0, nslots = 1;
+    size_t smem = 0;
+    if ((rc = pick_slots(kfn, 32 * warps, max_smem, bytes, &nslots, &smem)) ||
+        (rc = occupancy_grid(kfn, 32 * warps, smem, num_sms, &grid)))
+        return rc;
     grid = std::max(1, std::min(grid, (io->num_tiles + warps - 1) / warps));
     dev::SampleArgs a;
     a.tiles = reinterpret_cast<const int4*>(io->tiles);
@@ -1970,6 +2017,7 @@ extern "C" int lda_sample_chunk_noalloc(const lda_sample_io* io, int32_t device,
     a.ctr = reinterpret_cast<unsigned long long*>(scratch + 8);
     a.tok_base = 0;
     a.dt_base = 0;
+    a.nslots = nslots;
     if (io->K > dev::kLargeK) {
         a.smooth = reinterpret_cast<const float*>(scratch + kNoAllocSmooth);
         dev::k_smooth_table<<<1, 1024, 0, st>>>(io->n_k, io->K, a.Vbeta, io->alpha, io->beta,
