@@ -80,29 +80,56 @@ __global__ void __launch_bounds__(256) kb_wt(BatchArgs b) {
     }
 }
 
-// Every model's reciprocals r_k = 1 / ((float)n_k + V*beta) and beta * r_k in the sampler's
-// column layout: block per model.  (The statistics and the sampler each formed them per
-// warp whenever the warp's next item was another model's.)  Also counts the sweep.
-__global__ void __launch_bounds__(256) kb_recip(const StatsArgs* st, uint32_t* sweeps_done) {
+// Every model's reciprocals, column of a word without tokens and topic order, as
+// k_recip_order forms them: block per model, Kmax floats of shared memory.  (The statistics
+// and the sampler each formed the reciprocals per warp whenever the warp's next item was
+// another model's.)  Also counts the sweep.
+struct RecipOut {
+    float* recip;
+    float* base;
+    int* order;
+};
+__global__ void __launch_bounds__(256) kb_recip(const StatsArgs* st, const RecipOut* out, uint32_t* sweeps_done) {
+    extern __shared__ float smf[];
     const StatsArgs& a = st[blockIdx.x];
+    const RecipOut o = out[blockIdx.x];
+    const int K = a.K;
     if (blockIdx.x == 0 && threadIdx.x == 0) *sweeps_done += 1u;
-    for (int k = threadIdx.x; k < a.K; k += blockDim.x) {
+    for (int k = threadIdx.x; k < K; k += blockDim.x) {
         const float r = __fdiv_rn(1.0f, fadd(__int2float_rn(a.n_k[k]), a.Vbeta));
-        a.recip_out[k] = r;
-        a.base_out[col_skew(k)] = fmul(a.beta, r);
+        const float v = fmul(a.beta, r);
+        smf[k] = v;
+        o.recip[k] = r;
+        o.base[col_skew(k)] = v;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < K; k += blockDim.x) {
+        const float v = smf[k];
+        int n = 0;
+#pragma unroll 4
+        for (int j = 0; j < K; ++j) n += ranks_above(smf[j], j, v, k) ? 1 : 0;
+        if (n < kOrderList) o.order[n] = k;
     }
 }
 
 __global__ void __launch_bounds__(256) kb_stats(BatchArgs b) {
     extern __shared__ float smf[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* col = smf + (size_t)b.Kmax * wid;
+    float* col = smf + (size_t)stats_warp_words(b.Kmax) * wid;
+    int cur = -1;
+    bool clean = false;
     for (;;) {
         const int i = grab(b.counters + 1, lane);
         if (i >= b.n_st) break;
         const uint4 u = b.st_work[i];
         const StatsArgs& a = b.st[u.x];
-        for (uint32_t w = u.y; w < u.y + u.z; ++w) word_stats_word(a, (int)w, a.recip, col, lane);
+        if ((int)u.x != cur) {
+            cur = (int)u.x;
+            clean = false;
+            __syncwarp();
+        }
+        uint32_t* bits = reinterpret_cast<uint32_t*>(col + ((a.K + 3) & ~3));
+        for (uint32_t w = u.y; w < u.y + u.z; ++w) word_stats_word(a, (int)w, col, bits, clean, lane);
     }
 }
 
@@ -232,6 +259,7 @@ struct lda_batch {
     DevBuf<dev::StatsArgs> stt;
     DevBuf<dev::DtArgs> dt;
     DevBuf<dev::SampleArgs> sm;
+    DevBuf<dev::RecipOut> rout;
     DevBuf<uint2> wt_work, sm_work;
     DevBuf<uint4> st_work, dt_work;
     DevBuf<dev::ZeroSeg> zero;
@@ -288,6 +316,7 @@ static int batch_build(lda_batch* b) {
     std::vector<dev::StatsArgs> stt(M);
     std::vector<dev::DtArgs> dt(M);
     std::vector<dev::SampleArgs> sm(M);
+    std::vector<dev::RecipOut> rout(M);
     const int nslots = b->Kmax <= 512 ? 32 : 16;
     std::vector<dev::ZeroSeg> zero;
     std::vector<int*> errs;
@@ -309,9 +338,7 @@ static int batch_build(lda_batch* b) {
         const TrainerView& v = b->views[m];
         wt[m] = v.wt;
         stt[m] = v.st;
-        stt[m].recip = v.sm.recip;
-        stt[m].recip_out = const_cast<float*>(v.sm.recip);
-        stt[m].base_out = const_cast<float*>(v.sm.base);
+        rout[m] = dev::RecipOut{const_cast<float*>(v.st.recip), const_cast<float*>(v.sm.base), const_cast<int*>(v.st.order)};
         dt[m] = v.dt;
         sm[m] = v.sm;
         sm[m].tiles = b->sub_tiles.p + sub_base[m];
@@ -354,12 +381,12 @@ static int batch_build(lda_batch* b) {
     }
     if ((rc = b->wt.put(wt)) || (rc = b->stt.put(stt)) || (rc = b->dt.put(dt)) || (rc = b->sm.put(sm)) ||
         (rc = b->wt_work.put(wt_work)) || (rc = b->sm_work.put(sm_work)) || (rc = b->st_work.put(st_work)) ||
-        (rc = b->dt_work.put(dt_work)) || (rc = b->zero.put(zero)) || (rc = b->errs.put(errs)))
+        (rc = b->dt_work.put(dt_work)) || (rc = b->rout.put(rout)) || (rc = b->zero.put(zero)) || (rc = b->errs.put(errs)))
         return rc;
     // launch shapes
     const int threads = 32 * tu.warps;
     b->smem_hist = (size_t)tu.warps * (b->Kmax + (b->Kmax + 31) / 32) * 4;
-    b->smem_stats = (size_t)tu.warps * b->Kmax * 4;
+    b->smem_stats = (size_t)tu.warps * dev::stats_warp_words(b->Kmax) * 4;
     b->smem_sample = (size_t)tu.warps * dev::sample_warp_words(b->Kmax, nslots) * 4;
     b->nslots = nslots;
     b->smem_dt = (size_t)tu.warps * (b->Kmax + (b->Kmax + 31) / 32) * 4;
@@ -404,7 +431,7 @@ static int enqueue_sweeps(lda_batch* b, int sweeps, int ll) {
         const bool last_ll = ll && s == sweeps - 1;
         dev::kb_zero<<<std::min<int>((int)b->zero.n, 4 * b->num_sms), 256, 0, b->st>>>(b->zero.p, (int)b->zero.n, b->counters);
         dev::kb_wt<<<grid_for(b->grid_wt, a.n_wt, W), threads, b->smem_hist, b->st>>>(a);
-        dev::kb_recip<<<M, 256, 0, b->st>>>(b->stt.p, b->sweeps_done);
+        dev::kb_recip<<<M, 256, sizeof(float) * (size_t)b->Kmax, b->st>>>(b->stt.p, b->rout.p, b->sweeps_done);
         dev::kb_stats<<<grid_for(b->grid_stats, a.n_st, W), threads, b->smem_stats, b->st>>>(a);
         dev::kb_dt<<<grid_for(b->grid_dt, a.n_dt, W), threads, b->smem_dt, b->st>>>(a);
         const int gs = last_ll ? grid_for(b->grid_sample_ll, a.n_sm, W) : grid_for(b->grid_sample, a.n_sm, W);

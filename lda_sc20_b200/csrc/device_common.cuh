@@ -149,41 +149,6 @@ __device__ __forceinline__ void hist_segment(const uint16_t* __restrict__ z, uin
 __host__ __device__ __forceinline__ int col_skew(int k) { return k + (k >> 5); }
 __host__ __device__ __forceinline__ int col_words(int K) { return (K + (K >> 5) + 4) & ~3; }
 
-// phi_k = ((float)n_wk + beta) * r_k into a warp-private shared row (EZLDA builds the
-// same column as WTHead, utility.cu:1257-1269 sparse, :1698-1702 dense).
-__device__ __forceinline__ void build_column(float* col, const float* r, int w, int Vd, int K, float beta,
-                                             const int* __restrict__ dwt, const uint32_t* __restrict__ swt_off,
-                                             const uint32_t* __restrict__ swt_nnz,
-                                             const uint32_t* __restrict__ swt_ent, int lane) {
-    if (w < Vd) {
-        const int* row = dwt + (size_t)w * K;
-        for (int k = lane; k < K; k += 32) col[k] = fmul(fadd(__int2float_rn(__ldg(row + k)), beta), r[k]);
-    } else {
-        for (int k = lane; k < K; k += 32) col[k] = fmul(beta, r[k]);
-        __syncwarp();
-        const int s = w - Vd;
-        const uint32_t off = __ldg(swt_off + s), nnz = __ldg(swt_nnz + s);
-        for (uint32_t e = lane; e < nnz; e += 32) {
-            const uint32_t en = __ldg(swt_ent + off + e);
-            const uint32_t k = en >> 16;
-            col[k] = fmul(fadd(u2f(en & 0xffffu), beta), r[k]);
-        }
-    }
-    __syncwarp();
-}
-
-__device__ __forceinline__ void warp_argmax(float& v, int& k) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const float ov = __shfl_xor_sync(FULL, v, off);
-        const int ok = __shfl_xor_sync(FULL, k, off);
-        if (ov > v || (ov == v && ok < k)) {
-            v = ov;
-            k = ok;
-        }
-    }
-}
-
 __device__ __forceinline__ void fill_recip(float* r, const int* __restrict__ n_k, int K, float Vbeta) {
     for (int k = threadIdx.x; k < K; k += blockDim.x) r[k] = __fdiv_rn(1.0f, fadd(__int2float_rn(n_k[k]), Vbeta));
 }

@@ -539,24 +539,46 @@ __global__ void __launch_bounds__(256, LDA_DT_SMALL_MIN_BLOCKS) k_dt_build_small
     }
 }
 
-// Word statistics: warp per word.  CTA 0 also leaves the reciprocals and the column of a
-// word without tokens for the sampler.
+// The sweep's reciprocals r_k = 1 / ((float)n_k + V*beta), up to kLargeK topics beta * r_k
+// in the sampler's column layout (base, else null), and the order of the topics outside a
+// word: the first kOrderList by (beta * r_k desc, k asc).  A CTA takes 32 topics.  A topic's
+// place in the order is the number of topics that rank above it, counted by the CTA's 8
+// warps against an eighth of all K each, so K^2 comparisons spread over ceil(K/32) CTAs.
+// (64 arg-max rounds of one CTA over the table took 239 us at K=10,000.)  K floats of
+// shared memory.
+__global__ void __launch_bounds__(256) k_recip_order(const int* __restrict__ n_k, int K, float Vbeta, float beta,
+                                                     float* recip, float* base, int* order) {
+    extern __shared__ float smf[];
+    __shared__ int above[32];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int k = threadIdx.x; k < K; k += blockDim.x)
+        smf[k] = fmul(beta, __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta)));
+    if (threadIdx.x < 32) above[threadIdx.x] = 0;
+    __syncthreads();
+    const int k = blockIdx.x * 32 + lane;
+    const float v = k < K ? smf[k] : 0.0f;
+    if (wid == 0 && k < K) {
+        recip[k] = __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta));
+        if (base) base[col_skew(k)] = v;
+    }
+    const int part = (K + 7) >> 3, j0 = wid * part, j1 = min(K, j0 + part);
+    int n = 0;
+#pragma unroll 8
+    for (int j = j0; j < j1; ++j) n += ranks_above(smf[j], j, v, k) ? 1 : 0;
+    atomicAdd(&above[lane], n);
+    __syncthreads();
+    if (wid == 0 && k < K && above[lane] < kOrderList) order[above[lane]] = k;
+}
+
+// Word statistics: warp per word.
 __global__ void __launch_bounds__(256) k_word_stats(StatsArgs a) {
     extern __shared__ float smf[];
     const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* r = smf;
-    float* col = smf + (size_t)a.K * (1 + wid);
-    fill_recip(r, a.n_k, a.K, a.Vbeta);
-    __syncthreads();
-    if (blockIdx.x == 0 && a.recip_out) {
-        for (int k = threadIdx.x; k < a.K; k += blockDim.x) {
-            a.recip_out[k] = r[k];
-            a.base_out[col_skew(k)] = fmul(a.beta, r[k]);
-        }
-    }
-    for (int w = a.wlo + blockIdx.x * warps + wid; w < a.V; w += gridDim.x * warps) {
-        word_stats_word(a, w, r, col, lane);
-    }
+    float* col = smf + (size_t)stats_warp_words(a.K) * wid;
+    uint32_t* bits = reinterpret_cast<uint32_t*>(col + ((a.K + 3) & ~3));
+    bool clean = false;
+    for (int w = a.wlo + blockIdx.x * warps + wid; w < a.V; w += gridDim.x * warps)
+        word_stats_word(a, w, col, bits, clean, lane);
 }
 
 // Word statistics of dense words above kLargeK topics: warp per word, phi formed on the fly
@@ -566,10 +588,9 @@ __global__ void __launch_bounds__(256) k_word_stats_dense_rows(StatsArgs a) {
     extern __shared__ float smf[];
     const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* r = smf;
-    fill_recip(r, a.n_k, a.K, a.Vbeta);
+    for (int k = threadIdx.x; k < a.K; k += blockDim.x) r[k] = __ldg(a.recip + k);
     __syncthreads();
-    for (int w = a.wlo + blockIdx.x * warps + wid; w < a.V; w += gridDim.x * warps)
-    {
+    for (int w = a.wlo + blockIdx.x * warps + wid; w < a.V; w += gridDim.x * warps) {
         const DenseRowPhi phi{a.dwt + (size_t)w * a.K, r, a.beta};
         const int k1 = word_stats_from(a, w, phi, lane);
         if (a.qtab) word_qtab(a, w, k1, phi, lane);
@@ -790,7 +811,7 @@ __global__ void __launch_bounds__(256, LDA_DENSE_LARGE_MIN_BLOCKS) k_sample_dens
         const int w = t.x;
         const int* wrow = a.dwt + (size_t)w * a.K;
         // phi_k = ((float)n_wk + beta) * r_k with r_k = 1 / ((float)n_k + V*beta), the values
-        // fill_recip and build_column form
+        // of the per-warp columns
         // the count row is read once per tile and chunk (800 MB per chunk on the K=10,000
         // corpus): evict_first, so that it displaces fewer of the chunk's doc rows in L2
         // (that corpus: samplers 116.1 -> 115.6 ms per sweep)
@@ -873,51 +894,11 @@ __global__ void __launch_bounds__(256, LDA_DENSE_LARGE_MIN_BLOCKS) k_sample_dens
 // other topics of the CTA's list of topics in decreasing beta * r_k (ties to the lower k),
 // and its split Q from its own entries and the smoothing table (Qw in st_ql slot 0, Qs in
 // slot 1).  Dense words keep k_word_stats.
-constexpr int kOrderList = 64;
-
-// (v, k) ranks above (a, i): larger value, ties to the lower topic.
-__device__ __forceinline__ bool ranks_above(float v, int k, float a, int i) { return v > a || (v == a && k < i); }
-
-__device__ __forceinline__ void top3_insert(float v, int k, float& a1, int& i1, float& a2, int& i2, float& a3, int& i3) {
-    if (ranks_above(v, k, a1, i1)) {
-        a3 = a2; i3 = i2;
-        a2 = a1; i2 = i1;
-        a1 = v; i1 = k;
-    } else if (ranks_above(v, k, a2, i2)) {
-        a3 = a2; i3 = i2;
-        a2 = v; i2 = k;
-    } else if (ranks_above(v, k, a3, i3)) {
-        a3 = v; i3 = k;
-    }
-}
-
 // Shared memory of the sparse-word statistics: the order list, then per warp the bitmap.
-// The reciprocals are read from the global table (k_recip), so that the CTA does not
+// The reciprocals are read from the global table (k_recip_order), so that the CTA does not
 // hold K of them and eight CTAs fit per SM.
 __host__ __device__ __forceinline__ size_t stats_sparse_smem(int K, int warps) {
     return kOrderList * 4 + (size_t)warps * (large_bit_words(K) * 4);
-}
-
-// The first kOrderList topics by (beta * r_k desc, k asc): a topic's place is the number of
-// topics that rank above it, counted against all K of them from the global reciprocal
-// table (k_recip).  A CTA ranks 32 topics, its 8 warps each against an eighth of the table,
-// so K^2 comparisons spread over ceil(K/32) CTAs.  (64 arg-max rounds of one CTA over the
-// table took 239 us at K=10,000.)
-__global__ void __launch_bounds__(256) k_sparse_order(StatsArgs a, int* order) {
-    __shared__ int above[32];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float* __restrict__ r = a.recip;
-    if (threadIdx.x < 32) above[threadIdx.x] = 0;
-    __syncthreads();
-    const int k = blockIdx.x * 32 + lane;
-    const float v = k < a.K ? fmul(a.beta, __ldg(r + k)) : 0.0f;
-    const int part = (a.K + 7) >> 3, j0 = wid * part, j1 = min(a.K, j0 + part);
-    int n = 0;
-#pragma unroll 8
-    for (int j = j0; j < j1; ++j) n += ranks_above(fmul(a.beta, __ldg(r + j)), j, v, k) ? 1 : 0;
-    atomicAdd(&above[lane], n);
-    __syncthreads();
-    if (wid == 0 && k < a.K && above[lane] < kOrderList) order[above[lane]] = k;
 }
 
 __global__ void __launch_bounds__(256) k_word_stats_sparse_large(StatsArgs a) {
@@ -944,46 +925,11 @@ __global__ void __launch_bounds__(256) k_word_stats_sparse_large(StatsArgs a) {
             top3_insert(fmul(fadd(u2f(en & 0xffffu), a.beta), r[k]), k, a1, i1, a2, i2, a3, i3);
         }
         __syncwarp();
-        // the best three topics outside the word: the first three of the CTA's order that
-        // the word lacks (lane j looks at entry j), or, if the list runs out, every topic
-        int found = 0, o0 = 0, o1 = 0, o2 = 0;
-        for (int b = 0; b < L && found < 3; b += 32) {
-            const int j = b + lane;
-            const int kj = j < L ? order[j] : 0;
-            const bool out = j < L && !((bits[kj >> 5] >> (kj & 31)) & 1u);
-            for (unsigned m = __ballot_sync(FULL, out); m && found < 3; m &= m - 1u) {
-                const int k = __shfl_sync(FULL, kj, __ffs(m) - 1);
-                if (found == 0) o0 = k;
-                else if (found == 1) o1 = k;
-                else o2 = k;
-                ++found;
-            }
-        }
-        if (found == 3) {
-            if (lane == 0) {
-                top3_insert(fmul(a.beta, r[o0]), o0, a1, i1, a2, i2, a3, i3);
-                top3_insert(fmul(a.beta, r[o1]), o1, a1, i1, a2, i2, a3, i3);
-                top3_insert(fmul(a.beta, r[o2]), o2, a1, i1, a2, i2, a3, i3);
-            }
-        } else {
-            for (int k = lane; k < a.K; k += 32)
-                if (!((bits[k >> 5] >> (k & 31)) & 1u)) top3_insert(fmul(a.beta, r[k]), k, a1, i1, a2, i2, a3, i3);
-        }
+        // with the best three topics outside the word
+        top3_outside(a, order, bits, a1, i1, a2, i2, a3, i3, lane);
         float v[3];
         int kk[3];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            float bv = a1;
-            int bk = i1;
-            warp_argmax(bv, bk);
-            v[q] = bv;
-            kk[q] = bk;
-            if (i1 == bk) {
-                a1 = a2; i1 = i2;
-                a2 = a3; i2 = i3;
-                a3 = -1.0f; i3 = 0x7fffffff;
-            }
-        }
+        warp_top3(a1, i1, a2, i2, a3, i3, v, kk);
         const int k1 = kk[0];
         // Q = Qw + Qs (the split Q bucket): Qw over the word's own topics in rounds of 32
         // entries (ascending k, the max topic's term 0), Qs = T[K-1] - sm_max
@@ -1016,7 +962,7 @@ __global__ void __launch_bounds__(256) k_word_stats_sparse_large(StatsArgs a) {
 // The smoothing table of the split Q bucket (K > kLargeK): T[k] = carry + Kogge-Stone scan
 // of sm_k = alpha * (beta * r_k) over rounds of 32 topics, the carry being the previous
 // round's last prefix, so T is non-decreasing and T[K-1] is the total.  r_k is formed from
-// n_k as fill_recip forms it.  One CTA: its warps scan the rounds in parallel (the scan of
+// n_k as k_recip_order forms it.  One CTA: its warps scan the rounds in parallel (the scan of
 // a round does not depend on the carry), one thread chains the carries, then every T[k] is
 // one addition.  T holds each round's scan until the carries are known.
 __global__ void __launch_bounds__(1024) k_smooth_table(const int* __restrict__ n_k, int K, float Vbeta, float alpha,
@@ -1042,12 +988,6 @@ __global__ void __launch_bounds__(1024) k_smooth_table(const int* __restrict__ n
     }
     __syncthreads();
     for (int k = threadIdx.x; k < K; k += blockDim.x) T[k] = fadd(carry_s[k >> 5], T[k]);
-}
-
-// r_k = 1 / ((float)n_k + V*beta), the value fill_recip forms, into a global table.
-__global__ void __launch_bounds__(256) k_recip(const int* __restrict__ n_k, int K, float Vbeta, float* r) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < K) r[k] = __fdiv_rn(1.0f, fadd(__int2float_rn(n_k[k]), Vbeta));
 }
 
 // Fixed-order FP64 reduction of the per-tile LL partials (one CTA of 1024 threads).

@@ -134,18 +134,83 @@ struct StatsArgs {
     float* st_ql;       // [V*32]
     const float* smooth = nullptr;  // K > kLargeK: the smoothing table (k_smooth_table)
     int wlo = 0;                    // the words [wlo, V) get statistics (a word range)
-    const float* recip = nullptr;   // r_k as fill_recip forms it
-    float* recip_out = nullptr;     // K <= kLargeK: where the statistics leave r_k ...
-    float* base_out = nullptr;      // ... and beta * r_k in the skewed column layout
-    const int* order = nullptr;     // K > kLargeK: the sparse words' topic order (k_sparse_order)
+    const float* recip = nullptr;   // r_k = 1 / ((float)n_k + V*beta) (k_recip_order)
+    const int* order = nullptr;     // the sparse words' topic order (k_recip_order)
     // K > kLargeK: the dense words' Q-round tables (32 lane slots x qrounds float2 per word,
     // the table k_sample_dense_large would build per tile), or null
     float2* qtab = nullptr;
     int qrounds = 0;
 };
 
-// Statistics of word w from its column (built into the warp's shared `col`).
-// phi_k of dense word w formed on the fly from its count row, the value build_column stores
+// Topics of the order list: the first kOrderList by (beta * r_k desc, k asc).
+constexpr int kOrderList = 64;
+
+// (v, k) ranks above (a, i): larger value, ties to the lower topic.
+__device__ __forceinline__ bool ranks_above(float v, int k, float a, int i) { return v > a || (v == a && k < i); }
+
+__device__ __forceinline__ void top3_insert(float v, int k, float& a1, int& i1, float& a2, int& i2, float& a3, int& i3) {
+    if (ranks_above(v, k, a1, i1)) {
+        a3 = a2; i3 = i2;
+        a2 = a1; i2 = i1;
+        a1 = v; i1 = k;
+    } else if (ranks_above(v, k, a2, i2)) {
+        a3 = a2; i3 = i2;
+        a2 = v; i2 = k;
+    } else if (ranks_above(v, k, a3, i3)) {
+        a3 = v; i3 = k;
+    }
+}
+
+// The warp's top three from its lanes' (value desc, topic asc) lists.  Values are -1 (an
+// empty place) or non-negative, so their bits order like signed integers.
+__device__ __forceinline__ void warp_top3(float a1, int i1, float a2, int i2, float a3, int i3, float (&v)[3],
+                                          int (&kk)[3]) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const int best = __reduce_max_sync(FULL, __float_as_int(a1));
+        const int bk = __reduce_min_sync(FULL, __float_as_int(a1) == best ? i1 : 0x7fffffff);
+        v[q] = __int_as_float(best);
+        kk[q] = bk;
+        if (i1 == bk) {
+            a1 = a2; i1 = i2;
+            a2 = a3; i2 = i3;
+            a3 = -1.0f; i3 = 0x7fffffff;
+        }
+    }
+}
+
+// The first three topics of the order list that a sparse word (bitmap `bits`) lacks, into
+// lane 0's top three; if the list runs out, every topic outside the word into the lanes'.
+__device__ __forceinline__ void top3_outside(const StatsArgs& a, const int* order, const uint32_t* bits, float& a1,
+                                             int& i1, float& a2, int& i2, float& a3, int& i3, int lane) {
+    const int L = min(kOrderList, a.K);
+    int found = 0, o0 = 0, o1 = 0, o2 = 0;
+    for (int b = 0; b < L && found < 3; b += 32) {
+        const int j = b + lane;
+        const int kj = j < L ? order[j] : 0;
+        const bool out = j < L && !((bits[kj >> 5] >> (kj & 31)) & 1u);
+        for (unsigned m = __ballot_sync(FULL, out); m && found < 3; m &= m - 1u) {
+            const int k = __shfl_sync(FULL, kj, __ffs(m) - 1);
+            if (found == 0) o0 = k;
+            else if (found == 1) o1 = k;
+            else o2 = k;
+            ++found;
+        }
+    }
+    if (found == 3) {
+        if (lane == 0) {
+            top3_insert(fmul(a.beta, __ldg(a.recip + o0)), o0, a1, i1, a2, i2, a3, i3);
+            top3_insert(fmul(a.beta, __ldg(a.recip + o1)), o1, a1, i1, a2, i2, a3, i3);
+            top3_insert(fmul(a.beta, __ldg(a.recip + o2)), o2, a1, i1, a2, i2, a3, i3);
+        }
+    } else {
+        for (int k = lane; k < a.K; k += 32)
+            if (!((bits[k >> 5] >> (k & 31)) & 1u))
+                top3_insert(fmul(a.beta, __ldg(a.recip + k)), k, a1, i1, a2, i2, a3, i3);
+    }
+}
+
+// phi_k of dense word w formed on the fly from its count row, the value its column holds
 struct DenseRowPhi {
     const int* row;
     const float* r;
@@ -164,9 +229,76 @@ struct ColumnPhi {
 template <class Phi>
 __device__ __forceinline__ int word_stats_from(const StatsArgs& a, int w, const Phi& phi, int lane);
 
-__device__ __forceinline__ void word_stats_word(const StatsArgs& a, int w, const float* r, float* col, int lane) {
-    build_column(col, r, w, a.Vd, a.K, a.beta, a.dwt, a.swt_off, a.swt_nnz, a.swt_ent, lane);
-    word_stats_from(a, w, ColumnPhi{col}, lane);
+// Words of shared memory a warp of the K <= kLargeK statistics uses: a word column (plain
+// layout) and a topic bitmap, a multiple of 4.
+__host__ __device__ __forceinline__ int stats_warp_words(int K) { return ((K + 3) & ~3) + ((((K + 31) >> 5) + 3) & ~3); }
+
+// Statistics of word w, K <= kLargeK; `col` and `bits` are the warp's (stats_warp_words).
+// phi_k = ((float)n_wk + beta) * r_k; EZLDA builds the same column as WTHead
+// (utility.cu:1257-1269 sparse, :1698-1702 dense).  A sparse word needs no pass over K
+// topics for its top three (its own topics, and the first three of the order list outside
+// it) and no column of its own: `col` keeps the column of a word without tokens while
+// `clean`, gets the word's topics written over it for the serial Q sums and put back after.
+// What is left per topic is one shared load and one fmaf (42 instructions before: 1,357 per
+// word at K=1024).
+__device__ __forceinline__ void word_stats_word(const StatsArgs& a, int w, float* col, uint32_t* bits, bool& clean,
+                                                int lane) {
+    const int K = a.K;
+    if (w < a.Vd) {
+        const int* row = a.dwt + (size_t)w * K;
+        for (int k = lane; k < K; k += 32)
+            col[k] = fmul(fadd(__int2float_rn(__ldg(row + k)), a.beta), __ldg(a.recip + k));
+        __syncwarp();
+        word_stats_from(a, w, ColumnPhi{col}, lane);
+        clean = false;
+        return;
+    }
+    const uint32_t* ent = a.swt_ent + __ldg(a.swt_off + (w - a.Vd));
+    const uint32_t nnz = __ldg(a.swt_nnz + (w - a.Vd));
+    if (!clean) {
+        for (int k = lane; k < K; k += 32) col[k] = fmul(a.beta, __ldg(a.recip + k));
+        for (int i = lane; i < (K + 31) >> 5; i += 32) bits[i] = 0u;
+        __syncwarp();
+    }
+    float a1 = -1.0f, a2 = -1.0f, a3 = -1.0f;
+    int i1 = 0x7fffffff, i2 = 0x7fffffff, i3 = 0x7fffffff;
+    for (uint32_t e = lane; e < nnz; e += 32) {
+        const uint32_t en = __ldg(ent + e);
+        const int k = (int)(en >> 16);
+        const float x = fmul(fadd(u2f(en & 0xffffu), a.beta), __ldg(a.recip + k));
+        atomicOr(&bits[k >> 5], 1u << (k & 31));
+        col[k] = x;
+        top3_insert(x, k, a1, i1, a2, i2, a3, i3);
+    }
+    __syncwarp();
+    top3_outside(a, a.order, bits, a1, i1, a2, i2, a3, i3, lane);
+    float v[3];
+    int kk[3];
+    warp_top3(a1, i1, a2, i2, a3, i3, v, kk);
+    const int k1 = kk[0];
+    if (lane == 0) col[k1] = 0.0f;  // fmaf(alpha, 0, q) is q: the max topic adds nothing
+    __syncwarp();
+    float ql = 0.0f;
+#pragma unroll 8
+    for (int k = lane; k < K; k += 32) ql = ffma(a.alpha, col[k], ql);
+    const float Q = __shfl_sync(FULL, warp_ks_scan(ql, lane), 31);
+    a.st_ql[(size_t)w * 32 + lane] = ql;
+    if (lane == 0) {
+        a.st_top2[w] = ((uint32_t)kk[1] << 16) | (uint32_t)k1;
+        a.st_k3[w] = (uint32_t)kk[2];
+        a.st_phi[w] = make_float4(v[0], v[1], v[2], Q);
+    }
+    __syncwarp();
+    clean = nnz <= (uint32_t)K >> 2;
+    if (clean) {
+        for (uint32_t e = lane; e < nnz; e += 32) {
+            const int k = (int)(__ldg(ent + e) >> 16);
+            col[k] = fmul(a.beta, __ldg(a.recip + k));
+            bits[k >> 5] = 0u;
+        }
+        if (lane == 0) col[k1] = fmul(a.beta, __ldg(a.recip + k1));
+        __syncwarp();
+    }
 }
 
 template <class Phi>
@@ -190,19 +322,7 @@ __device__ __forceinline__ int word_stats_from(const StatsArgs& a, int w, const 
     }
     float v[3];
     int kk[3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        float bv = a1;
-        int bk = i1;
-        warp_argmax(bv, bk);
-        v[r] = bv;
-        kk[r] = bk;
-        if (i1 == bk) {
-            a1 = a2; i1 = i2;
-            a2 = a3; i2 = i3;
-            a3 = -1.0f; i3 = 0x7fffffff;
-        }
-    }
+    warp_top3(a1, i1, a2, i2, a3, i3, v, kk);
     const float v1 = v[0], v2 = v[1], v3 = v[2];
     const int k1 = kk[0], k2 = kk[1], k3 = kk[2];
     float ql = 0.0f;

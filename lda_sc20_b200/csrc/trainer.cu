@@ -451,7 +451,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
             (orc = pick_slots(sparse_large_kernel(false), 32 * T.pwarps, max_smem, sparse_bytes, &T.slots_sparse, &T.smem_sparse)))
             return orc;
     }
-    T.smem_stats = (size_t)(T.warps + 1) * row;
+    T.smem_stats = (size_t)T.warps * dev::stats_warp_words(T.K) * 4;
     // the rebuilds' warp-private histograms hold 16-bit counts, two per word: a dense
     // word-topic tile has at most kWtTileMax tokens, a sparse word fewer than 65,536 and a doc at most
     // 65,535 (the corpus layout's limit), so every count fits.  Each rebuild takes as many
@@ -586,7 +586,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
                                  nb((int64_t)T.Vd * T.K, 4) + 2 * nb(std::max<int64_t>(Vs, 1), 4) + nb(T.swt_cap, 4) +
                                  nb(T.K, 4) + 2 * nb(V, 4) + nb(V, 16) + nb(V * 32, 4) + 2 * nb((int64_t)T.C * V, 4) +
                                  nb(ns, 16) + nb(nw, 16) + nb(ns, 8) + nb(1, 8) + nb(3 + 2 * T.C, 4) + nb(kCounters, 8) + nb(T.K, 4) +
-                                 (T.large ? nb(T.K, 4) + nb(dev::kOrderList, 4) : nb(dev::col_words(T.K), 4)) +
+                                 nb(dev::kOrderList, 4) + (T.large ? nb(T.K, 4) : nb(dev::col_words(T.K), 4)) +
                                  (T.large && dev::qtab_rounds(T.K) > 0 && T.Vd > 0 ? nb((int64_t)T.Vd * 32 * dev::qtab_rounds(T.K), 8) : 0) +
                                  nb(1, 4);
         T.streaming = cfg->stream_mode == 2 || (cfg->stream_mode == 0 && T.budget > 0 && resident > T.budget);
@@ -634,8 +634,8 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     ALLOC(T.s_tiles, (int64_t)st.size()); ALLOC(T.w_tiles, (int64_t)wt.size());
     ALLOC(T.tile_ll, (int64_t)st.size()); ALLOC(T.ll_dev, 1);
     ALLOC(T.tile_ctr, 3 + 2 * T.C); ALLOC(T.ctr, kCounters); ALLOC(T.err, 1);
-    ALLOC(T.recip, T.K);
-    if (T.large) { ALLOC(T.smooth, T.K); ALLOC(T.order, dev::kOrderList); }
+    ALLOC(T.recip, T.K); ALLOC(T.order, dev::kOrderList);
+    if (T.large) { ALLOC(T.smooth, T.K); }
     else { ALLOC(T.base, dev::col_words(T.K)); }
     if (T.large && dev::qtab_rounds(T.K) > 0 && T.Vd > 0) {
         T.qrounds = dev::qtab_rounds(T.K);
@@ -671,6 +671,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     CUDA_TRY(cudaMemset(T.st_phi, 0, sizeof(float4) * (size_t)V));
     CUDA_TRY(cudaMemset(T.st_ql, 0, sizeof(float) * 32 * (size_t)V));
     CUDA_TRY(cudaMemset(T.n_k, 0, sizeof(int) * (size_t)T.K));
+    CUDA_TRY(cudaMemset(T.order, 0, sizeof(int) * dev::kOrderList));
     CUDA_TRY(cudaMemset(T.recip, 0, sizeof(float) * (size_t)T.K));
     if (T.base) CUDA_TRY(cudaMemset(T.base, 0, sizeof(float) * (size_t)dev::col_words(T.K)));
     CUDA_TRY(cudaMemset(T.err, 0, sizeof(int)));
@@ -685,11 +686,14 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     const int threads = 32 * T.warps;
     const void* wt_fn = (const void*)dev::k_wt_build<true>;
     const void* dt_fn = (const void*)dev::k_dt_build<true>;
-    for (auto kv : {std::make_pair(wt_fn, T.smem_wt), std::make_pair((const void*)dev::k_word_stats, T.smem_stats),
+    for (auto kv : {std::make_pair(wt_fn, T.smem_wt), std::make_pair((const void*)dev::k_recip_order, (size_t)row),
                     std::make_pair(dt_fn, T.smem_dt)})
         CUDA_TRY(raise_smem_limit(kv.first, kv.second));
+    if (!T.large) CUDA_TRY(raise_smem_limit((const void*)dev::k_word_stats, T.smem_stats));
     if ((rc = occupancy_grid(wt_fn, 32 * T.warps_wt, T.smem_wt, T.num_sms, &T.grid_wt))) return rc;
-    if ((rc = occupancy_grid((const void*)dev::k_word_stats, threads, T.smem_stats, T.num_sms, &T.grid_stats))) return rc;
+    if (!T.large &&
+        (rc = occupancy_grid((const void*)dev::k_word_stats, threads, T.smem_stats, T.num_sms, &T.grid_stats)))
+        return rc;
     if ((rc = occupancy_grid(dt_fn, 32 * T.warps_dt, T.smem_dt, T.num_sms, &T.grid_dt))) return rc;
     if (T.large) {
         // the CTA-per-unit rebuilds: one shared histogram and bitmap (plus a sparse word's
@@ -876,6 +880,8 @@ static dev::StatsArgs stats_args(const lda_trainer* t) {
     a.n_k = t->n_k; a.dwt = t->dwt; a.swt_off = t->swt_off; a.swt_nnz = t->swt_nnz; a.swt_ent = t->swt_ent;
     a.st_top2 = t->st_top2; a.st_k3 = t->st_k3; a.st_phi = t->st_phi; a.st_ql = t->st_ql;
     a.smooth = t->smooth;
+    a.recip = t->recip;
+    a.order = t->order;
     return a;
 }
 
@@ -943,19 +949,19 @@ extern "C" int lda_max_topic(lda_trainer* t) {
         a.wlo = t->wt_lo;
         a.V = t->wt_hi;
     }
+    // the sweep's reciprocals and the topic order of the words' statistics
+    dev::k_recip_order<<<(t->K + 31) / 32, 256, sizeof(float) * (size_t)t->K, t->stream>>>(t->n_k, t->K, t->Vbeta, t->beta,
+                                                                                        t->recip, t->base, t->order);
+    CUDA_TRY(cudaGetLastError());
     if (!t->large) {
-        // (an empty word range still leaves the sampler its tables)
-        a.recip_out = t->recip;
-        a.base_out = t->base;
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(t->grid_stats, (a.V - a.wlo + t->warps - 1) / t->warps));
-        dev::k_word_stats<<<grid, 32 * t->warps, t->smem_stats, t->stream>>>(a);
-        CUDA_TRY(cudaGetLastError());
+        if (a.V > a.wlo) {
+            const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(t->grid_stats, (a.V - a.wlo + t->warps - 1) / t->warps));
+            dev::k_word_stats<<<grid, 32 * t->warps, t->smem_stats, t->stream>>>(a);
+            CUDA_TRY(cudaGetLastError());
+        }
     } else {
-        // the sweep's reciprocals (the sparse-word statistics and the dense-word sampler's
-        // column builds read them), the smoothing table of the sparse words' split Q bucket,
-        // then dense words from their count rows, sparse words from their entries
-        dev::k_recip<<<(t->K + 255) / 256, 256, 0, t->stream>>>(t->n_k, t->K, t->Vbeta, t->recip);
-        CUDA_TRY(cudaGetLastError());
+        // the smoothing table of the sparse words' split Q bucket, then dense words from
+        // their count rows, sparse words from their entries
         dev::k_smooth_table<<<1, 1024, 0, t->stream>>>(t->n_k, t->K, t->Vbeta, t->alpha, t->beta, t->smooth);
         CUDA_TRY(cudaGetLastError());
         dev::StatsArgs ad = a;
@@ -968,15 +974,10 @@ extern "C" int lda_max_topic(lda_trainer* t) {
             CUDA_TRY(cudaGetLastError());
         }
         if (a.V > std::max(t->Vd, a.wlo)) {
-            // sparse words: the topic order once, then warp per word from the global reciprocals
-            dev::StatsArgs as = a;
-            as.recip = t->recip;
-            as.order = t->order;
-            dev::k_sparse_order<<<(t->K + 31) / 32, 256, 0, t->stream>>>(as, t->order);
-            CUDA_TRY(cudaGetLastError());
+            // sparse words: warp per word from the global reciprocals
             const int64_t ns = a.V - std::max(t->Vd, a.wlo);
             const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(t->grid_stats_sparse, (ns + kLargeWarps - 1) / kLargeWarps));
-            dev::k_word_stats_sparse_large<<<grid, 32 * kLargeWarps, t->smem_stats_sparse, t->stream>>>(as);
+            dev::k_word_stats_sparse_large<<<grid, 32 * kLargeWarps, t->smem_stats_sparse, t->stream>>>(a);
             CUDA_TRY(cudaGetLastError());
         }
     }
