@@ -14,6 +14,31 @@
 namespace lda {
 namespace dev {
 
+// Tiles are claimed from a counter that stays zero between launches: every claimant (a warp
+// or a CTA) makes exactly one claim that finds no tile left, so the claimant that gets
+// ntiles + claimants - 1 is the last one of all and puts the counter back.  One thread of
+// the claimant calls it with what its claim returned.
+__device__ __forceinline__ void last_claim_resets(unsigned* counter, int got, int ntiles, int claimants) {
+    if (got == ntiles + claimants - 1) atomicExch(counter, 0u);
+}
+__device__ __forceinline__ int claim_warp(unsigned* counter, int ntiles, int lane) {
+    int tile = 0;
+    if (lane == 0) {
+        tile = (int)atomicAdd(counter, 1u);
+        last_claim_resets(counter, tile, ntiles, (int)(gridDim.x * (blockDim.x >> 5)));
+    }
+    return tile;  // lane 0's
+}
+
+// Zeroes the topic totals and the dense word-topic rows (n4 16-byte pieces of them, then the
+// rest) before a rebuild: one launch instead of a memset each.
+__global__ void __launch_bounds__(256) k_zero_counts(int* n_k, int K, int4* dwt, int64_t n4, int* rest, int nrest) {
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, st = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = i0; i < n4; i += st) dwt[i] = make_int4(0, 0, 0, 0);
+    for (int64_t i = i0; i < K; i += st) n_k[i] = 0;
+    if (i0 < nrest) rest[i0] = 0;
+}
+
 // Word-topic rebuild: warp per word tile, topic totals privatised per CTA.  P16: 16-bit
 // histogram counts (a dense tile holds at most 16,384 tokens and a sparse word fewer than
 // 65,536, so every count fits).
@@ -29,9 +54,7 @@ __global__ void __launch_bounds__(256) k_wt_build(WtArgs a) {
     for (int i = threadIdx.x; i < a.K + per * warps; i += blockDim.x) smu[i] = 0u;
     __syncthreads();
     for (;;) {
-        int tile = 0;
-        if (lane == 0) tile = (int)atomicAdd(a.tile_counter, 1u);
-        tile = __shfl_sync(FULL, tile, 0);
+        const int tile = __shfl_sync(FULL, claim_warp(a.tile_counter, a.ntiles, lane), 0);
         if (tile >= a.ntiles) break;
         const int4 t = a.tiles[tile];
         wt_tile(a, t, hist, bits, nk, lane);
@@ -148,7 +171,10 @@ __global__ void __launch_bounds__(kRebuildThreads, 8) k_wt_build_cta(WtArgs a) {
     for (int i = threadIdx.x; i < hw + bw; i += blockDim.x) smu[i] = 0u;
     for (;;) {
         __syncthreads();  // the previous tile is done with the shared state
-        if (threadIdx.x == 0) s_tile = (int)atomicAdd(a.tile_counter, 1u);
+        if (threadIdx.x == 0) {
+            s_tile = (int)atomicAdd(a.tile_counter, 1u);
+            last_claim_resets(a.tile_counter, s_tile, a.ntiles, (int)gridDim.x);
+        }
         __syncthreads();
         const int tile = s_tile;
         if (tile >= a.ntiles) break;
@@ -228,9 +254,7 @@ __global__ void __launch_bounds__(256) k_wt_sparse_small(WtArgs a) {
     for (int i = lane; i < kSmallSparse; i += 32) cnt[i] = 0u;
     __syncwarp();
     for (;;) {
-        int tile = 0;
-        if (lane == 0) tile = (int)atomicAdd(a.tile_counter, 1u);
-        tile = __shfl_sync(FULL, tile, 0);
+        const int tile = __shfl_sync(FULL, claim_warp(a.tile_counter, a.ntiles, lane), 0);
         if (tile >= a.ntiles) break;
         const int w = a.tiles[tile].x;
         // lane c: chunk c's segment of the word, as z index minus the segment's first rank
@@ -352,9 +376,7 @@ __global__ void __launch_bounds__(256) k_topic_totals(WtArgs a) {
         }
     };
     for (;;) {
-        int tile = 0;
-        if (lane == 0) tile = (int)atomicAdd(a.tile_counter, 1u);
-        tile = __shfl_sync(FULL, tile, 0);
+        const int tile = __shfl_sync(FULL, claim_warp(a.tile_counter, a.ntiles, lane), 0);
         if (tile >= a.ntiles) break;
         const int4 t = a.tiles[tile];
         if (t.w & 1) {
@@ -630,12 +652,9 @@ k_sample_t(SampleArgs a) {
     if (lane < C_NUM) ctr[lane] = 0u;
     __syncwarp();
     bool clean = false;
-    int tile = 0;
-    if (lane == 0) tile = (int)atomicAdd(a.tile_counter, 1u);
-    tile = __shfl_sync(FULL, tile, 0);
+    int tile = __shfl_sync(FULL, claim_warp(a.tile_counter, a.ntiles, lane), 0);
     while (tile < a.ntiles) {
-        int next = 0;
-        if (lane == 0) next = (int)atomicAdd(a.tile_counter, 1u);
+        const int next = claim_warp(a.tile_counter, a.ntiles, lane);
         sample_tile<LL, QB, SKEWKEYS>(a, tile, a.tiles[tile], a.iter, col, slots, clean, ctr, lane);
         tile = __shfl_sync(FULL, next, 0);
     }
@@ -734,13 +753,10 @@ __global__ void __launch_bounds__(256, LDA_SPARSE_LARGE_MIN_BLOCKS) k_sample_spa
     __syncthreads();
     // the next tile is claimed when a tile starts, so that the claim's round trip overlaps
     // the tile's work
-    int tile = 0;
-    if (lane == 0) tile = (int)atomicAdd(a.tile_counter, 1u);
-    tile = __shfl_sync(FULL, tile, 0);
+    int tile = __shfl_sync(FULL, claim_warp(a.tile_counter, a.ntiles, lane), 0);
     for (;;) {
         if (tile >= a.ntiles) break;
-        int next = 0;
-        if (lane == 0) next = (int)atomicAdd(a.tile_counter, 1u);
+        const int next = claim_warp(a.tile_counter, a.ntiles, lane);
         const int4 t = a.tiles[tile];
         const int w = t.x;
         const int s = w - a.Vd;
@@ -803,7 +819,10 @@ __global__ void __launch_bounds__(256, LDA_DENSE_LARGE_MIN_BLOCKS) k_sample_dens
     if (lane < C_NUM) ctr[lane] = 0u;
     __syncthreads();
     for (;;) {
-        if (threadIdx.x == 0) s_tile = (int)atomicAdd(a.tile_counter, 1u);
+        if (threadIdx.x == 0) {
+            s_tile = (int)atomicAdd(a.tile_counter, 1u);
+            last_claim_resets(a.tile_counter, s_tile, a.ntiles, (int)gridDim.x);
+        }
         __syncthreads();
         const int tile = s_tile;
         if (tile >= a.ntiles) break;

@@ -672,6 +672,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     CUDA_TRY(cudaMemset(T.st_ql, 0, sizeof(float) * 32 * (size_t)V));
     CUDA_TRY(cudaMemset(T.n_k, 0, sizeof(int) * (size_t)T.K));
     CUDA_TRY(cudaMemset(T.order, 0, sizeof(int) * dev::kOrderList));
+    CUDA_TRY(cudaMemset(T.tile_ctr, 0, sizeof(unsigned) * (size_t)(3 + 2 * T.C)));
     CUDA_TRY(cudaMemset(T.recip, 0, sizeof(float) * (size_t)T.K));
     if (T.base) CUDA_TRY(cudaMemset(T.base, 0, sizeof(float) * (size_t)dev::col_words(T.K)));
     CUDA_TRY(cudaMemset(T.err, 0, sizeof(int)));
@@ -889,19 +890,22 @@ extern "C" int lda_update_wt(lda_trainer* t) {
     if (!t) return fail(LDA_ERR_ARG, "null trainer");
     CUDA_TRY(cudaSetDevice(t->device));
     t->begin_stage(0);
-    CUDA_TRY(cudaMemsetAsync(t->n_k, 0, sizeof(int) * (size_t)t->K, t->stream));
     dev::WtArgs a = wt_args(t);
     if (t->w_tiles_rng) {
         // a word range: its dense rows, its sparse rows and its words' share of n_k
+        CUDA_TRY(cudaMemsetAsync(t->n_k, 0, sizeof(int) * (size_t)t->K, t->stream));
         const int64_t d0 = std::min<int64_t>(t->wt_lo, t->Vd), d1 = std::min<int64_t>(t->wt_hi, t->Vd);
         if (d1 > d0)
             CUDA_TRY(cudaMemsetAsync(t->dwt + d0 * t->K, 0, sizeof(int) * (size_t)(d1 - d0) * t->K, t->stream));
         a.tiles = t->w_tiles_rng;
         a.ntiles = t->n_wtiles_rng;
-    } else if (t->Vd > 0) {
-        CUDA_TRY(cudaMemsetAsync(t->dwt, 0, sizeof(int) * (size_t)t->Vd * t->K, t->stream));
+    } else {
+        const int64_t n = (int64_t)t->Vd * t->K;
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(8 * t->num_sms, (std::max<int64_t>(n / 4, t->K) + 255) / 256));
+        dev::k_zero_counts<<<grid, 256, 0, t->stream>>>(t->n_k, t->K, reinterpret_cast<int4*>(t->dwt), n / 4,
+                                                        t->dwt + n / 4 * 4, (int)(n % 4));
+        CUDA_TRY(cudaGetLastError());
     }
-    CUDA_TRY(cudaMemsetAsync(t->tile_ctr, 0, sizeof(unsigned), t->stream));
     if (t->large) {
         // rows by CTA per tile (small sparse words by warp per word), then the totals over
         // the same tiles
@@ -918,14 +922,12 @@ extern "C" int lda_update_wt(lda_trainer* t) {
             as.tiles = a.tiles + ab.ntiles;
             as.ntiles = nsmall;
             as.tile_counter = t->tile_ctr + 2 + 2 * t->C;
-            CUDA_TRY(cudaMemsetAsync(as.tile_counter, 0, sizeof(unsigned), t->stream));
             const int grid = std::max(1, std::min(t->grid_wsmall, (nsmall + 7) / 8));
             dev::k_wt_sparse_small<<<grid, 256, t->smem_wsmall, t->stream>>>(as);
             CUDA_TRY(cudaGetLastError());
         }
         dev::WtArgs at = a;
         at.tile_counter = t->tile_ctr + 1 + 2 * t->C;
-        CUDA_TRY(cudaMemsetAsync(at.tile_counter, 0, sizeof(unsigned), t->stream));
         const int gt = std::max(1, std::min(t->grid_totals, (a.ntiles + 7) / 8));
         if (t->smem_totals) dev::k_topic_totals<true><<<gt, 256, t->smem_totals, t->stream>>>(at);
         else dev::k_topic_totals<false><<<gt, 256, 0, t->stream>>>(at);
@@ -1098,8 +1100,6 @@ static int sample_launch(lda_trainer* t, int chunk, int slot, int ll_mode, cudaS
         as.tile_ll += nd;
         as.ntiles = ns;
         as.tile_counter = t->tile_ctr + 1 + t->C + chunk;
-        CUDA_TRY(cudaMemsetAsync(ad.tile_counter, 0, sizeof(unsigned), q));
-        CUDA_TRY(cudaMemsetAsync(as.tile_counter, 0, sizeof(unsigned), q));
         ad.nslots = t->slots_dense;
         as.nslots = t->slots_sparse;
         const bool ll = ll_mode != 0;
@@ -1141,7 +1141,6 @@ static int sample_launch(lda_trainer* t, int chunk, int slot, int ll_mode, cudaS
         t->chunk_sampled_ll[chunk] = ll;
         return LDA_OK;
     }
-    CUDA_TRY(cudaMemsetAsync(a.tile_counter, 0, sizeof(unsigned), q));
     if (n > 0) {
         const int cap = a.ll_mode ? t->grid_sample_ll : t->grid_sample;
         const int grid = std::max(1, std::min(cap, (n + t->swarps - 1) / t->swarps));
@@ -1170,7 +1169,6 @@ static int sample_launch_group(lda_trainer* t, int c0, int c1, int ll_mode, cuda
     }
     dev::SampleArgs a = sample_args(t, c0, 0, ll_mode);
     a.ntiles = t->s_tile_base[c1] - t->s_tile_base[c0];
-    CUDA_TRY(cudaMemsetAsync(a.tile_counter, 0, sizeof(unsigned), q));
     if (a.ntiles > 0) {
         const int cap = a.ll_mode ? t->grid_sample_ll : t->grid_sample;
         const int grid = std::max(1, std::min(cap, (a.ntiles + t->swarps - 1) / t->swarps));
