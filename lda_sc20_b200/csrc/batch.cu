@@ -293,10 +293,13 @@ struct lda_batch {
     }
 };
 
-// Batched sampler instantiation: Q-bucket rounds four per batch when some model has K > 1024.
-static const void* batch_sample_kernel(bool ll, int Kmax) {
-    if (Kmax > 1024) return ll ? (const void*)dev::kb_sample<true, 4> : (const void*)dev::kb_sample<false, 4>;
-    return ll ? (const void*)dev::kb_sample<true, 1> : (const void*)dev::kb_sample<false, 1>;
+// Batched sampler instantiation: thread-per-token Q draws when every model has at most
+// kThreadQTopics topics, Q-bucket rounds four per batch when some model has K > 1024.
+using BatchKernel = void (*)(dev::BatchArgs);
+static BatchKernel batch_sample_kernel(bool ll, int Kmax) {
+    if (Kmax > 1024) return ll ? dev::kb_sample<true, 4> : dev::kb_sample<false, 4>;
+    if (Kmax > dev::kThreadQTopics) return ll ? dev::kb_sample<true, 1> : dev::kb_sample<false, 1>;
+    return ll ? dev::kb_sample<true, 0> : dev::kb_sample<false, 0>;
 }
 
 static int occupancy(const void* fn, int threads, size_t smem, int num_sms, int* grid) {
@@ -393,8 +396,8 @@ static int batch_build(lda_batch* b) {
     if ((rc = occupancy((const void*)dev::kb_wt, threads, b->smem_hist, b->num_sms, &b->grid_wt)) ||
         (rc = occupancy((const void*)dev::kb_stats, threads, b->smem_stats, b->num_sms, &b->grid_stats)) ||
         (rc = occupancy((const void*)dev::kb_dt, threads, b->smem_dt, b->num_sms, &b->grid_dt)) ||
-        (rc = occupancy(batch_sample_kernel(false, b->Kmax), threads, b->smem_sample, b->num_sms, &b->grid_sample)) ||
-        (rc = occupancy(batch_sample_kernel(true, b->Kmax), threads, b->smem_sample, b->num_sms, &b->grid_sample_ll)))
+        (rc = occupancy((const void*)batch_sample_kernel(false, b->Kmax), threads, b->smem_sample, b->num_sms, &b->grid_sample)) ||
+        (rc = occupancy((const void*)batch_sample_kernel(true, b->Kmax), threads, b->smem_sample, b->num_sms, &b->grid_sample_ll)))
         return rc;
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
@@ -435,13 +438,7 @@ static int enqueue_sweeps(lda_batch* b, int sweeps, int ll) {
         dev::kb_stats<<<grid_for(b->grid_stats, a.n_st, W), threads, b->smem_stats, b->st>>>(a);
         dev::kb_dt<<<grid_for(b->grid_dt, a.n_dt, W), threads, b->smem_dt, b->st>>>(a);
         const int gs = last_ll ? grid_for(b->grid_sample_ll, a.n_sm, W) : grid_for(b->grid_sample, a.n_sm, W);
-        if (b->Kmax > 1024) {
-            if (last_ll) dev::kb_sample<true, 4><<<gs, threads, b->smem_sample, b->st>>>(a);
-            else dev::kb_sample<false, 4><<<gs, threads, b->smem_sample, b->st>>>(a);
-        } else {
-            if (last_ll) dev::kb_sample<true, 1><<<gs, threads, b->smem_sample, b->st>>>(a);
-            else dev::kb_sample<false, 1><<<gs, threads, b->smem_sample, b->st>>>(a);
-        }
+        batch_sample_kernel(last_ll, b->Kmax)<<<gs, threads, b->smem_sample, b->st>>>(a);
         if (last_ll) dev::kb_ll<<<M, 1024, 0, b->st>>>(b->sm.p, b->ll_dev);
         CUDA_TRY(cudaGetLastError());
         b->kernel_launches += last_ll ? 8 : 7;

@@ -674,28 +674,20 @@ constexpr int kSampleWarps = LDA_SAMPLE_WARPS;
 // row at [33 s, 33 s + 32), so that 32 threads reading element i of 32 different rows touch
 // 32 banks.
 constexpr int kSlotWords = 33;
+// Up to this many topics Q-bucket draws run thread per token (QB 0, thread_q_draw).
+constexpr int kThreadQTopics = 256;
 // Words of a warp's row slots, even (the rows' list, 32 x {offset, length}, follows them).
 __host__ __device__ __forceinline__ int slot_words(int nslots) { return (kSlotWords * nslots + 1) & ~1; }
 __host__ __device__ __forceinline__ int row_state_words(int nslots) { return slot_words(nslots) + 64; }
 
-// A warp's search for the S bucket's lane, for one token (the whole warp works on it): the
-// first lane whose prefix exceeds tt and whose sum is positive, else the last lane with a
-// positive sum.
-__device__ __forceinline__ int warp_s_lane(float SL, float tt, int lane, float& prev) {
-    const float SP = warp_ks_scan(SL, lane);
-    const unsigned cand = __ballot_sync(FULL, tt < SP && SL > 0.0f), pos = __ballot_sync(FULL, SL > 0.0f);
-    const int ls = cand ? __ffs(cand) - 1 : 31 - __clz(pos);
-    prev = __shfl_sync(FULL, SP, ls > 0 ? ls - 1 : 0);
-    return ls;
-}
-
-// The Kogge-Stone scan of 32 values held by one thread: element l adds element l - off at
-// each step off = 1, 2, ..., 16, the additions of warp_ks_scan.
-__device__ __forceinline__ void thread_ks_scan(float (&v)[32]) {
+// The Kogge-Stone scan of N values held by one thread: element l adds element l - off at
+// each step off = 1, 2, ..., the additions of warp_ks_scan's first N lanes.
+template <int N>
+__device__ __forceinline__ void thread_ks_scan(float (&v)[N]) {
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
+    for (int off = 1; off < N; off <<= 1) {
 #pragma unroll
-        for (int l = 31; l >= off; --l) v[l] = fadd(v[l], v[l - off]);
+        for (int l = N - 1; l >= off; --l) v[l] = fadd(v[l], v[l - off]);
     }
 }
 
@@ -723,6 +715,152 @@ __device__ __forceinline__ void thread_crossing(const float (&v)[32], float t, i
         for (int i = 0; i < h; ++i) w[i] = up ? w[h + i] : w[i];
     }
     sure = t < w[0] && !(t < fmul(prev, 1.0f + 0x1p-19f));
+}
+
+// What a group's tokens drew so far: the branch, and for the S bucket the lane and the rest
+// of the target inside it, for the Q bucket the rest of the target.
+struct Draw {
+    int kind;
+    uint32_t ls;
+    float t;
+    float total;  // LL mode: S + Q + the max topic's term
+};
+
+// Fewest tokens that decide_tokens takes thread per token: below, the whole warp decides
+// them one by one (about 45 warp instructions each against 280).
+#ifndef LDA_DECIDE_MIN
+#define LDA_DECIDE_MIN 3
+#endif
+constexpr int kDecideMin = LDA_DECIDE_MIN;
+
+// The tokens (lane = token, those with `act`) whose doc row's lane sums sit in slot my_s of
+// `slots`: S from the row's 32 sums, the branch, and for an S-bucket draw the lane: the
+// first whose prefix exceeds the target and whose sum is positive, else the last with a
+// positive sum.  Thread per token, each scanning its row's sums in registers and searching
+// the prefixes; a token whose search is not sure, and all of a few tokens, are decided by
+// the whole warp.
+template <bool LL>
+__device__ __forceinline__ void decide_tokens(const float* slots, int my_s, bool act, bool ea, float pmax, float Q,
+                                              float u, int lane, Draw& dr) {
+    unsigned by_warp = __ballot_sync(FULL, act);
+    if (__popc(by_warp) >= kDecideMin) {
+        const float* p = slots + kSlotWords * my_s;
+        float v[32];
+#pragma unroll
+        for (int l = 0; l < 32; ++l) v[l] = p[l];
+        thread_ks_scan(v);
+        const float pS = fadd(pmax, v[31]);
+        const float total = fadd(pS, Q);
+        const float target = fmul(u, total);
+        const float tt = fsub(target, pmax);
+        int ls;
+        float prev;
+        bool sure;
+        thread_crossing(v, tt, ls, prev, sure);
+        bool slow = false;
+        if (act) {
+            if (LL) dr.total = total;
+            if (!LL || !ea) {
+                if (target < pmax) {
+                    dr.kind = BR_MAX;
+                } else if (target < pS) {
+                    dr.kind = BR_S;
+                    dr.ls = (uint32_t)ls;
+                    dr.t = ls > 0 ? fsub(tt, prev) : tt;
+                    slow = !sure || !(p[ls] > 0.0f);
+                } else {
+                    dr.kind = BR_Q;
+                    dr.t = fsub(target, pS);
+                }
+            }
+        }
+        by_warp = __ballot_sync(FULL, slow);
+    }
+    for (; by_warp; by_warp &= by_warp - 1u) {
+        const int j = __ffs(by_warp) - 1;
+        const float SL = slots[kSlotWords * __shfl_sync(FULL, my_s, j) + lane];
+        const float SP = warp_ks_scan(SL, lane);
+        const float pmj = __shfl_sync(FULL, pmax, j);
+        const float pS = fadd(pmj, __shfl_sync(FULL, SP, 31));
+        const float total = fadd(pS, __shfl_sync(FULL, Q, j));
+        const float target = fmul(__shfl_sync(FULL, u, j), total);
+        const float tt = fsub(target, pmj);
+        const unsigned cand = __ballot_sync(FULL, tt < SP && SL > 0.0f), pos = __ballot_sync(FULL, SL > 0.0f);
+        const int ls = cand ? __ffs(cand) - 1 : 31 - __clz(pos);
+        const float prev = __shfl_sync(FULL, SP, ls > 0 ? ls - 1 : 0);
+        if (lane == j) {
+            if (LL) dr.total = total;
+            if (!LL || !ea) {
+                const bool s = target < pS;
+                dr.kind = target < pmj ? BR_MAX : (s ? BR_S : BR_Q);
+                dr.ls = (uint32_t)ls;
+                dr.t = s ? (ls > 0 ? fsub(tt, prev) : tt) : fsub(target, pS);
+            }
+        }
+    }
+}
+
+// A Q-bucket draw of a word by its column, for the rest tt of the target (the whole warp
+// works on one token): the lane from the word's Q partials, then one of its topics.
+template <int QB, class View>
+__device__ __forceinline__ int warp_q_draw(const View& colz, float tt, float QL, float QP, int K, float alpha, int maxK,
+                                           int lane, const float2* qtab, int qrounds) {
+    const unsigned cand = __ballot_sync(FULL, tt < QP && QL > 0.0f);
+    const unsigned pos = __ballot_sync(FULL, QL > 0.0f);
+    const int ls = cand ? __ffs(cand) - 1 : (pos ? 31 - __clz(pos) : 0);
+    const float prev = __shfl_sync(FULL, QP, ls > 0 ? ls - 1 : 0);
+    const float t2 = ls > 0 ? fsub(tt, prev) : tt;
+    const uint32_t n = (uint32_t)((K - ls + 31) / 32);
+    auto slot = [&](uint32_t i, int& key, float& term, bool& ok) {
+        const int k = ls + 32 * (int)i;
+        const float cz = colz(k);
+        key = k;
+        term = fmul(alpha, cz);
+        ok = cz > 0.0f;
+    };
+    int z = qtab ? warp_level2_table(n, t2, lane, slot, qtab + ls * qrounds) : -1;
+    if (z < 0) z = warp_level2_rounds<QB>(n, t2, maxK, lane, slot);
+    return z;
+}
+
+// Most topics for which a Q-bucket draw's second level is a thread's own search: a lane of Q
+// then has at most kThreadQ topics.  (A warp's draw takes 85 warp instructions per token, a
+// thread's about 130 per group, and a fifth of the draws are from Q at these sizes; with 32
+// topics per lane the thread's search costs as much as four tokens' draws by the warp.)
+constexpr int kThreadQ = kThreadQTopics / 32;
+
+// Q-bucket draws of all of a group's tokens with `act` (rest tt of the target each), thread
+// per token, for K <= 32 kThreadQ: the draws of warp_q_draw.  qps holds the word's 32 Q
+// prefixes, qpos the lanes with a positive partial.  `unsure` gets the tokens whose lane the
+// search could not be sure of (as thread_crossing).
+template <class View>
+__device__ __forceinline__ int thread_q_draw(const View& colz, const float* qps, unsigned qpos, float tt, int K,
+                                             float alpha, int maxK, bool& unsure) {
+    int ls = 0;
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1)
+        if (!(tt < qps[ls + h - 1])) ls += h;
+    // ls in 0..31: lane 31 is not probed, it is the answer when no other lane exceeds tt
+    const float prev = ls > 0 ? qps[ls - 1] : 0.0f;
+    unsure = !(tt < qps[ls]) || tt < fmul(prev, 1.0f + 0x1p-19f) || !((qpos >> ls) & 1u);
+    const float t2 = ls > 0 ? fsub(tt, prev) : tt;
+    float cz[kThreadQ], v[kThreadQ];
+#pragma unroll
+    for (int i = 0; i < kThreadQ; ++i) {
+        const int k = ls + 32 * i;
+        cz[i] = k < K ? colz(k) : 0.0f;
+        v[i] = fmul(alpha, cz[i]);
+    }
+    thread_ks_scan(v);
+    int first = -1, last = -1;
+#pragma unroll
+    for (int i = kThreadQ - 1; i >= 0; --i) {
+        const bool ok = cz[i] > 0.0f;
+        if (ok && t2 < v[i]) first = i;
+        if (ok && last < 0) last = i;
+    }
+    const int i = first >= 0 ? first : last;
+    return i >= 0 ? ls + 32 * i : maxK;
 }
 
 // The 32-token groups g0, g0 + gstep, ... of the token range [start, start + cnt) of one
@@ -757,6 +895,12 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
     const E* rows = reinterpret_cast<const E*>(a.dt_ent);
     const int nslots = a.nslots;
     uint2* list = reinterpret_cast<uint2*>(slots + slot_words(nslots));
+    float* qps = reinterpret_cast<float*>(ctr + ((C_NUM + 3) & ~3));  // QB 0: the word's Q prefixes
+    const unsigned qpos = __ballot_sync(FULL, QL > 0.0f);
+    if (QB == 0) {
+        qps[lane] = QP;
+        __syncwarp();
+    }
     uint32_t cur = 0xffffffffu;  // the doc of the last row summed, in slot cslot
     int cslot = 0;
     for (uint32_t g = gq ? claim() : g0; g < cnt; g = gq ? claim() : g + gstep) {
@@ -779,9 +923,7 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
             ea = fmul(u, bound) < pmax;
         }
         int znew = maxK;
-        uint32_t my_ls = 0;
-        float my_t = 0.0f, my_total = 0.0f;
-        int kind = BR_NONE;
+        Draw dr{BR_NONE, 0u, 0.0f, 0.0f};
         const unsigned vmask = __ballot_sync(FULL, valid);
         const unsigned emask = __ballot_sync(FULL, ea);
         const unsigned need = LL ? vmask : (vmask & ~emask);
@@ -820,88 +962,32 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
                 // the tokens of these rows, thread per token
                 const bool act = mine && (unsigned)(ri - r0) < (unsigned)n;
                 const int my_s = act ? ri - r0 : 0;
-                const float* p = slots + kSlotWords * my_s;
-                float tt;
-                bool slow = false;
-                {
-                    float v[32];
-#pragma unroll
-                    for (int l = 0; l < 32; ++l) v[l] = p[l];
-                    thread_ks_scan(v);
-                    const float pS = fadd(pmax, v[31]);
-                    const float total = fadd(pS, Q);
-                    const float target = fmul(u, total);
-                    tt = fsub(target, pmax);
-                    int ls;
-                    float prev;
-                    bool sure;
-                    thread_crossing(v, tt, ls, prev, sure);
-                    if (act) {
-                        if (LL) my_total = total;
-                        if (!LL || !ea) {
-                            if (target < pmax) {
-                                kind = BR_MAX;
-                            } else if (target < pS) {
-                                kind = BR_S;
-                                my_ls = (uint32_t)ls;
-                                my_t = ls > 0 ? fsub(tt, prev) : tt;
-                                slow = !sure || !(p[ls] > 0.0f);
-                            } else {
-                                kind = BR_Q;
-                                my_t = fsub(target, pS);
-                            }
-                        }
-                    }
-                }
-                // a token whose lane the search could not be sure of: with the whole warp
-                for (unsigned b = __ballot_sync(FULL, slow); b; b &= b - 1u) {
-                    const int j = __ffs(b) - 1;
-                    const float SL = slots[kSlotWords * __shfl_sync(FULL, my_s, j) + lane];
-                    const float ttj = __shfl_sync(FULL, tt, j);
-                    float prev;
-                    const int ls = warp_s_lane(SL, ttj, lane, prev);
-                    if (lane == j) {
-                        my_ls = (uint32_t)ls;
-                        my_t = ls > 0 ? fsub(ttj, prev) : ttj;
-                    }
-                }
+                decide_tokens<LL>(slots, my_s, act, ea, pmax, Q, u, lane, dr);
                 __syncwarp();  // the slots may be overwritten
             }
             cslot = (nrows - 1) % nslots;
             cur = __shfl_sync(FULL, d, 31 - __clz(need));
         }
-        const unsigned qm = __ballot_sync(FULL, kind == BR_Q);
-        for (unsigned b = qm; b; b &= b - 1u) {
-            const int j = __ffs(b) - 1;
-            const float tt = __shfl_sync(FULL, my_t, j);
+        const unsigned qm = __ballot_sync(FULL, dr.kind == BR_Q);
+        unsigned by_warp = qm;
+        if (QB == 0 && qm) {
+            bool unsure;
+            const int zq = thread_q_draw(colz, qps, qpos, dr.t, a.K, a.alpha, maxK, unsure);
+            if (dr.kind == BR_Q) znew = zq;
+            by_warp = __ballot_sync(FULL, dr.kind == BR_Q && unsure);
+        }
+        for (; by_warp; by_warp &= by_warp - 1u) {
+            const int j = __ffs(by_warp) - 1;
+            const float tt = __shfl_sync(FULL, dr.t, j);
             int zq;
-            if (SPLIT) {
-                zq = split_q_draw(*sq, tt, maxK, a.K, a.alpha, a.beta, lane);
-            } else {
-                const unsigned cand = __ballot_sync(FULL, tt < QP && QL > 0.0f);
-                const unsigned pos = __ballot_sync(FULL, QL > 0.0f);
-                const int ls = cand ? __ffs(cand) - 1 : (pos ? 31 - __clz(pos) : 0);
-                const float prev = __shfl_sync(FULL, QP, ls > 0 ? ls - 1 : 0);
-                const float t2 = ls > 0 ? fsub(tt, prev) : tt;
-                const int K = a.K;
-                const float alpha = a.alpha;
-                const uint32_t n = (uint32_t)((K - ls + 31) / 32);
-                auto slot = [&](uint32_t i, int& key, float& term, bool& ok) {
-                    const int k = ls + 32 * (int)i;
-                    const float cz = colz(k);
-                    key = k;
-                    term = fmul(alpha, cz);
-                    ok = cz > 0.0f;
-                };
-                zq = qtab ? warp_level2_table(n, t2, lane, slot, qtab + ls * qrounds) : -1;
-                if (zq < 0) zq = warp_level2_rounds<QB>(n, t2, maxK, lane, slot);
-            }
+            if (SPLIT) zq = split_q_draw(*sq, tt, maxK, a.K, a.alpha, a.beta, lane);
+            else zq = warp_q_draw<QB == 0 ? 1 : QB>(colz, tt, QL, QP, a.K, a.alpha, maxK, lane, qtab, qrounds);
             if (lane == j) znew = zq;
         }
         // each lane's own token's log-likelihood factors, all lanes at once (every lane
         // accumulates only its own tokens, in group order)
         if (LL && valid) {
-            ll_num *= (double)my_total;
+            ll_num *= (double)dr.total;
             ll_den *= (double)nd + a.den_add;
             if (++ll_n == 16 || ll_num < 1e-150 || ll_num > 1e150 || ll_den > 1e150) {
                 ll += log(ll_num / ll_den);
@@ -910,10 +996,10 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
             }
         }
         // an S-bucket token's row is its own doc's: the lane holds its offset and length
-        if (kind == BR_S) znew = lane_draw(rows + my_off, my_ls, my_nnz, colz, my_t, maxK);
+        if (dr.kind == BR_S) znew = lane_draw(rows + my_off, dr.ls, my_nnz, colz, dr.t, maxK);
         if (valid) a.z[tok] = (uint16_t)znew;
         // counters of the group: ballots and warp sums instead of per-token updates
-        const unsigned sm = __ballot_sync(FULL, kind == BR_S), xm = __ballot_sync(FULL, kind == BR_MAX);
+        const unsigned sm = __ballot_sync(FULL, dr.kind == BR_S), xm = __ballot_sync(FULL, dr.kind == BR_MAX);
         const uint32_t nnz_full = __reduce_add_sync(FULL, mine ? my_nnz : 0u);
         const uint32_t nnz_rows = __reduce_add_sync(FULL, lead ? my_nnz : 0u);
         if (lane == 0) {
@@ -933,9 +1019,10 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
 }
 
 // Words of shared memory that a warp of the column samplers uses: its word column, its row
-// slots and its counter row, a multiple of 4 (the columns are 16-byte aligned).
+// slots, its counter row and (QB 0) the word's Q prefixes, a multiple of 4 (the columns are
+// 16-byte aligned).
 __host__ __device__ __forceinline__ int sample_warp_words(int K, int nslots) {
-    return col_words(K) + ((row_state_words(nslots) + 3) & ~3) + ((C_NUM + 3) & ~3);
+    return col_words(K) + ((row_state_words(nslots) + 3) & ~3) + ((C_NUM + 3) & ~3) + (K <= kThreadQTopics ? 32 : 0);
 }
 
 // One sampler tile (tile index `tile` of a.tiles, content t) with the word column in the

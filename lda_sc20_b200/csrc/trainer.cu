@@ -316,19 +316,20 @@ static int occupancy_grid(const void* fn, int threads, size_t smem, int num_sms,
     return LDA_OK;
 }
 
-// The sampler instantiation for (LL mode, K): for K > 1024 a lane's Q-bucket topics span
-// several rounds, which are decided four per batch.
-static int sample_qb(int K) { return K > 1024 ? 4 : 1; }
-
-// skew: the doc rows' keys are word-column slot indices (the trainer's own rows); the
-// allocation-free entry point samples rows whose keys are topics.
-static const void* sample_kernel(bool ll, int K, bool skew = true) {
-    if (sample_qb(K) == 4) {
-        if (skew) return ll ? (const void*)dev::k_sample_t<true, 4, true> : (const void*)dev::k_sample_t<false, 4, true>;
-        return ll ? (const void*)dev::k_sample_t<true, 4, false> : (const void*)dev::k_sample_t<false, 4, false>;
+// The sampler instantiation for (LL mode, K, trainer's or caller's rows): up to
+// kThreadQTopics topics the trainer's Q-bucket draws run thread per token (QB 0); for K >
+// 1024 a lane's Q-bucket topics span several rounds, which are decided four per batch.
+// trainer: the trainer's own rows and tables; the allocation-free entry point's rows carry
+// topics as keys.
+using SampleKernel = void (*)(dev::SampleArgs);
+static SampleKernel sample_kernel(bool ll, int K, bool trainer = true) {
+    if (!trainer) {
+        if (K > 1024) return ll ? dev::k_sample_t<true, 4, false> : dev::k_sample_t<false, 4, false>;
+        return ll ? dev::k_sample_t<true, 1, false> : dev::k_sample_t<false, 1, false>;
     }
-    if (skew) return ll ? (const void*)dev::k_sample_t<true, 1, true> : (const void*)dev::k_sample_t<false, 1, true>;
-    return ll ? (const void*)dev::k_sample_t<true, 1, false> : (const void*)dev::k_sample_t<false, 1, false>;
+    if (K > 1024) return ll ? dev::k_sample_t<true, 4, true> : dev::k_sample_t<false, 4, true>;
+    if (K > dev::kThreadQTopics) return ll ? dev::k_sample_t<true, 1, true> : dev::k_sample_t<false, 1, true>;
+    return ll ? dev::k_sample_t<true, 0, true> : dev::k_sample_t<false, 0, true>;
 }
 
 // K > kLargeK: the dense-word (CTA per tile) and sparse-word (no column) samplers; a lane's
@@ -340,32 +341,14 @@ static const void* sparse_large_kernel(bool ll) {
     return ll ? (const void*)dev::k_sample_sparse_large<true, 4> : (const void*)dev::k_sample_sparse_large<false, 4>;
 }
 
-static void launch_sample(bool ll, int K, int grid, int threads, size_t smem, cudaStream_t q, const dev::SampleArgs& a,
-                          bool skew = true) {
-    if (sample_qb(K) == 4) {
-        if (skew) {
-            if (ll) dev::k_sample_t<true, 4, true><<<grid, threads, smem, q>>>(a);
-            else dev::k_sample_t<false, 4, true><<<grid, threads, smem, q>>>(a);
-        } else {
-            if (ll) dev::k_sample_t<true, 4, false><<<grid, threads, smem, q>>>(a);
-            else dev::k_sample_t<false, 4, false><<<grid, threads, smem, q>>>(a);
-        }
-    } else {
-        if (skew) {
-            if (ll) dev::k_sample_t<true, 1, true><<<grid, threads, smem, q>>>(a);
-            else dev::k_sample_t<false, 1, true><<<grid, threads, smem, q>>>(a);
-        } else {
-            if (ll) dev::k_sample_t<true, 1, false><<<grid, threads, smem, q>>>(a);
-            else dev::k_sample_t<false, 1, false><<<grid, threads, smem, q>>>(a);
-        }
-    }
-}
-
 // The row slots per warp of a sampler whose CTA takes bytes(slots) of shared memory: as many,
 // up to a group's 32, as leave the CTAs per SM that kMinRowSlots leave (a group whose rows do
 // not fit is taken in parts, each with a whole per-token part); fewer only where the shared
 // memory of one CTA asks for it.
-constexpr int kMinRowSlots = 8;
+#ifndef LDA_MIN_ROW_SLOTS
+#define LDA_MIN_ROW_SLOTS 8
+#endif
+constexpr int kMinRowSlots = LDA_MIN_ROW_SLOTS;
 template <class Bytes>
 static int pick_slots(const void* fn, int threads, int max_smem, const Bytes& bytes, int* slots, size_t* smem) {
     int least = kMinRowSlots;
@@ -435,8 +418,8 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
         auto bytes = [&](int ns) { return (size_t)T.swarps * dev::sample_warp_words(T.K, ns) * 4; };
         T.swarps = dev::kSampleWarps;
         while (T.swarps > 1 && bytes(1) > (size_t)max_smem) --T.swarps;
-        if ((orc = pick_slots(sample_kernel(false, T.K), 32 * T.swarps, max_smem, bytes, &T.slots_sample, &T.smem_sample)) ||
-            (orc = pick_slots(sample_kernel(true, T.K), 32 * T.swarps, max_smem, bytes, &T.slots_sample_ll, &T.smem_sample_ll)))
+        if ((orc = pick_slots((const void*)sample_kernel(false, T.K), 32 * T.swarps, max_smem, bytes, &T.slots_sample, &T.smem_sample)) ||
+            (orc = pick_slots((const void*)sample_kernel(true, T.K), 32 * T.swarps, max_smem, bytes, &T.slots_sample_ll, &T.smem_sample_ll)))
             return orc;
     } else {
         auto dense_bytes = [&](int ns) { return dev::dense_large_smem(T.K, T.dwarps, ns); };
@@ -501,7 +484,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     }
     if (!T.large) {
         int g = 0;
-        if ((orc = occupancy_grid(sample_kernel(false, T.K), 32 * T.swarps, T.smem_sample, T.num_sms, &g))) return orc;
+        if ((orc = occupancy_grid((const void*)sample_kernel(false, T.K), 32 * T.swarps, T.smem_sample, T.num_sms, &g))) return orc;
         resident_warps = (int64_t)g * T.swarps;
     }
     std::vector<int4> st;
@@ -734,8 +717,8 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     }
     if (!T.large) {
         const int st = 32 * T.swarps;
-        if ((rc = occupancy_grid(sample_kernel(false, T.K), st, T.smem_sample, T.num_sms, &T.grid_sample))) return rc;
-        if ((rc = occupancy_grid(sample_kernel(true, T.K), st, T.smem_sample_ll, T.num_sms, &T.grid_sample_ll))) return rc;
+        if ((rc = occupancy_grid((const void*)sample_kernel(false, T.K), st, T.smem_sample, T.num_sms, &T.grid_sample))) return rc;
+        if ((rc = occupancy_grid((const void*)sample_kernel(true, T.K), st, T.smem_sample_ll, T.num_sms, &T.grid_sample_ll))) return rc;
     } else {
         const int lt = 32 * kLargeWarps, td = 32 * T.dwarps, tp = 32 * T.pwarps;
         int g0 = 0, g1 = 0, g2 = 0, g3 = 0;
@@ -1144,8 +1127,7 @@ static int sample_launch(lda_trainer* t, int chunk, int slot, int ll_mode, cudaS
     if (n > 0) {
         const int cap = a.ll_mode ? t->grid_sample_ll : t->grid_sample;
         const int grid = std::max(1, std::min(cap, (n + t->swarps - 1) / t->swarps));
-        launch_sample(a.ll_mode != 0, t->K, grid, 32 * t->swarps,
-                      a.ll_mode ? t->smem_sample_ll : t->smem_sample, q, a);
+        sample_kernel(a.ll_mode != 0, t->K)<<<grid, 32 * t->swarps, a.ll_mode ? t->smem_sample_ll : t->smem_sample, q>>>(a);
         CUDA_TRY(cudaGetLastError());
     }
     t->chunk_sampled_ll[chunk] = ll_mode != 0;
@@ -1172,8 +1154,7 @@ static int sample_launch_group(lda_trainer* t, int c0, int c1, int ll_mode, cuda
     if (a.ntiles > 0) {
         const int cap = a.ll_mode ? t->grid_sample_ll : t->grid_sample;
         const int grid = std::max(1, std::min(cap, (a.ntiles + t->swarps - 1) / t->swarps));
-        launch_sample(a.ll_mode != 0, t->K, grid, 32 * t->swarps,
-                      a.ll_mode ? t->smem_sample_ll : t->smem_sample, q, a);
+        sample_kernel(a.ll_mode != 0, t->K)<<<grid, 32 * t->swarps, a.ll_mode ? t->smem_sample_ll : t->smem_sample, q>>>(a);
         CUDA_TRY(cudaGetLastError());
     }
     for (int ch = c0; ch < c1; ++ch) t->chunk_sampled_ll[ch] = ll_mode != 0;
@@ -1990,13 +1971,13 @@ extern "C" int lda_sample_chunk_noalloc(const lda_sample_io* io, int32_t device,
     const int64_t row = (int64_t)io->K * 4;
     const int warps = (int)std::min<int64_t>(std::min(8, dev::kSampleWarps), ((int64_t)max_smem - 2048) / (row + 256) - 1);
     if (warps < 1) return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory", io->K);
-    const void* kfn = sample_kernel(io->ll_mode != 0, io->K, false);
+    const SampleKernel kfn = sample_kernel(io->ll_mode != 0, io->K, false);
     auto bytes = [&](int ns) { return (size_t)warps * dev::sample_warp_words(io->K, ns) * 4; };
     if (bytes(1) > (size_t)max_smem) return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory", io->K);
     int grid = 0, nslots = 1;
     size_t smem = 0;
-    if ((rc = pick_slots(kfn, 32 * warps, max_smem, bytes, &nslots, &smem)) ||
-        (rc = occupancy_grid(kfn, 32 * warps, smem, num_sms, &grid)))
+    if ((rc = pick_slots((const void*)kfn, 32 * warps, max_smem, bytes, &nslots, &smem)) ||
+        (rc = occupancy_grid((const void*)kfn, 32 * warps, smem, num_sms, &grid)))
         return rc;
     grid = std::max(1, std::min(grid, (io->num_tiles + warps - 1) / warps));
     dev::SampleArgs a;
@@ -2031,7 +2012,7 @@ extern "C" int lda_sample_chunk_noalloc(const lda_sample_io* io, int32_t device,
     chk.n_sp = io->num_sparse_entries; chk.status = io->status; chk.tile_counter = a.tile_counter;
     k_check_sample_io<<<4 * num_sms, 256, 0, st>>>(chk);
     CUDA_TRY(cudaGetLastError());
-    launch_sample(a.ll_mode != 0, io->K, grid, 32 * warps, smem, st, a, false);
+    kfn<<<grid, 32 * warps, smem, st>>>(a);
     CUDA_TRY(cudaGetLastError());
     if (io->ll_mode) {
         dev::k_ll_reduce<<<1, 1024, 0, st>>>(a.tile_ll, io->num_tiles, io->ll_sum);
