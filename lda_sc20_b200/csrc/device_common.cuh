@@ -295,6 +295,8 @@ __host__ __device__ __forceinline__ uint32_t row_topic(int K, uint32_t key) {
 template <bool SLOTKEYS>
 struct ColSharedT {
     using Entry = uint32_t;  // a doc-row entry: (key << 16) | count
+    // rows are loaded one ahead (row_load), which reads past their end
+    static constexpr bool kAhead = SLOTKEYS;
     const float* col;
     __device__ __forceinline__ float operator()(int k) const { return col[col_skew(k)]; }
     __device__ __forceinline__ float row(uint32_t key) const {
@@ -345,9 +347,8 @@ __device__ __forceinline__ float lane_steps(const typename View::Entry* __restri
 // loops with predicated ends took 100 warp instructions per row of 122 entries.
 template <class View>
 __device__ __forceinline__ float lane_mass(const typename View::Entry* __restrict__ row, uint32_t lane, uint32_t nnz,
-                                           const View& colz) {
+                                           const View& colz, float acc = 0.0f) {
     const typename View::Entry* __restrict__ p = row + lane;
-    float acc = 0.0f;
     for (; nnz > 128u; nnz -= 128u, p += 128) acc = lane_steps<4, false>(p, lane, 0u, colz, acc);
     if (nnz > 64u) {
         if (nnz > 96u) return lane_steps<4, true>(p, lane, nnz - 96u, colz, acc);
@@ -355,6 +356,42 @@ __device__ __forceinline__ float lane_mass(const typename View::Entry* __restric
     }
     if (nnz > 32u) return lane_steps<2, true>(p, lane, nnz - 32u, colz, acc);
     return lane_steps<1, true>(p, lane, nnz, colz, acc);
+}
+
+// lane_mass in two halves: the loads of a row's first four steps (two when it has no more),
+// and the sum.  The loads are not masked: they may read up to kRowSlack entries past the row,
+// whose values the sum leaves out.
+constexpr int kRowSlack = 128;
+__device__ __forceinline__ void row_load(uint32_t (&e)[4], const uint32_t* __restrict__ row, uint32_t lane,
+                                         uint32_t nnz) {
+    const uint32_t* __restrict__ p = row + lane;
+    e[0] = __ldg(p);
+    e[1] = __ldg(p + 32);
+    if (nnz > 64u) {
+        e[2] = __ldg(p + 64);
+        e[3] = __ldg(p + 96);
+    }
+}
+template <int N, class View>
+__device__ __forceinline__ float row_steps(const uint32_t (&e)[4], uint32_t lane, uint32_t left, const View& colz) {
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const uint32_t x = j < N - 1 || lane < left ? e[j] : 0u;
+        acc = ffma(colz.cnt(x), colz.row(colz.key(x)), acc);
+    }
+    return acc;
+}
+template <class View>
+__device__ __forceinline__ float row_sum(const uint32_t (&e)[4], const uint32_t* __restrict__ row, uint32_t lane,
+                                         uint32_t nnz, const View& colz) {
+    if (nnz <= 64u) {
+        if (nnz <= 32u) return row_steps<1>(e, lane, nnz, colz);
+        return row_steps<2>(e, lane, nnz - 32u, colz);
+    }
+    if (nnz <= 96u) return row_steps<3>(e, lane, nnz - 64u, colz);
+    const float acc = row_steps<4>(e, lane, nnz - 96u, colz);
+    return nnz > 128u ? lane_mass(row + 128, lane, nnz - 128u, colz, acc) : acc;
 }
 
 // The S-bucket draw among lane ls's entries ls, ls + 32, ... of the row: their serial

@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(256) k_dt_build(DtArgs a) {
 // and tables up to kLargeK topics).
 template <bool LL, int QB = 1, bool SKEWKEYS = true>
 __global__ void __launch_bounds__(32 * kSampleWarps, QB > 1 ? LDA_SAMPLE_QB_MIN_BLOCKS
-                                                       : (LL ? LDA_SAMPLE_LL_MIN_BLOCKS : LDA_SAMPLE_MIN_BLOCKS))
+                                                       : (!LL ? LDA_SAMPLE_MIN_BLOCKS : QB == 0 ? LDA_SAMPLE_LL0_MIN_BLOCKS : LDA_SAMPLE_LL_MIN_BLOCKS))
 k_sample_t(SampleArgs a) {
     extern __shared__ float smf[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -675,6 +675,7 @@ k_sample_t(SampleArgs a) {
 // word's row (ascending k), and phi_k is formed exactly as build_column forms it.
 struct ColBits {
     using Entry = uint32_t;  // a doc-row entry: (k << 16) | count
+    static constexpr bool kAhead = false;
     const uint32_t* bits;  // ceil(K/32) words
     const uint16_t* pre;   // set bits before each word
     const uint32_t* ent;   // the word's row, (k << 16) | count

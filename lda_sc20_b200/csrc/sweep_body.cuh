@@ -648,8 +648,11 @@ enum { C_TOK, C_EA, C_FULL, C_NNZ, C_MAX, C_S, C_Q, C_WNNZ, C_TDENSE, C_TSPARSE,
 
 // Warps per CTA of the K <= 2048 sampler (one shared word column per warp), and the CTAs
 // per SM it is compiled for: the register cap is 65536 / (32 * warps * blocks) per
-// thread.  The LL-mode kernel (its FP64 term) and the K > 1024 kernel (four Q rounds per
-// batch) keep more state live and are compiled for fewer.
+// thread.  A thread holds a row's 32 lane sums, so the plain kernels take 4 CTAs (64
+// registers; 5 CTAs of 48 spill: 1.96 against 1.92 ms per sweep at K=1024, and 3 leave too
+// few warps, 2.23 ms).  The K > 1024 kernels (four Q rounds per batch) and the LL kernel up
+// to kThreadQTopics (its FP64 products; K=64: 119 -> 109 us per sweep) take 3; above, the LL
+// kernel spills 22 bytes at 4 and is still faster (K=1024: 701 against 755 us).
 // Branch taken by a token (counters only).
 enum { BR_NONE = 0, BR_MAX = 1, BR_S = 2, BR_Q = 3 };
 
@@ -665,6 +668,9 @@ constexpr int kSampleWarps = LDA_SAMPLE_WARPS;
 #endif
 #ifndef LDA_SAMPLE_LL_MIN_BLOCKS
 #define LDA_SAMPLE_LL_MIN_BLOCKS 4
+#endif
+#ifndef LDA_SAMPLE_LL0_MIN_BLOCKS
+#define LDA_SAMPLE_LL0_MIN_BLOCKS 3
 #endif
 #ifndef LDA_SPARSE_LARGE_MIN_BLOCKS
 #define LDA_SPARSE_LARGE_MIN_BLOCKS 4
@@ -954,9 +960,32 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
                     i = c1;
                     out += kSlotWords * c1;
                 }
-                for (; i < n; ++i, out += kSlotWords) {
-                    const uint2 q = list[r0 + i];
-                    *out = lane_mass(rows + q.x, (uint32_t)lane, q.y, colz);
+                if constexpr (View::kAhead && (!LL || QB == 0)) {
+                    // the next row's first steps are loaded while a row is summed (K=1024,
+                    // 14.4M tokens: 1.92 -> 1.87 ms per sweep; the LL kernels above
+                    // kThreadQTopics spill and lose 1%)
+                    uint2 q = make_uint2(0u, 0u);
+                    uint32_t e[4] = {}, f[4];
+                    if (i < n) {
+                        q = list[r0 + i];
+                        row_load(e, rows + q.x, (uint32_t)lane, q.y);
+                    }
+#pragma unroll(QB == 0 ? 2 : 1)
+                    for (; i < n; ++i, out += kSlotWords) {
+                        const uint2 c = q;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) f[j] = e[j];
+                        if (i + 1 < n) {
+                            q = list[r0 + i + 1];
+                            row_load(e, rows + q.x, (uint32_t)lane, q.y);
+                        }
+                        *out = row_sum(f, rows + c.x, (uint32_t)lane, c.y, colz);
+                    }
+                } else {
+                    for (; i < n; ++i, out += kSlotWords) {
+                        const uint2 q = list[r0 + i];
+                        *out = lane_mass(rows + q.x, (uint32_t)lane, q.y, colz);
+                    }
                 }
                 __syncwarp();
                 // the tokens of these rows, thread per token

@@ -565,7 +565,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
         // the exact bytes of the resident layout (the allocations below, in resident mode)
         auto nb = [](int64_t n, int64_t size) { return std::max<int64_t>(n, 1) * size; };
         const int64_t ns = (int64_t)st.size(), nw = (int64_t)wt.size();
-        const int64_t resident = 4 * nb(N, 4) + nb(T.dt_cap, 4) + nb(N, 2) + nb(D + 1, 4) + 3 * nb(D, 4) +
+        const int64_t resident = 4 * nb(N, 4) + nb(T.dt_cap + dev::kRowSlack, 4) + nb(N, 2) + nb(D + 1, 4) + 3 * nb(D, 4) +
                                  nb((int64_t)T.Vd * T.K, 4) + 2 * nb(std::max<int64_t>(Vs, 1), 4) + nb(T.swt_cap, 4) +
                                  nb(T.K, 4) + 2 * nb(V, 4) + nb(V, 16) + nb(V * 32, 4) + 2 * nb((int64_t)T.C * V, 4) +
                                  nb(ns, 16) + nb(nw, 16) + nb(ns, 8) + nb(1, 8) + nb(3 + 2 * T.C, 4) + nb(kCounters, 8) + nb(T.K, 4) +
@@ -577,13 +577,13 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     int rc;
 #define ALLOC(p, n) if ((rc = T.alloc(&(p), (n))) != LDA_OK) return rc
     if (!T.streaming) {
-        ALLOC(T.tok_doc, N); ALLOC(T.meta, N); ALLOC(T.dtok_pos, N); ALLOC(T.dtok_word, N); ALLOC(T.dt_ent, T.dt_cap);
+        ALLOC(T.tok_doc, N); ALLOC(T.meta, N); ALLOC(T.dtok_pos, N); ALLOC(T.dtok_word, N); ALLOC(T.dt_ent, T.dt_cap + dev::kRowSlack);
     } else {
         const int ns = cfg->num_streams > 0 ? cfg->num_streams : 4;
         T.slots.resize(ns);
         for (auto& sl : T.slots) {
             ALLOC(sl.tok_doc, T.max_chunk_tok); ALLOC(sl.dtok_pos, T.max_chunk_tok); ALLOC(sl.dtok_word, T.max_chunk_tok);
-            ALLOC(sl.meta, T.max_chunk_tok); ALLOC(sl.dt_ent, T.max_chunk_dt);
+            ALLOC(sl.meta, T.max_chunk_tok); ALLOC(sl.dt_ent, T.max_chunk_dt + dev::kRowSlack);
         }
         T.sstreams.resize(ns, nullptr);
         T.ev_slot.resize(ns, nullptr);
