@@ -77,29 +77,6 @@ __global__ void __launch_bounds__(256) k_wt_build(WtArgs a) {
 constexpr int kRebuildThreads = 256;
 constexpr int kSmoothMaxRounds = 2048;  // rounds of 32 topics in the smoothing table (K <= 65,536)
 
-// Exclusive scan of one value per thread across the CTA; *total gets the sum.  wsum holds
-// a word per warp.  Every thread of the CTA calls it.
-__device__ __forceinline__ uint32_t cta_exclusive_scan(uint32_t v, uint32_t* wsum, uint32_t* total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    uint32_t incl = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t t = __shfl_up_sync(FULL, incl, off);
-        if (lane >= off) incl += t;
-    }
-    if (lane == 31) wsum[wid] = incl;
-    __syncthreads();
-    uint32_t before = 0, tot = 0;
-    for (int i = 0; i < nw; ++i) {
-        const uint32_t x = wsum[i];
-        before += i < wid ? x : 0u;
-        tot += x;
-    }
-    *total = tot;
-    __syncthreads();
-    return before + incl - v;
-}
-
 // Adds topics topic_of(i), i in [0, n), to the CTA's histogram (16-bit counts) and sets
 // the bit of each topic whose count leaves zero; a topic >= K sets *err and is skipped.
 // Four 256-token steps of loads are in flight per thread.  n is uniform across the CTA.
@@ -126,32 +103,6 @@ __device__ __forceinline__ void cta_hist(uint32_t n, const F& topic_of, const Hi
             if (valid) hist_token(hist, bits, kk);
         }
     }
-}
-
-// Walks the CTA's bitmap (bw words) in ascending topic order: thread t takes words
-// [t R, t R + R), R = ceil(bw / threads), an exclusive scan of their popcounts places
-// its entries, and emit(k, count, position) is called for each non-zero topic; bits and
-// counts are cleared.  Returns the number of non-zero topics.
-template <class E>
-__device__ __forceinline__ uint32_t cta_compact(int bw, const Hist<true>& hist, uint32_t* bits, uint32_t* wsum,
-                                                const E& emit) {
-    const int R = (bw + blockDim.x - 1) / blockDim.x;
-    const int w0 = min(bw, (int)threadIdx.x * R), w1 = min(bw, w0 + R);
-    uint32_t c = 0;
-    for (int wi = w0; wi < w1; ++wi) c += (uint32_t)__popc(bits[wi]);
-    uint32_t total;
-    uint32_t p = cta_exclusive_scan(c, wsum, &total);
-    for (int wi = w0; wi < w1; ++wi) {
-        uint32_t m = bits[wi];
-        if (m) bits[wi] = 0u;
-        while (m) {
-            const uint32_t k = (uint32_t)wi * 32u + (uint32_t)(__ffs(m) - 1);
-            m &= m - 1u;
-            emit(k, hist.get(k), p++);
-            hist.clear(k);
-        }
-    }
-    return total;
 }
 
 // Word-topic rows above kLargeK topics: CTA per word tile (a dense word's chunk segment

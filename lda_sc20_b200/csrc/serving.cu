@@ -7,8 +7,8 @@
 // as the training sampler (max topic / S over the document's row / Q bucket, early accept).
 //
 // Device layout of a server: a token pool (word + topic per token, each request a
-// contiguous range), a theta pool (K floats per request slot) and a request table rebuilt
-// every step.  A step runs one sweep for every active request (each at its own sweep
+// contiguous range), a row pool (up to K entries per request slot: the request's topic counts
+// at the start of the sweep) and a request table.  A step runs one sweep for every active request (each at its own sweep
 // index); requests that arrive while others run are admitted at the next step when the
 // token pool and the slots have room.  Each request's randoms are keyed on (seed, request
 // id, sweep, position), so its result does not depend on what it was batched with.
@@ -22,8 +22,8 @@
 #include <vector>
 
 #include "common.h"
-#include "device_common.cuh"
 #include "launch_util.h"
+#include "sweep_body.cuh"
 
 using namespace lda;
 
@@ -89,14 +89,12 @@ __global__ void __launch_bounds__(256) k_model_lane_q(int V, int Vd, int K, floa
     }
 }
 
-// One active request of a step: its tokens sit at [tok_off, tok_off+len) of the pool and
-// it is split into items of `item_tokens` tokens, one warp each.  flags: FOLD_INIT (sweep
-// 0: sweep-start counts from the Philox initial topics), FOLD_LAST (the last sweep:
-// theta); bits 8.. hold the request's item count.
+// One active request: its tokens sit at [tok_off, tok_off+len) of the pool, its topic counts
+// in row slot `slot`, and at step s it runs sweep s - start.  It is sampled in items of
+// `item_tokens` tokens, one warp each.
 struct FoldReq {
-    uint32_t tok_off, len, rid, sweep, flags, slot, pad0, pad1;
+    uint32_t tok_off, len, rid, start, slot, pad0, pad1, pad2;
 };
-enum { FOLD_INIT = 1, FOLD_LAST = 2 };
 
 struct FoldArgs {
     int K;
@@ -110,11 +108,13 @@ struct FoldArgs {
     const uint32_t* item_req;  // per item: request index << 16 | item index within the request
     int nitems;
     uint32_t item_tokens;
+    uint32_t step;
+    uint32_t sweeps;
     const uint32_t* words;
-    uint16_t* z0;  // topics after even sweep counts
-    uint16_t* z1;  // topics after odd sweep counts
-    float* theta;
-    unsigned* done;  // per slot: items of the last sweep that finished
+    uint16_t* z;
+    uint32_t* rows;     // per slot K entries (k << 16 | count), ascending k
+    uint32_t* row_nnz;  // per slot
+    float* theta;       // per slot K floats, in pinned host memory
 };
 
 __device__ __forceinline__ float foldin_uniform(uint32_t seed_lo, uint32_t seed_hi, uint32_t rid, uint32_t sweep,
@@ -129,51 +129,28 @@ __device__ __forceinline__ uint32_t foldin_init(uint32_t seed_lo, uint32_t seed_
     return (uint32_t)(((unsigned long long)x * (unsigned long long)(uint32_t)K) >> 32);
 }
 
-// phi of topic k for word row `prow` with the word's max topic zeroed (the sweep's colz).
-__device__ __forceinline__ float colz_of(const float* __restrict__ prow, int mk, uint32_t k) {
-    return (int)k == mk ? 0.0f : __ldg(prow + k);
-}
+// A word's phi row in the frozen matrix with its max topic zeroed, as a sampler's view of a
+// word column.
+struct PhiRow {
+    const float* __restrict__ prow;
+    int mk;
+    __device__ __forceinline__ float operator()(int k) const { return k == mk ? 0.0f : __ldg(prow + k); }
+};
 
-// Serial fmaf chain over the lane's entries l, l + 32, ... of the document row (in shared
-// memory, so a step's 32 reads are conflict-free) with phi gathered from the frozen
-// matrix.  The gathers of up to four entries are issued before their products are summed,
-// also when the lane has fewer than four left (rows of short requests hold only a few
-// entries per lane).
-__device__ __forceinline__ float fold_lane_mass(const uint32_t* row, uint32_t lane, uint32_t nnz,
-                                                const float* __restrict__ prow, int mk) {
-    float acc = 0.0f;
-    for (uint32_t q = lane; q < nnz; q += 128u) {
-        uint32_t e[4];
-        float c[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t i = q + 32u * j;
-            e[j] = i < nnz ? row[i] : 0u;
-            c[j] = i < nnz ? colz_of(prow, mk, e[j] >> 16) : 0.0f;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (q + 32u * j < nnz) acc = ffma(u2f(e[j] & 0xffffu), c[j], acc);
-    }
-    return acc;
-}
-
-// The S-bucket draw among lane ls's entries ls, ls + 32, ... (the partial sums of
-// fold_lane_mass): the first entry with colz > 0 whose partial sum exceeds t2, else the
-// last entry with colz > 0, else mk.
-__device__ __forceinline__ int fold_lane_draw(const uint32_t* row, uint32_t ls, uint32_t nnz,
-                                              const float* __restrict__ prow, int mk, float t2) {
+// The S-bucket draw among lane ls's entries ls, ls + 32, ... of the row (lane_draw with phi
+// gathered from the frozen matrix): the first entry with phi > 0 whose partial sum exceeds
+// t2, else the last entry with phi > 0, else the max topic.
+__device__ __forceinline__ int fold_lane_draw(const uint32_t* __restrict__ row, uint32_t ls, uint32_t nnz,
+                                              const PhiRow& phi, float t2) {
     float acc = 0.0f;
     int last = -1;
     for (uint32_t q = ls; q < nnz; q += 128u) {
         uint32_t e[4];
         float c[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t i = q + 32u * j;
-            e[j] = i < nnz ? row[i] : 0u;
-            c[j] = i < nnz ? colz_of(prow, mk, e[j] >> 16) : 0.0f;
-        }
+        for (int j = 0; j < 4; ++j) e[j] = q + 32u * j < nnz ? __ldg(row + q + 32u * j) : 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = q + 32u * j < nnz ? phi((int)(e[j] >> 16)) : 0.0f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (q + 32u * j >= nnz) break;
@@ -184,174 +161,198 @@ __device__ __forceinline__ int fold_lane_draw(const uint32_t* row, uint32_t ls, 
             }
         }
     }
-    return last >= 0 ? last : mk;
+    return last >= 0 ? last : phi.mk;
 }
 
-// Doc-topic counts are at most 65535 (the request length limit), so two topics share a
-// 32-bit shared word: topic k is the (k & 1) half of word k >> 1.
-__device__ __forceinline__ uint32_t hist_get(const uint32_t* hist, uint32_t k) {
-    return (hist[k >> 1] >> ((k & 1u) << 4)) & 0xffffu;
-}
-
-// Doc-topic histogram of one request into the warp's shared counts, from the Philox
-// initial topics (init) or from a topic array.
-__device__ __forceinline__ void fold_hist(uint32_t* hist, const FoldArgs& a, const FoldReq& q,
-                                          const uint16_t* zsrc, bool init, int lane) {
-    for (uint32_t base = 0; base < q.len; base += 32) {
-        const uint32_t pos = base + lane;
-        const bool valid = pos < q.len;
-        uint32_t k = 0xffffffffu;
-        if (valid) {
-            k = init ? foldin_init(a.seed_lo, a.seed_hi, q.rid, pos, a.K) : (uint32_t)__ldcg(zsrc + q.tok_off + pos);
-            if (k >= (uint32_t)a.K) k = 0;  // topics are written < K; keep the index in bounds
-        }
-        if (valid) atomicAdd(&hist[k >> 1], 1u << ((k & 1u) << 4));
+// The row's count of topic k (0 when it has none), by binary search.
+__device__ __forceinline__ uint32_t row_count(const uint32_t* __restrict__ row, uint32_t nnz, uint32_t k) {
+    uint32_t lo = 0, hi = nnz;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if ((__ldg(row + mid) >> 16) < k) lo = mid + 1; else hi = mid;
     }
-    __syncwarp();
+    if (lo >= nnz) return 0u;
+    const uint32_t e = __ldg(row + lo);
+    return (e >> 16) == k ? e & 0xffffu : 0u;
 }
 
-// One sweep of every active request: warp per work item.  The warp rebuilds the request's
-// sweep-start doc-topic histogram and its ascending-k row in warp-private shared memory,
-// screens each 32-token group thread-per-token by the max-topic bound, evaluates the row
-// mass of the tokens it does not settle with the whole warp (lane blocks of the row, phi
-// gathered from the frozen matrix, reused while consecutive tokens share a word), and
-// finishes S-bucket draws inside the chosen block thread-per-token.  Topics are read from
-// one buffer and written to the other, so items of one request can run on any warps in
-// any order.  On a request's last sweep the item that finishes last (a per-slot counter)
-// writes theta = (n_dk + alpha) / (n_d + K*alpha) of the new topics.
-__global__ void __launch_bounds__(256) k_foldin(FoldArgs a) {
-    extern __shared__ uint32_t smu[];
+// Lane sums of one row against kFoldWords words at a time, into their slots: lane l sums the
+// row's entries l, l + 32, ... serially (the training sampler's order), the gathers of all
+// words' first NS steps issued before any is used.  c and k hold the lane's first four
+// entries (count 0 where the row has none: fmaf(0, phi, acc) is acc, as is the max topic's
+// term).
+constexpr int kFoldWords = 4;
+template <int NS>
+__device__ __forceinline__ void fold_rows(const FoldArgs& a, const uint32_t* __restrict__ row, uint32_t nnz,
+                                          const float (&c)[4], const uint32_t (&k)[4], const uint2* list, int nrows,
+                                          float* slots, int lane) {
+    for (int i = 0; i < nrows; i += kFoldWords) {
+        const float* prow[kFoldWords];
+        uint32_t mk[kFoldWords];
+        float v[kFoldWords][NS], acc[kFoldWords];
+#pragma unroll
+        for (int t = 0; t < kFoldWords; ++t) {
+            const uint2 q = list[min(i + t, nrows - 1)];
+            prow[t] = a.phi + (size_t)q.x * a.K;
+            mk[t] = q.y;
+#pragma unroll
+            for (int s = 0; s < NS; ++s) v[t][s] = __ldg(prow[t] + k[s]);
+        }
+#pragma unroll
+        for (int t = 0; t < kFoldWords; ++t) {
+            acc[t] = 0.0f;
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                if (k[s] != mk[t]) acc[t] = ffma(c[s], v[t][s], acc[t]);
+        }
+        if (NS == 4) {
+            for (uint32_t q = 128u + (uint32_t)lane; q < nnz; q += 32u) {
+                const uint32_t e = __ldg(row + q), kk = e >> 16;
+                const float cc = u2f(e & 0xffffu);
+#pragma unroll
+                for (int t = 0; t < kFoldWords; ++t)
+                    if (kk != mk[t]) acc[t] = ffma(cc, __ldg(prow[t] + kk), acc[t]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < kFoldWords; ++t)
+            if (i + t < nrows) slots[kSlotWords * (i + t) + lane] = acc[t];
+    }
+}
+
+// One sweep of every active request: warp per work item, the three parts of the training
+// sampler's groups (sample_groups) with every token its own word: the tokens are screened
+// thread-per-token, the request's row is summed against each unsettled token's word
+// (consecutive tokens of one word share a sum), and each token decides by itself.  What
+// bounds it is the gathers of phi, 4 KB a word at K=1024 from a matrix larger than L2: the
+// lane's row entries sit in registers for the whole item and four words' gathers are in
+// flight together.  (Rebuilding the request's counts and row for every item, and summing one
+// word at a time, took 350 us per sweep of 2,048 requests against 200 for this kernel and the
+// row builds.)
+constexpr int kFoldWarpWords = 32 * kSlotWords + 64;
+__global__ void __launch_bounds__(256, 3) k_foldin(FoldArgs a) {
+    extern __shared__ float smf[];
     const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int hwords = (a.K + 1) >> 1;
-    uint32_t* hist = smu + (size_t)(hwords + a.K) * wid;
-    uint32_t* row = hist + hwords;
-    for (int k = lane; k < hwords; k += 32) hist[k] = 0u;
-    __syncwarp();
+    float* slots = smf + (size_t)kFoldWarpWords * wid;
+    uint2* list = reinterpret_cast<uint2*>(slots + 32 * kSlotWords);
     for (int r = blockIdx.x * warps + wid; r < a.nitems; r += gridDim.x * warps) {
         const uint32_t ir = __ldg(a.item_req + r);
         const FoldReq it = a.reqs[ir >> 16];
-        const uint32_t begin = (ir & 0xffffu) * a.item_tokens;
-        const uint16_t* zin = (it.sweep & 1u) ? a.z1 : a.z0;
-        uint16_t* zout = (it.sweep & 1u) ? a.z0 : a.z1;
-        const uint32_t off = it.tok_off, len = it.len;
-        fold_hist(hist, a, it, zin, (it.flags & FOLD_INIT) != 0, lane);
-        uint32_t nnz = 0;
-        for (int kb = 0; kb < a.K; kb += 32) {
-            const int k = kb + lane;
-            const uint32_t h = k < a.K ? hist_get(hist, (uint32_t)k) : 0u;
-            const unsigned bal = __ballot_sync(FULL, h != 0u);
-            if (h) row[nnz + __popc(bal & ((1u << lane) - 1u))] = ((uint32_t)k << 16) | h;
-            nnz += (uint32_t)__popc(bal);
+        const uint32_t begin = (ir & 0xffffu) * a.item_tokens, end = min(begin + a.item_tokens, it.len);
+        const uint32_t sweep = a.step - it.start;
+        const uint32_t* row = a.rows + (size_t)it.slot * a.K;
+        const uint32_t nnz = __ldg(a.row_nnz + it.slot);
+        float c[4];
+        uint32_t k[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const uint32_t e = (uint32_t)lane + 32u * s < nnz ? __ldg(row + lane + 32 * s) : 0u;
+            c[s] = u2f(e & 0xffffu);
+            k[s] = e >> 16;
         }
-        __syncwarp();
-        uint32_t cur_w = 0xffffffffu;
-        float SL = 0.0f, SP = 0.0f, S = 0.0f;
-        const uint32_t end = min(begin + a.item_tokens, len);
         for (uint32_t g = begin; g < end; g += 32) {
             const uint32_t pos = g + lane;
             const bool valid = pos < end;
             uint32_t w = 0;
             int mk = 0;
-            float pmax = 0.0f, u = 0.0f, Qw = 0.0f;
+            float pmax = 0.0f, u = 0.0f, Q = 0.0f;
             bool ea = false;
             if (valid) {
-                w = __ldg(a.words + off + pos);
+                w = __ldg(a.words + it.tok_off + pos);
                 const uint32_t t2 = __ldg(a.top2 + w);
                 mk = (int)(t2 & 0xffffu);
                 const float4 ph = __ldg(a.phi4 + w);
-                const uint32_t cmax = hist_get(hist, (uint32_t)mk), c2 = hist_get(hist, t2 >> 16);
-                u = foldin_uniform(a.seed_lo, a.seed_hi, it.rid, it.sweep, pos);
+                const uint32_t cmax = row_count(row, nnz, t2 & 0xffffu), c2 = row_count(row, nnz, t2 >> 16);
+                u = foldin_uniform(a.seed_lo, a.seed_hi, it.rid, sweep, pos);
                 pmax = fmul(fadd(u2f(cmax), a.alpha), ph.x);
-                const float shat = ffma(u2f(c2), ph.y, fmul(u2f(len - cmax - c2), ph.z));
-                Qw = ph.w;
-                ea = fmul(u, fadd(fadd(pmax, shat), Qw)) < pmax;
+                const float shat = ffma(u2f(c2), ph.y, fmul(u2f(it.len - cmax - c2), ph.z));
+                Q = ph.w;
+                ea = fmul(u, fadd(fadd(pmax, shat), Q)) < pmax;
             }
             int znew = mk;
-            bool defer = false;
-            uint32_t my_ls = 0;
-            float my_t2 = 0.0f;
-            unsigned need = __ballot_sync(FULL, valid && !ea);
-            while (need) {
-                const int j = __ffs(need) - 1;
-                need &= need - 1u;
+            Draw dr{BR_NONE, 0u, 0.0f, 0.0f};
+            const unsigned need = __ballot_sync(FULL, valid && !ea);
+            const bool mine = (need >> lane) & 1u;
+            const unsigned below = need & ((1u << lane) - 1u);
+            const uint32_t wp = __shfl_sync(FULL, w, below ? 31 - __clz(below) : lane);
+            const bool lead = mine && (!below || w != wp);
+            const unsigned leaders = __ballot_sync(FULL, lead);
+            if (need) {
+                const int nrows = __popc(leaders);
+                const int ri = __popc(leaders & ((2u << lane) - 1u)) - 1;
+                if (lead) list[ri] = make_uint2(w, (uint32_t)mk);
+                __syncwarp();
+                if (nnz > 64u) fold_rows<4>(a, row, nnz, c, k, list, nrows, slots, lane);
+                else if (nnz > 32u) fold_rows<2>(a, row, nnz, c, k, list, nrows, slots, lane);
+                else fold_rows<1>(a, row, nnz, c, k, list, nrows, slots, lane);
+                __syncwarp();
+                decide_tokens<false>(slots, mine ? ri : 0, mine, false, pmax, Q, u, lane, dr);
+                __syncwarp();  // the slots may be overwritten
+            }
+            uint32_t qw = 0xffffffffu;
+            float QL = 0.0f, QP = 0.0f;
+            for (unsigned b = __ballot_sync(FULL, dr.kind == BR_Q); b; b &= b - 1u) {
+                const int j = __ffs(b) - 1;
                 const uint32_t wj = __shfl_sync(FULL, w, j);
                 const int mkj = __shfl_sync(FULL, mk, j);
-                const float pmj = __shfl_sync(FULL, pmax, j);
-                const float uj = __shfl_sync(FULL, u, j);
-                const float Qj = __shfl_sync(FULL, Qw, j);
-                const float* prow = a.phi + (size_t)wj * a.K;
-                if (wj != cur_w) {
-                    cur_w = wj;
-                    SL = fold_lane_mass(row, (uint32_t)lane, nnz, prow, mkj);
-                    SP = warp_ks_scan(SL, lane);
-                    S = __shfl_sync(FULL, SP, 31);
+                if (wj != qw) {
+                    qw = wj;
+                    QL = __ldg(a.ql + (size_t)wj * 32 + lane);
+                    QP = warp_ks_scan(QL, lane);
                 }
-                const float pS = fadd(pmj, S);
-                const float total = fadd(pS, Qj);
-                const float target = fmul(uj, total);
-                if (target < pmj) {
-                    // the max topic (znew already holds it)
-                } else if (target < pS) {
-                    const float tt = fsub(target, pmj);
-                    const unsigned cand = __ballot_sync(FULL, tt < SP && SL > 0.0f);
-                    const unsigned pos_l = __ballot_sync(FULL, SL > 0.0f);
-                    const int ls = cand ? __ffs(cand) - 1 : 31 - __clz(pos_l);
-                    const float prev = __shfl_sync(FULL, SP, ls > 0 ? ls - 1 : 0);
-                    if (lane == j) {
-                        defer = true;
-                        my_ls = (uint32_t)ls;
-                        my_t2 = ls > 0 ? fsub(tt, prev) : tt;
-                    }
-                } else {
-                    const float tt = fsub(target, pS);
-                    const float QL = __ldg(a.ql + (size_t)wj * 32 + lane);
-                    const float QP = warp_ks_scan(QL, lane);
-                    const unsigned cand = __ballot_sync(FULL, tt < QP && QL > 0.0f);
-                    const unsigned pos_l = __ballot_sync(FULL, QL > 0.0f);
-                    const int ls = cand ? __ffs(cand) - 1 : (pos_l ? 31 - __clz(pos_l) : 0);
-                    const float prev = __shfl_sync(FULL, QP, ls > 0 ? ls - 1 : 0);
-                    const float t2 = ls > 0 ? fsub(tt, prev) : tt;
-                    const int K = a.K;
-                    const float alpha = a.alpha;
-                    const uint32_t n = (uint32_t)((K - ls + 31) / 32);
-                    const int zq = warp_level2(n, t2, mkj, lane, [&](uint32_t i, int& key, float& term, bool& ok) {
-                        const int k = ls + 32 * (int)i;
-                        const float cz = colz_of(prow, mkj, (uint32_t)k);
-                        key = k;
-                        term = fmul(alpha, cz);
-                        ok = cz > 0.0f;
-                    });
-                    if (lane == j) znew = zq;
-                }
+                const float tt = __shfl_sync(FULL, dr.t, j);
+                const int zq = warp_q_draw<1>(PhiRow{a.phi + (size_t)wj * a.K, mkj}, tt, QL, QP, a.K, a.alpha, mkj, lane,
+                                              nullptr, 0);
+                if (lane == j) znew = zq;
             }
-            if (defer) znew = fold_lane_draw(row, my_ls, nnz, a.phi + (size_t)w * a.K, mk, my_t2);
-            if (valid) zout[off + pos] = (uint16_t)znew;
-        }
-        __syncwarp();
-        for (int k = lane; k < hwords; k += 32) hist[k] = 0u;
-        __syncwarp();
-        if (it.flags & FOLD_LAST) {
-            // publish this item's topics, then count it; the last item of the request
-            // (whatever warp runs it) sees every other item's topics
-            __threadfence();
-            __syncwarp();
-            unsigned prior = 0;
-            if (lane == 0) prior = atomicAdd(a.done + it.slot, 1u);
-            prior = __shfl_sync(FULL, prior, 0);
-            const unsigned nitems = it.flags >> 8;
-            if (prior + 1u == nitems) {
-                __threadfence();
-                fold_hist(hist, a, it, zout, false, lane);
-                float* th = a.theta + (size_t)it.slot * a.K;
-                const float den = fadd(u2f(len), a.Kalpha);
-                for (int k = lane; k < a.K; k += 32) th[k] = __fdiv_rn(fadd(u2f(hist_get(hist, (uint32_t)k)), a.alpha), den);
-                __syncwarp();
-                for (int k = lane; k < hwords; k += 32) hist[k] = 0u;
-                if (lane == 0) a.done[it.slot] = 0u;
-                __syncwarp();
-            }
+            if (dr.kind == BR_S) znew = fold_lane_draw(row, dr.ls, nnz, PhiRow{a.phi + (size_t)w * a.K, mk}, dr.t);
+            if (valid) a.z[it.tok_off + pos] = (uint16_t)znew;
         }
     }
+}
+
+// The requests' topic counts, CTA per request from `first` on: the row of the next sweep's
+// start (of the first sweep's, from the Philox initial topics, with INIT), or after the last
+// sweep theta = (n_dk + alpha) / (n_d + K*alpha), written straight to host memory.  Shared
+// memory: 16-bit counts (a request has at most 65,535 tokens) and the bitmap of the topics
+// that have one.
+template <bool INIT>
+__global__ void __launch_bounds__(256) k_fold_build(FoldArgs a, int first) {
+    extern __shared__ uint32_t smu[];
+    __shared__ uint32_t wsum[8];
+    const FoldReq q = a.reqs[first + blockIdx.x];
+    const int hw = Hist<true>::words(a.K), bw = (a.K + 31) >> 5;
+    const Hist<true> hist{smu};
+    uint32_t* bits = smu + hw;
+    for (int i = threadIdx.x; i < hw + bw; i += blockDim.x) smu[i] = 0u;
+    __syncthreads();
+    for (uint32_t base = 0; base < q.len; base += 4u * blockDim.x) {
+        uint32_t k[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const uint32_t pos = base + (uint32_t)s * blockDim.x + threadIdx.x;
+            k[s] = 0xffffffffu;
+            if (pos < q.len) {
+                k[s] = INIT ? foldin_init(a.seed_lo, a.seed_hi, q.rid, pos, a.K) : (uint32_t)__ldg(a.z + q.tok_off + pos);
+                if (k[s] >= (uint32_t)a.K) k[s] = 0;  // topics are written < K; keep the index in bounds
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            if (k[s] != 0xffffffffu) hist_token(hist, bits, k[s]);
+    }
+    __syncthreads();
+    if (!INIT && a.step - q.start == a.sweeps - 1u) {
+        float* th = a.theta + (size_t)q.slot * a.K;
+        const float den = fadd(u2f(q.len), a.Kalpha);
+        for (int k = threadIdx.x; k < a.K; k += blockDim.x)
+            th[k] = __fdiv_rn(fadd(u2f(hist.get((uint32_t)k)), a.alpha), den);
+        return;
+    }
+    uint32_t* out = a.rows + (size_t)q.slot * a.K;
+    const uint32_t nnz =
+        cta_compact(bw, hist, bits, wsum, [&](uint32_t k, uint32_t h, uint32_t p) { out[p] = (k << 16) | h; });
+    if (threadIdx.x == 0) a.row_nnz[q.slot] = nnz;
 }
 
 }  // namespace dev
@@ -469,6 +470,7 @@ namespace {
 using Clock = std::chrono::steady_clock;
 double now_s() { return std::chrono::duration<double>(Clock::now().time_since_epoch()).count(); }
 constexpr int kRing = 3;      // host item buffers / events
+constexpr int kFoldWarps = 8; // most warps per CTA of the fold-in kernel
 constexpr int kInFlight = 2;  // steps queued on the stream before the host waits
 }  // namespace
 
@@ -476,19 +478,20 @@ struct lda_server {
     lda_model* m = nullptr;
     int device = 0;
     cudaStream_t st = nullptr;
-    int sweeps = 30, max_active = 0, warps = 8, grid = 0;
+    int sweeps = 30, max_active = 0, num_sms = 0, grid = 0;
     uint32_t item_tokens = 32;
     uint64_t seed = 0;
     int64_t tok_cap = 0, max_items = 0;
-    size_t smem = 0;
+    size_t smem_build = 0;
     uint32_t* d_words = nullptr;
-    uint16_t* d_z = nullptr;  // [2][tok_cap]
-    float* d_theta = nullptr;
-    unsigned* d_done = nullptr;
-    dev::FoldReq* d_reqs = nullptr;
-    uint32_t* d_items = nullptr;
-    dev::FoldReq* h_reqs[kRing] = {};
-    uint32_t* h_items[kRing] = {};
+    uint16_t* d_z = nullptr;
+    uint32_t *d_rows = nullptr, *d_row_nnz = nullptr;  // per slot
+    // the active requests' table and the item list behind it, uploaded when the set of active
+    // requests has changed
+    unsigned char* d_table = nullptr;
+    unsigned char* h_table[kRing] = {};
+    int64_t table_items = 0;  // of the table on the device
+    bool table_stale = true;
     cudaEvent_t ev[kRing] = {};
     uint32_t* h_words = nullptr;
     float* h_theta = nullptr;
@@ -502,6 +505,7 @@ struct lda_server {
     struct Active {
         uint32_t rid, len;
         int64_t off;
+        uint32_t start;   // the step of its first sweep
         int sweep, slot;  // sweeps issued so far
         double t_submit;
         int64_t last_step;
@@ -523,18 +527,20 @@ struct lda_server {
         if (st) cudaStreamSynchronize(st);
         cudaFree(d_words);
         cudaFree(d_z);
-        cudaFree(d_theta);
-        cudaFree(d_done);
-        cudaFree(d_items);
-        cudaFree(d_reqs);
+        cudaFree(d_rows);
+        cudaFree(d_row_nnz);
+        cudaFree(d_table);
         for (int i = 0; i < kRing; ++i) {
-            cudaFreeHost(h_items[i]);
-            cudaFreeHost(h_reqs[i]);
+            cudaFreeHost(h_table[i]);
             if (ev[i]) cudaEventDestroy(ev[i]);
         }
         cudaFreeHost(h_words);
         cudaFreeHost(h_theta);
         if (st) cudaStreamDestroy(st);
+    }
+
+    size_t table_bytes(int64_t items) const {
+        return sizeof(dev::FoldReq) * (size_t)max_active + sizeof(uint32_t) * (size_t)items;
     }
 
     bool alloc_tokens(int64_t len, int64_t* off) {
@@ -627,8 +633,8 @@ extern "C" int lda_server_create(lda_model* m, int64_t max_tokens, int32_t max_a
     s->seed = seed;
     CUDA_TRY(cudaSetDevice(s->device));
     if (max_tokens == 0) {
-        // admission by free HBM: a quarter of the free device memory holds the token pool
-        // (4 B word + 2 x 2 B topics per token)
+        // admission by free HBM: the token pool (4 B word + 2 B topic per token) holds one
+        // token per 8 bytes of a quarter of the free device memory
         size_t fr = 0, tot = 0;
         CUDA_TRY(cudaMemGetInfo(&fr, &tot));
         max_tokens = std::min<int64_t>((int64_t)(fr / 4) / 8, (int64_t)1 << 30);
@@ -637,15 +643,12 @@ extern "C" int lda_server_create(lda_model* m, int64_t max_tokens, int32_t max_a
     s->max_items = (int64_t)max_active + max_tokens / s->item_tokens + 1;
     cudaError_t e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&s->d_words, sizeof(uint32_t) * (size_t)max_tokens);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_z, sizeof(uint16_t) * 2 * (size_t)max_tokens);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_theta, sizeof(float) * (size_t)max_active * m->K);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_done, sizeof(unsigned) * (size_t)max_active);
-    if (e == cudaSuccess) e = cudaMemset(s->d_done, 0, sizeof(unsigned) * (size_t)max_active);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_items, sizeof(uint32_t) * (size_t)s->max_items);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_reqs, sizeof(dev::FoldReq) * (size_t)max_active);
+    if (e == cudaSuccess) e = cudaMalloc(&s->d_z, sizeof(uint16_t) * (size_t)max_tokens);
+    if (e == cudaSuccess) e = cudaMalloc(&s->d_rows, sizeof(uint32_t) * (size_t)max_active * m->K);
+    if (e == cudaSuccess) e = cudaMalloc(&s->d_row_nnz, sizeof(uint32_t) * (size_t)max_active);
+    if (e == cudaSuccess) e = cudaMalloc(&s->d_table, s->table_bytes(s->max_items));
     for (int i = 0; i < kRing && e == cudaSuccess; ++i) {
-        e = cudaMallocHost(&s->h_items[i], sizeof(uint32_t) * (size_t)s->max_items);
-        if (e == cudaSuccess) e = cudaMallocHost(&s->h_reqs[i], sizeof(dev::FoldReq) * (size_t)max_active);
+        e = cudaMallocHost(&s->h_table[i], s->table_bytes(s->max_items));
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev[i], cudaEventDisableTiming);
     }
     if (e == cudaSuccess) e = cudaMallocHost(&s->h_words, sizeof(uint32_t) * (size_t)max_tokens);
@@ -656,16 +659,17 @@ extern "C" int lda_server_create(lda_model* m, int64_t max_tokens, int32_t max_a
     }
     s->free_iv[0] = max_tokens;
     for (int i = max_active - 1; i >= 0; --i) s->free_slots.push_back(i);
-    int max_smem = 0, num_sms = 0, per_sm = 0;
+    int max_smem = 0, per_sm = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
-    CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, s->device));
-    const int64_t per_warp = 4 * ((int64_t)(m->K + 1) / 2 + m->K);  // packed counts + row
-    s->warps = (int)std::min<int64_t>(8, (int64_t)max_smem / per_warp);
-    if (s->warps < 1) return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory", m->K);
-    s->smem = (size_t)(s->warps * per_warp);
-    CUDA_TRY(raise_smem_limit((const void*)dev::k_foldin, s->smem));
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)dev::k_foldin, 32 * s->warps, s->smem));
-    s->grid = std::max(1, per_sm * num_sms);
+    CUDA_TRY(cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, s->device));
+    s->smem_build = ((size_t)dev::Hist<true>::words(m->K) + (size_t)(m->K + 31) / 32) * 4;
+    if (s->smem_build > (size_t)max_smem) return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory", m->K);
+    CUDA_TRY(raise_smem_limit((const void*)dev::k_fold_build<true>, s->smem_build));
+    CUDA_TRY(raise_smem_limit((const void*)dev::k_fold_build<false>, s->smem_build));
+    const size_t smem = sizeof(float) * dev::kFoldWarpWords * kFoldWarps;
+    CUDA_TRY(raise_smem_limit((const void*)dev::k_foldin, smem));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)dev::k_foldin, 32 * kFoldWarps, smem));
+    s->grid = std::max(1, per_sm * s->num_sms);
     CUDA_TRY(cudaStreamSynchronize(s->st));
     *out = s.release();
     return LDA_OK;
@@ -683,16 +687,16 @@ extern "C" int lda_server_set_item_tokens(lda_server* s, int32_t n) {
     if (need > s->max_items) {
         CUDA_TRY(cudaSetDevice(s->device));
         CUDA_TRY(cudaStreamSynchronize(s->st));
-        cudaFree(s->d_items);
-        s->d_items = nullptr;
+        cudaFree(s->d_table);
+        s->d_table = nullptr;
         for (int i = 0; i < kRing; ++i) {
-            cudaFreeHost(s->h_items[i]);
-            s->h_items[i] = nullptr;
+            cudaFreeHost(s->h_table[i]);
+            s->h_table[i] = nullptr;
         }
         s->max_items = 0;
-        cudaError_t e = cudaMalloc(&s->d_items, sizeof(uint32_t) * (size_t)need);
-        for (int i = 0; i < kRing && e == cudaSuccess; ++i)
-            e = cudaMallocHost(&s->h_items[i], sizeof(uint32_t) * (size_t)need);
+        s->table_stale = true;
+        cudaError_t e = cudaMalloc(&s->d_table, s->table_bytes(need));
+        for (int i = 0; i < kRing && e == cudaSuccess; ++i) e = cudaMallocHost(&s->h_table[i], s->table_bytes(need));
         if (e != cudaSuccess) {
             cudaGetLastError();
             return fail(LDA_ERR_DEVICE_MEM, "item table allocation failed: %s", cudaGetErrorString(e));
@@ -730,6 +734,16 @@ static int server_issue(lda_server* s) {
     // the host buffers of step `steps` were last used by step `steps - kRing`
     s->collect(kInFlight - 1, &rc);
     if (rc) return rc;
+    const int64_t k = s->steps;
+    const int nold = (int)s->active.size();
+    // new requests' words go up in one copy per run of neighbouring pool ranges
+    int64_t run0 = 0, run1 = 0;
+    auto upload = [&]() -> int {
+        if (run1 > run0)
+            CUDA_TRY(cudaMemcpyAsync(s->d_words + run0, s->h_words + run0, sizeof(uint32_t) * (size_t)(run1 - run0),
+                                     cudaMemcpyHostToDevice, s->st));
+        return LDA_OK;
+    };
     while (!s->queue.empty() && (int)s->active.size() < s->max_active && !s->free_slots.empty()) {
         auto& p = s->queue.front();
         int64_t off;
@@ -739,41 +753,43 @@ static int server_issue(lda_server* s) {
         a.len = (uint32_t)p.words.size();
         a.off = off;
         a.sweep = 0;
+        a.start = (uint32_t)k;
         a.slot = s->free_slots.back();
         s->free_slots.pop_back();
         a.t_submit = p.t_submit;
         a.last_step = -1;
         std::memcpy(s->h_words + off, p.words.data(), sizeof(uint32_t) * a.len);
-        CUDA_TRY(cudaMemcpyAsync(s->d_words + off, s->h_words + off, sizeof(uint32_t) * a.len, cudaMemcpyHostToDevice,
-                                 s->st));
+        if (off != run1) {
+            if ((rc = upload())) return rc;
+            run0 = off;
+        }
+        run1 = off + a.len;
         s->active.push_back(a);
         s->queue.pop_front();
+        s->table_stale = true;
     }
+    if ((rc = upload())) return rc;
     if (s->active.empty()) return LDA_OK;
     if (s->max_items == 0) return fail(LDA_ERR_STATE, "the server has no item table (a failed resize)");
-    const int64_t k = s->steps;
-    uint32_t* items = s->h_items[k % kRing];
-    dev::FoldReq* reqs = s->h_reqs[k % kRing];
-    int64_t n = 0;
     const uint32_t T = s->item_tokens;
     const int nreq = (int)s->active.size();
-    for (int r = 0; r < nreq; ++r) {
-        const auto& a = s->active[r];
-        const uint32_t nitems = (a.len + T - 1) / T;
-        dev::FoldReq& q = reqs[r];
-        q.tok_off = (uint32_t)a.off;
-        q.len = a.len;
-        q.rid = a.rid;
-        q.sweep = (uint32_t)a.sweep;
-        q.flags = (a.sweep == 0 ? (uint32_t)dev::FOLD_INIT : 0u) |
-                  (a.sweep == s->sweeps - 1 ? (uint32_t)dev::FOLD_LAST : 0u) | (nitems << 8);
-        q.slot = (uint32_t)a.slot;
-        q.pad0 = q.pad1 = 0;
-        const uint32_t tag = (uint32_t)r << 16;
-        for (uint32_t j = 0; j < nitems; ++j) items[n++] = tag | j;
+    if (s->table_stale) {
+        dev::FoldReq* reqs = reinterpret_cast<dev::FoldReq*>(s->h_table[k % kRing]);
+        uint32_t* items = reinterpret_cast<uint32_t*>(reqs + nreq);
+        int64_t n = 0;
+        for (int r = 0; r < nreq; ++r) {
+            const auto& a = s->active[r];
+            const uint32_t nitems = (a.len + T - 1) / T;
+            reqs[r] = dev::FoldReq{(uint32_t)a.off, a.len, a.rid, a.start, (uint32_t)a.slot, 0u, 0u, 0u};
+            const uint32_t tag = (uint32_t)r << 16;
+            for (uint32_t j = 0; j < nitems; ++j) items[n++] = tag | j;
+        }
+        CUDA_TRY(cudaMemcpyAsync(s->d_table, reqs, sizeof(dev::FoldReq) * (size_t)nreq + sizeof(uint32_t) * (size_t)n,
+                                 cudaMemcpyHostToDevice, s->st));
+        s->table_items = n;
+        s->table_stale = false;
     }
-    CUDA_TRY(cudaMemcpyAsync(s->d_reqs, reqs, sizeof(dev::FoldReq) * (size_t)nreq, cudaMemcpyHostToDevice, s->st));
-    CUDA_TRY(cudaMemcpyAsync(s->d_items, items, sizeof(uint32_t) * (size_t)n, cudaMemcpyHostToDevice, s->st));
+    const int64_t n = s->table_items;
     dev::FoldArgs fa;
     fa.K = s->m->K;
     fa.alpha = s->m->alpha;
@@ -784,34 +800,42 @@ static int server_issue(lda_server* s) {
     fa.top2 = s->m->top2;
     fa.phi4 = s->m->phi4;
     fa.ql = s->m->ql;
-    fa.reqs = s->d_reqs;
-    fa.item_req = s->d_items;
+    fa.reqs = reinterpret_cast<const dev::FoldReq*>(s->d_table);
+    fa.item_req = reinterpret_cast<const uint32_t*>(fa.reqs + nreq);
     fa.nitems = (int)n;
     fa.item_tokens = T;
+    fa.step = (uint32_t)k;
+    fa.sweeps = (uint32_t)s->sweeps;
     fa.words = s->d_words;
-    fa.z0 = s->d_z;
-    fa.z1 = s->d_z + s->tok_cap;
-    fa.theta = s->d_theta;
-    fa.done = s->d_done;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(s->grid, (n + s->warps - 1) / s->warps));
-    dev::k_foldin<<<grid, 32 * s->warps, s->smem, s->st>>>(fa);
+    fa.z = s->d_z;
+    fa.rows = s->d_rows;
+    fa.row_nnz = s->d_row_nnz;
+    fa.theta = s->h_theta;
+    if (nreq > nold) {
+        dev::k_fold_build<true><<<nreq - nold, 256, s->smem_build, s->st>>>(fa, nold);
+        CUDA_TRY(cudaGetLastError());
+    }
+    // few items: one or a few warps per CTA, so that they spread over the SMs
+    const int warps = (int)std::max<int64_t>(1, std::min<int64_t>(kFoldWarps, (n + s->num_sms - 1) / s->num_sms));
+    const int64_t ctas = warps < kFoldWarps ? (n + warps - 1) / warps : std::min<int64_t>(s->grid, (n + warps - 1) / warps);
+    dev::k_foldin<<<(int)ctas, 32 * warps, sizeof(float) * dev::kFoldWarpWords * warps, s->st>>>(fa);
     CUDA_TRY(cudaGetLastError());
     s->kernel_launches++;
-    std::vector<lda_server::Active> keep;
-    keep.reserve(s->active.size());
+    dev::k_fold_build<false><<<nreq, 256, s->smem_build, s->st>>>(fa, 0);
+    CUDA_TRY(cudaGetLastError());
+    size_t kept = 0;
     for (auto& a : s->active) {
-        if (a.sweep == s->sweeps - 1) {
-            CUDA_TRY(cudaMemcpyAsync(s->h_theta + (size_t)a.slot * s->m->K, s->d_theta + (size_t)a.slot * s->m->K,
-                                     sizeof(float) * s->m->K, cudaMemcpyDeviceToHost, s->st));
+        if (a.sweep++ == s->sweeps - 1) {
             a.last_step = k;
-            a.sweep++;
             s->finishing.push_back(a);
         } else {
-            a.sweep++;
-            keep.push_back(a);
+            s->active[kept++] = a;
         }
     }
-    s->active.swap(keep);
+    if (kept < s->active.size()) {
+        s->active.resize(kept);
+        s->table_stale = true;
+    }
     CUDA_TRY(cudaEventRecord(s->ev[k % kRing], s->st));
     s->inflight.push_back(k);
     s->steps++;
@@ -866,8 +890,7 @@ extern "C" int lda_server_get_topics(lda_server* s, uint32_t rid, uint16_t* out,
             if (a.sweep == 0) return fail(LDA_ERR_STATE, "request %u has not run a sweep yet", rid);
             CUDA_TRY(cudaSetDevice(s->device));
             CUDA_TRY(cudaStreamSynchronize(s->st));
-            const uint16_t* z = s->d_z + (size_t)(a.sweep & 1) * s->tok_cap;
-            CUDA_TRY(cudaMemcpy(out, z + a.off, sizeof(uint16_t) * a.len, cudaMemcpyDeviceToHost));
+            CUDA_TRY(cudaMemcpy(out, s->d_z + a.off, sizeof(uint16_t) * a.len, cudaMemcpyDeviceToHost));
             return LDA_OK;
         }
     return fail(LDA_ERR_STATE, "request %u is not active", rid);
