@@ -164,16 +164,68 @@ __device__ __forceinline__ int fold_lane_draw(const uint32_t* __restrict__ row, 
     return last >= 0 ? last : phi.mk;
 }
 
-// The row's count of topic k (0 when it has none), by binary search.
-__device__ __forceinline__ uint32_t row_count(const uint32_t* __restrict__ row, uint32_t nnz, uint32_t k) {
-    uint32_t lo = 0, hi = nnz;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if ((__ldg(row + mid) >> 16) < k) lo = mid + 1; else hi = mid;
+// The row's counts of topics k1 and k2 (0 when it has none), by one binary search for both.
+__device__ __forceinline__ void row_counts(const uint32_t* __restrict__ row, uint32_t nnz, uint32_t k1, uint32_t k2,
+                                           uint32_t& c1, uint32_t& c2) {
+    const uint32_t* p1 = row;
+    const uint32_t* p2 = row;
+    for (uint32_t n = nnz; n > 1u;) {
+        const uint32_t h = n >> 1;
+        const uint32_t e1 = __ldg(p1 + h), e2 = __ldg(p2 + h);
+        if ((e1 >> 16) <= k1) p1 += h;
+        if ((e2 >> 16) <= k2) p2 += h;
+        n -= h;
     }
-    if (lo >= nnz) return 0u;
-    const uint32_t e = __ldg(row + lo);
-    return (e >> 16) == k ? e & 0xffffu : 0u;
+    const uint32_t e1 = __ldg(p1), e2 = __ldg(p2);
+    c1 = (e1 >> 16) == k1 ? e1 & 0xffffu : 0u;
+    c2 = (e2 >> 16) == k2 ? e2 & 0xffffu : 0u;
+}
+
+// Q-bucket draws of the tokens in `todo` (words w, max topics mk, rests tt of the targets;
+// lane = token) for K <= 1024, where a lane of Q has one round of topics: warp_q_draw for
+// four tokens at a time, their loads and scans side by side.  The lane's own token's topic
+// goes to znew.
+constexpr int kFoldQ = 4;
+__device__ __forceinline__ void fold_q_draws(const FoldArgs& a, unsigned todo, uint32_t w, int mk, float tt, int& znew,
+                                             int lane) {
+    while (todo) {
+        int j[kFoldQ], m[kFoldQ], key[kFoldQ];
+        const float* prow[kFoldQ];
+        float QL[kFoldQ], QP[kFoldQ], t2[kFoldQ], cz[kFoldQ], P[kFoldQ];
+        int n = 0;
+#pragma unroll
+        for (int t = 0; t < kFoldQ; ++t) {
+            // past the last token the first is drawn again
+            j[t] = t == 0 || todo ? __ffs(todo) - 1 : j[0];
+            if (todo) ++n;
+            todo &= todo - 1u;
+            const uint32_t wj = __shfl_sync(FULL, w, j[t]);
+            m[t] = __shfl_sync(FULL, mk, j[t]);
+            QL[t] = __ldg(a.ql + (size_t)wj * 32 + lane);
+            prow[t] = a.phi + (size_t)wj * a.K;
+        }
+#pragma unroll
+        for (int t = 0; t < kFoldQ; ++t) QP[t] = warp_ks_scan(QL[t], lane);
+#pragma unroll
+        for (int t = 0; t < kFoldQ; ++t) {
+            const float ttj = __shfl_sync(FULL, tt, j[t]);
+            const unsigned cand = __ballot_sync(FULL, ttj < QP[t] && QL[t] > 0.0f), pos = __ballot_sync(FULL, QL[t] > 0.0f);
+            const int ls = cand ? __ffs(cand) - 1 : (pos ? 31 - __clz(pos) : 0);
+            const float prev = __shfl_sync(FULL, QP[t], ls > 0 ? ls - 1 : 0);
+            t2[t] = ls > 0 ? fsub(ttj, prev) : ttj;
+            key[t] = ls + 32 * lane;
+            cz[t] = key[t] < a.K && key[t] != m[t] ? __ldg(prow[t] + key[t]) : 0.0f;
+        }
+#pragma unroll
+        for (int t = 0; t < kFoldQ; ++t) P[t] = warp_ks_scan(fmul(a.alpha, cz[t]), lane);
+#pragma unroll
+        for (int t = 0; t < kFoldQ; ++t) {
+            const unsigned f = __ballot_sync(FULL, cz[t] > 0.0f && t2[t] < P[t]), v = __ballot_sync(FULL, cz[t] > 0.0f);
+            const int from = f ? __ffs(f) - 1 : 31 - __clz(v);
+            const int z = f || v ? __shfl_sync(FULL, key[t], from) : m[t];
+            if (t < n && lane == j[t]) znew = z;
+        }
+    }
 }
 
 // Lane sums of one row against kFoldWords words at a time, into their slots: lane l sums the
@@ -206,12 +258,25 @@ __device__ __forceinline__ void fold_rows(const FoldArgs& a, const uint32_t* __r
                 if (k[s] != mk[t]) acc[t] = ffma(c[s], v[t][s], acc[t]);
         }
         if (NS == 4) {
-            for (uint32_t q = 128u + (uint32_t)lane; q < nnz; q += 32u) {
-                const uint32_t e = __ldg(row + q), kk = e >> 16;
-                const float cc = u2f(e & 0xffffu);
+            for (uint32_t q = 128u; q < nnz; q += 128u) {
+                float cc[NS];
+                uint32_t kk[NS];
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    const uint32_t at = q + 32u * s + (uint32_t)lane;
+                    const uint32_t e = at < nnz ? __ldg(row + at) : 0u;
+                    cc[s] = u2f(e & 0xffffu);
+                    kk[s] = e >> 16;
+                }
 #pragma unroll
                 for (int t = 0; t < kFoldWords; ++t)
-                    if (kk != mk[t]) acc[t] = ffma(cc, __ldg(prow[t] + kk), acc[t]);
+#pragma unroll
+                    for (int s = 0; s < NS; ++s) v[t][s] = __ldg(prow[t] + kk[s]);
+#pragma unroll
+                for (int t = 0; t < kFoldWords; ++t)
+#pragma unroll
+                    for (int s = 0; s < NS; ++s)
+                        if (kk[s] != mk[t]) acc[t] = ffma(cc[s], v[t][s], acc[t]);
             }
         }
 #pragma unroll
@@ -224,18 +289,21 @@ __device__ __forceinline__ void fold_rows(const FoldArgs& a, const uint32_t* __r
 // sampler's groups (sample_groups) with every token its own word: the tokens are screened
 // thread-per-token, the request's row is summed against each unsettled token's word
 // (consecutive tokens of one word share a sum), and each token decides by itself.  What
-// bounds it is the gathers of phi, 4 KB a word at K=1024 from a matrix larger than L2: the
-// lane's row entries sit in registers for the whole item and four words' gathers are in
-// flight together.  (Rebuilding the request's counts and row for every item, and summing one
-// word at a time, took 350 us per sweep of 2,048 requests against 200 for this kernel and the
-// row builds.)
+// bounds it is the latency of the gathers of phi, 4 KB a word at K=1024 from a matrix larger
+// than L2: the lane's first four row entries sit in registers for the whole item, and four
+// words' gathers of four row steps are in flight together (16 loads; two words: 8.4 against
+// 8.1 ms per 2,048 requests, eight at 2 CTAs per SM: 10.6).  A warp takes one item, so that
+// the hardware's CTA scheduler balances the items, longest requests first (7.2 -> 6.7 ms).
+// With the request's counts and row rebuilt for every item and one word at a time, 2,048
+// requests of 30 sweeps took 27.3 ms, one of 900 tokens 1.81 ms (now 6.7 and 0.71).
 constexpr int kFoldWarpWords = 32 * kSlotWords + 64;
 __global__ void __launch_bounds__(256, 3) k_foldin(FoldArgs a) {
     extern __shared__ float smf[];
     const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* slots = smf + (size_t)kFoldWarpWords * wid;
     uint2* list = reinterpret_cast<uint2*>(slots + 32 * kSlotWords);
-    for (int r = blockIdx.x * warps + wid; r < a.nitems; r += gridDim.x * warps) {
+    const int r = blockIdx.x * warps + wid;
+    if (r < a.nitems) {
         const uint32_t ir = __ldg(a.item_req + r);
         const FoldReq it = a.reqs[ir >> 16];
         const uint32_t begin = (ir & 0xffffu) * a.item_tokens, end = min(begin + a.item_tokens, it.len);
@@ -262,7 +330,8 @@ __global__ void __launch_bounds__(256, 3) k_foldin(FoldArgs a) {
                 const uint32_t t2 = __ldg(a.top2 + w);
                 mk = (int)(t2 & 0xffffu);
                 const float4 ph = __ldg(a.phi4 + w);
-                const uint32_t cmax = row_count(row, nnz, t2 & 0xffffu), c2 = row_count(row, nnz, t2 >> 16);
+                uint32_t cmax, c2;
+                row_counts(row, nnz, t2 & 0xffffu, t2 >> 16, cmax, c2);
                 u = foldin_uniform(a.seed_lo, a.seed_hi, it.rid, sweep, pos);
                 pmax = fmul(fadd(u2f(cmax), a.alpha), ph.x);
                 const float shat = ffma(u2f(c2), ph.y, fmul(u2f(it.len - cmax - c2), ph.z));
@@ -289,9 +358,11 @@ __global__ void __launch_bounds__(256, 3) k_foldin(FoldArgs a) {
                 decide_tokens<false>(slots, mine ? ri : 0, mine, false, pmax, Q, u, lane, dr);
                 __syncwarp();  // the slots may be overwritten
             }
+            const unsigned qm = __ballot_sync(FULL, dr.kind == BR_Q);
             uint32_t qw = 0xffffffffu;
             float QL = 0.0f, QP = 0.0f;
-            for (unsigned b = __ballot_sync(FULL, dr.kind == BR_Q); b; b &= b - 1u) {
+            if (a.K <= 1024) fold_q_draws(a, qm, w, mk, dr.t, znew, lane);
+            else for (unsigned b = qm; b; b &= b - 1u) {
                 const int j = __ffs(b) - 1;
                 const uint32_t wj = __shfl_sync(FULL, w, j);
                 const int mkj = __shfl_sync(FULL, mk, j);
@@ -478,7 +549,7 @@ struct lda_server {
     lda_model* m = nullptr;
     int device = 0;
     cudaStream_t st = nullptr;
-    int sweeps = 30, max_active = 0, num_sms = 0, grid = 0;
+    int sweeps = 30, max_active = 0, num_sms = 0;
     uint32_t item_tokens = 32;
     uint64_t seed = 0;
     int64_t tok_cap = 0, max_items = 0;
@@ -491,6 +562,7 @@ struct lda_server {
     unsigned char* d_table = nullptr;
     unsigned char* h_table[kRing] = {};
     int64_t table_items = 0;  // of the table on the device
+    std::vector<int64_t> item_at;  // scratch of the item list's sort
     bool table_stale = true;
     cudaEvent_t ev[kRing] = {};
     uint32_t* h_words = nullptr;
@@ -659,17 +731,14 @@ extern "C" int lda_server_create(lda_model* m, int64_t max_tokens, int32_t max_a
     }
     s->free_iv[0] = max_tokens;
     for (int i = max_active - 1; i >= 0; --i) s->free_slots.push_back(i);
-    int max_smem = 0, per_sm = 0;
+    int max_smem = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
     CUDA_TRY(cudaDeviceGetAttribute(&s->num_sms, cudaDevAttrMultiProcessorCount, s->device));
     s->smem_build = ((size_t)dev::Hist<true>::words(m->K) + (size_t)(m->K + 31) / 32) * 4;
     if (s->smem_build > (size_t)max_smem) return fail(LDA_ERR_ARG, "K=%d does not fit in shared memory", m->K);
     CUDA_TRY(raise_smem_limit((const void*)dev::k_fold_build<true>, s->smem_build));
     CUDA_TRY(raise_smem_limit((const void*)dev::k_fold_build<false>, s->smem_build));
-    const size_t smem = sizeof(float) * dev::kFoldWarpWords * kFoldWarps;
-    CUDA_TRY(raise_smem_limit((const void*)dev::k_foldin, smem));
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)dev::k_foldin, 32 * kFoldWarps, smem));
-    s->grid = std::max(1, per_sm * s->num_sms);
+    CUDA_TRY(raise_smem_limit((const void*)dev::k_foldin, sizeof(float) * dev::kFoldWarpWords * kFoldWarps));
     CUDA_TRY(cudaStreamSynchronize(s->st));
     *out = s.release();
     return LDA_OK;
@@ -776,13 +845,26 @@ static int server_issue(lda_server* s) {
     if (s->table_stale) {
         dev::FoldReq* reqs = reinterpret_cast<dev::FoldReq*>(s->h_table[k % kRing]);
         uint32_t* items = reinterpret_cast<uint32_t*>(reqs + nreq);
+        // the longest requests' items first (their rows are the longest): a counting sort of
+        // the requests by their items
         int64_t n = 0;
+        std::vector<int64_t>& at = s->item_at;
+        at.assign((65535 + T - 1) / T + 1, 0);
         for (int r = 0; r < nreq; ++r) {
             const auto& a = s->active[r];
-            const uint32_t nitems = (a.len + T - 1) / T;
             reqs[r] = dev::FoldReq{(uint32_t)a.off, a.len, a.rid, a.start, (uint32_t)a.slot, 0u, 0u, 0u};
-            const uint32_t tag = (uint32_t)r << 16;
-            for (uint32_t j = 0; j < nitems; ++j) items[n++] = tag | j;
+            at[(a.len + T - 1) / T] += (a.len + T - 1) / T;
+        }
+        for (size_t b = at.size(); b-- > 0;) {
+            const int64_t c = at[b];
+            at[b] = n;
+            n += c;
+        }
+        for (int r = 0; r < nreq; ++r) {
+            const uint32_t nitems = (s->active[r].len + T - 1) / T, tag = (uint32_t)r << 16;
+            uint32_t* out = items + at[nitems];
+            for (uint32_t j = 0; j < nitems; ++j) out[j] = tag | j;
+            at[nitems] += nitems;
         }
         CUDA_TRY(cudaMemcpyAsync(s->d_table, reqs, sizeof(dev::FoldReq) * (size_t)nreq + sizeof(uint32_t) * (size_t)n,
                                  cudaMemcpyHostToDevice, s->st));
@@ -817,8 +899,7 @@ static int server_issue(lda_server* s) {
     }
     // few items: one or a few warps per CTA, so that they spread over the SMs
     const int warps = (int)std::max<int64_t>(1, std::min<int64_t>(kFoldWarps, (n + s->num_sms - 1) / s->num_sms));
-    const int64_t ctas = warps < kFoldWarps ? (n + warps - 1) / warps : std::min<int64_t>(s->grid, (n + warps - 1) / warps);
-    dev::k_foldin<<<(int)ctas, 32 * warps, sizeof(float) * dev::kFoldWarpWords * warps, s->st>>>(fa);
+    dev::k_foldin<<<(int)((n + warps - 1) / warps), 32 * warps, sizeof(float) * dev::kFoldWarpWords * warps, s->st>>>(fa);
     CUDA_TRY(cudaGetLastError());
     s->kernel_launches++;
     dev::k_fold_build<false><<<nreq, 256, s->smem_build, s->st>>>(fa, 0);
