@@ -33,13 +33,13 @@ struct BatchArgs {
     const StatsArgs* st;
     const DtArgs* dt;
     const SampleArgs* sm;
-    const uint2* wt_work;  // {model, word tile}
+    const uint4* wt_work;  // {model, first word tile, word tiles, 0}
     int n_wt;
     const uint4* st_work;  // {model, first word, words, 0}
     int n_st;
     const uint4* dt_work;  // {model, first doc, docs, 0}
     int n_dt;
-    const uint2* sm_work;  // {model, sampler tile}
+    const uint4* sm_work;  // {model, first sampler tile, sampler tiles, 0}
     int n_sm;
     unsigned* counters;    // [4] work counters of the stages, zeroed at the start of a sweep
     const uint32_t* sweeps_done;  // sweeps this batch has begun: with a model's base iteration, its iteration
@@ -74,9 +74,10 @@ __global__ void __launch_bounds__(256) kb_wt(BatchArgs b) {
     for (;;) {
         const int i = grab(b.counters + 0, lane);
         if (i >= b.n_wt) break;
-        const uint2 w = b.wt_work[i];
-        const WtArgs& a = b.wt[w.x];
-        wt_tile(a, a.tiles[w.y], Hist<false>{hist}, bits, reinterpret_cast<unsigned*>(a.n_k), lane);
+        const uint4 w = b.wt_work[i];
+        const WtArgs a = b.wt[w.x];
+        for (uint32_t t = w.y; t < w.y + w.z; ++t)
+            wt_tile(a, a.tiles[t], Hist<false>{hist}, bits, reinterpret_cast<unsigned*>(a.n_k), lane);
     }
 }
 
@@ -118,18 +119,20 @@ __global__ void __launch_bounds__(256) kb_stats(BatchArgs b) {
     float* col = smf + (size_t)stats_warp_words(b.Kmax) * wid;
     int cur = -1;
     bool clean = false;
+    NoTokenStats none;
     for (;;) {
         const int i = grab(b.counters + 1, lane);
         if (i >= b.n_st) break;
         const uint4 u = b.st_work[i];
-        const StatsArgs& a = b.st[u.x];
+        const StatsArgs a = b.st[u.x];
         if ((int)u.x != cur) {
             cur = (int)u.x;
             clean = false;
+            none.have = false;
             __syncwarp();
         }
         uint32_t* bits = reinterpret_cast<uint32_t*>(col + ((a.K + 3) & ~3));
-        for (uint32_t w = u.y; w < u.y + u.z; ++w) word_stats_word(a, (int)w, col, bits, clean, lane);
+        for (uint32_t w = u.y; w < u.y + u.z; ++w) word_stats_word(a, (int)w, col, bits, clean, none, lane);
     }
 }
 
@@ -145,7 +148,7 @@ __global__ void __launch_bounds__(256) kb_dt(BatchArgs b) {
         const int i = grab(b.counters + 2, lane);
         if (i >= b.n_dt) break;
         const uint4 u = b.dt_work[i];
-        const DtArgs& a = b.dt[u.x];
+        const DtArgs a = b.dt[u.x];
         for (uint32_t d = u.y; d < u.y + u.z; ++d) dt_doc(a, d, Hist<false>{hist}, bits, lane);
     }
 }
@@ -167,7 +170,7 @@ __global__ void __launch_bounds__(256, 3) kb_sample(BatchArgs b) {
     while (i < b.n_sm) {
         int next = 0;
         if (lane == 0) next = (int)atomicAdd(b.counters + 3, 1u);
-        const uint2 w = b.sm_work[i];
+        const uint4 w = b.sm_work[i];
         if ((int)w.x != cur) {
             __syncwarp();
             if (ca && lane < C_NUM && ctr[lane]) atomicAdd(ca->ctr + lane, (unsigned long long)ctr[lane]);
@@ -178,7 +181,8 @@ __global__ void __launch_bounds__(256, 3) kb_sample(BatchArgs b) {
             clean = false;
         }
         const SampleArgs& a = *ca;
-        sample_tile<LL, QB>(a, (int)w.y, a.tiles[w.y], a.iter + done, col, slots, clean, ctr, lane);
+        for (uint32_t t = w.y; t < w.y + w.z; ++t)
+            sample_tile<LL, QB>(a, (int)t, a.tiles[t], a.iter + done, col, slots, clean, ctr, lane);
         i = __shfl_sync(FULL, next, 0);
     }
     __syncwarp();
@@ -260,8 +264,7 @@ struct lda_batch {
     DevBuf<dev::DtArgs> dt;
     DevBuf<dev::SampleArgs> sm;
     DevBuf<dev::RecipOut> rout;
-    DevBuf<uint2> wt_work, sm_work;
-    DevBuf<uint4> st_work, dt_work;
+    DevBuf<uint4> wt_work, sm_work, st_work, dt_work;
     DevBuf<dev::ZeroSeg> zero;
     DevBuf<int*> errs;
     DevBuf<int4> sub_tiles;      // sampler tiles split to tile_tokens
@@ -311,6 +314,15 @@ static int occupancy(const void* fn, int threads, size_t smem, int num_sms, int*
     return LDA_OK;
 }
 
+#ifndef LDA_RUN_TOKENS
+#define LDA_RUN_TOKENS 256
+#endif
+#ifndef LDA_RUN_TILES
+#define LDA_RUN_TILES 16
+#endif
+constexpr int kRunTokens = LDA_RUN_TOKENS;  // most tokens of a run of small tiles
+constexpr int kRunTiles = LDA_RUN_TILES;    // most tiles of a run
+
 // Builds the tables, work lists and launch shapes for the current tuning.
 static int batch_build(lda_batch* b) {
     const int M = (int)b->trainers.size();
@@ -353,29 +365,40 @@ static int batch_build(lda_batch* b) {
         errs.push_back(v.wt.err);
     }
     // work lists
-    std::vector<uint2> wt_work, sm_work;
+    // A word-topic or sampler item is one tile, or a run of one model's small tiles (its
+    // lists are largest first): a claim, the model's arguments, its column of a word without
+    // tokens and the flush of its counters are then paid once per run.  (An average sampler
+    // tile of the 512-model workload has 20 tokens, and the next tile that a warp claims is
+    // nearly always another model's.)
+    std::vector<uint4> wt_work, sm_work;
     std::vector<uint4> st_work, dt_work;
     std::vector<int> wt_cnt, sm_cnt;
+    auto add_runs = [](std::vector<uint4>& work, std::vector<int>& cnt, int m, int64_t n, int most, auto tokens) {
+        for (int64_t j = 0; j < n;) {
+            int64_t e = j;
+            int sum = 0;
+            do sum += tokens(e++);
+            while (e < n && e - j < kRunTiles && sum + tokens(e) <= most);
+            work.push_back(make_uint4((unsigned)m, (unsigned)j, (unsigned)(e - j), 0u));
+            cnt.push_back(sum);
+            j = e;
+        }
+    };
     for (int m = 0; m < M; ++m) {
         const TrainerView& v = b->views[m];
-        for (int j = 0; j < v.n_wtiles; ++j) {
-            wt_work.push_back(make_uint2((unsigned)m, (unsigned)j));
-            wt_cnt.push_back(v.w_tiles[j].z);
-        }
-        for (int64_t j = 0; j < sub_base[m + 1] - sub_base[m]; ++j) {
-            sm_work.push_back(make_uint2((unsigned)m, (unsigned)j));
-            sm_cnt.push_back(sub[sub_base[m] + j].z);
-        }
+        add_runs(wt_work, wt_cnt, m, v.n_wtiles, kRunTokens, [&](int64_t j) { return v.w_tiles[j].z; });
+        add_runs(sm_work, sm_cnt, m, sub_base[m + 1] - sub_base[m], std::min(tu.tile_tokens, kRunTokens),
+                 [&](int64_t j) { return sub[sub_base[m] + j].z; });
         for (int64_t w = 0; w < v.V; w += 32) st_work.push_back(make_uint4((unsigned)m, (unsigned)w, (unsigned)std::min<int64_t>(32, v.V - w), 0u));
         for (int64_t d = 0; d < v.D; d += 16) dt_work.push_back(make_uint4((unsigned)m, (unsigned)d, (unsigned)std::min<int64_t>(16, v.D - d), 0u));
     }
     if (tu.schedule == 0) {
         // largest tiles first across all models (each model's lists are already largest first)
-        auto by_size = [](std::vector<uint2>& work, const std::vector<int>& cnt) {
+        auto by_size = [](std::vector<uint4>& work, const std::vector<int>& cnt) {
             std::vector<size_t> idx(work.size());
             std::iota(idx.begin(), idx.end(), 0);
             std::stable_sort(idx.begin(), idx.end(), [&](size_t x, size_t y) { return cnt[x] > cnt[y]; });
-            std::vector<uint2> out(work.size());
+            std::vector<uint4> out(work.size());
             for (size_t i = 0; i < idx.size(); ++i) out[i] = work[idx[i]];
             work.swap(out);
         };

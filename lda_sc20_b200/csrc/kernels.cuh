@@ -550,8 +550,9 @@ __global__ void __launch_bounds__(256) k_word_stats(StatsArgs a) {
     float* col = smf + (size_t)stats_warp_words(a.K) * wid;
     uint32_t* bits = reinterpret_cast<uint32_t*>(col + ((a.K + 3) & ~3));
     bool clean = false;
+    NoTokenStats none;
     for (int w = a.wlo + blockIdx.x * warps + wid; w < a.V; w += gridDim.x * warps)
-        word_stats_word(a, w, col, bits, clean, lane);
+        word_stats_word(a, w, col, bits, clean, none, lane);
 }
 
 // Word statistics of dense words above kLargeK topics: warp per word, phi formed on the fly

@@ -241,8 +241,17 @@ __host__ __device__ __forceinline__ int stats_warp_words(int K) { return ((K + 3
 // `clean`, gets the word's topics written over it for the serial Q sums and put back after.
 // What is left per topic is one shared load and one fmaf (42 instructions before: 1,357 per
 // word at K=1024).
+//
+// Words without tokens all have the same statistics: a warp keeps the ones it forms first
+// (`none`; one corpus and sweep).
+struct NoTokenStats {
+    bool have = false;
+    uint32_t top2 = 0, k3 = 0;
+    float4 phi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float ql = 0.0f;
+};
 __device__ __forceinline__ void word_stats_word(const StatsArgs& a, int w, float* col, uint32_t* bits, bool& clean,
-                                                int lane) {
+                                                NoTokenStats& none, int lane) {
     const int K = a.K;
     if (w < a.Vd) {
         const int* row = a.dwt + (size_t)w * K;
@@ -255,6 +264,15 @@ __device__ __forceinline__ void word_stats_word(const StatsArgs& a, int w, float
     }
     const uint32_t* ent = a.swt_ent + __ldg(a.swt_off + (w - a.Vd));
     const uint32_t nnz = __ldg(a.swt_nnz + (w - a.Vd));
+    if (nnz == 0u && none.have) {
+        a.st_ql[(size_t)w * 32 + lane] = none.ql;
+        if (lane == 0) {
+            a.st_top2[w] = none.top2;
+            a.st_k3[w] = none.k3;
+            a.st_phi[w] = none.phi;
+        }
+        return;
+    }
     if (!clean) {
         for (int k = lane; k < K; k += 32) col[k] = fmul(a.beta, __ldg(a.recip + k));
         for (int i = lane; i < (K + 31) >> 5; i += 32) bits[i] = 0u;
@@ -282,11 +300,20 @@ __device__ __forceinline__ void word_stats_word(const StatsArgs& a, int w, float
 #pragma unroll 8
     for (int k = lane; k < K; k += 32) ql = ffma(a.alpha, col[k], ql);
     const float Q = __shfl_sync(FULL, warp_ks_scan(ql, lane), 31);
+    const uint32_t top2 = ((uint32_t)kk[1] << 16) | (uint32_t)k1;
+    const float4 ph = make_float4(v[0], v[1], v[2], Q);
     a.st_ql[(size_t)w * 32 + lane] = ql;
     if (lane == 0) {
-        a.st_top2[w] = ((uint32_t)kk[1] << 16) | (uint32_t)k1;
+        a.st_top2[w] = top2;
         a.st_k3[w] = (uint32_t)kk[2];
-        a.st_phi[w] = make_float4(v[0], v[1], v[2], Q);
+        a.st_phi[w] = ph;
+    }
+    if (nnz == 0u) {
+        none.have = true;
+        none.top2 = top2;
+        none.k3 = (uint32_t)kk[2];
+        none.phi = ph;
+        none.ql = ql;
     }
     __syncwarp();
     clean = nnz <= (uint32_t)K >> 2;
