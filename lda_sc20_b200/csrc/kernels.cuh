@@ -676,14 +676,31 @@ __host__ __device__ __forceinline__ size_t dense_large_smem(int K, int warps, in
            (LDA_QTAB ? (size_t)32 * qtab_rounds(K) * sizeof(float2) : 0) + (size_t)warps * row_state_words(nslots) * 4;
 }
 
+// Warps per CTA of the two samplers and the CTAs per SM they are compiled for.  Dense: the
+// CTAs share the SM's registers four ways (64 a thread) so that one CTA's column build and
+// tile end overlap the others' sampling; fewer, larger CTAs with more row slots lose (10M
+// tokens at K=10,000: 4.79 ms per sweep against 5.05 with two CTAs of 16 warps, 5.07 with
+// three of 8).  Sparse: the reciprocals (41 KB at K=10,000) are the CTA's, so two CTAs of 12
+// warps hold as many warps as three of 8, and 80 registers a thread avoid 130 bytes of
+// spills (5.40 -> 4.79 ms with the dense kernel as it is; 16 warps at 64 registers 5.6).
+#ifndef LDA_DENSE_WARPS
+#define LDA_DENSE_WARPS 8
+#endif
 #ifndef LDA_DENSE_LARGE_MIN_BLOCKS
 #define LDA_DENSE_LARGE_MIN_BLOCKS 4
 #endif
+#ifndef LDA_SPARSE_WARPS
+#define LDA_SPARSE_WARPS 12
+#endif
+#ifndef LDA_SPARSE_LARGE_MIN_BLOCKS
+#define LDA_SPARSE_LARGE_MIN_BLOCKS 2
+#endif
+constexpr int kDenseWarps = LDA_DENSE_WARPS, kSparseWarps = LDA_SPARSE_WARPS;
 
 // The sparse-word sampler keeps each word's Qw rounds' table in registers (lane r: round
 // r), so a Q draw evaluates the one round that holds its target instead of walking them.
 template <bool LL, int QB>
-__global__ void __launch_bounds__(256, LDA_SPARSE_LARGE_MIN_BLOCKS) k_sample_sparse_large(SampleArgs a) {
+__global__ void __launch_bounds__(32 * kSparseWarps, LDA_SPARSE_LARGE_MIN_BLOCKS) k_sample_sparse_large(SampleArgs a) {
     extern __shared__ float smf[];
     const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int bw = large_bit_words(a.K), pw = large_pre_words(a.K);
@@ -756,7 +773,7 @@ __global__ void __launch_bounds__(256, LDA_SPARSE_LARGE_MIN_BLOCKS) k_sample_spa
 }
 
 template <bool LL, int QB>
-__global__ void __launch_bounds__(256, LDA_DENSE_LARGE_MIN_BLOCKS) k_sample_dense_large(SampleArgs a) {
+__global__ void __launch_bounds__(32 * kDenseWarps, LDA_DENSE_LARGE_MIN_BLOCKS) k_sample_dense_large(SampleArgs a) {
     extern __shared__ float smf[];
     __shared__ int s_tile;
     __shared__ uint32_t s_group;  // plain sweeps: the tile's next 32-token group

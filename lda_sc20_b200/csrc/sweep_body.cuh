@@ -699,9 +699,6 @@ constexpr int kSampleWarps = LDA_SAMPLE_WARPS;
 #ifndef LDA_SAMPLE_LL0_MIN_BLOCKS
 #define LDA_SAMPLE_LL0_MIN_BLOCKS 3
 #endif
-#ifndef LDA_SPARSE_LARGE_MIN_BLOCKS
-#define LDA_SPARSE_LARGE_MIN_BLOCKS 4
-#endif
 
 // The slots in which a warp keeps doc rows' lane sums: row slot s holds the 32 sums of one
 // row at [33 s, 33 s + 32), so that 32 threads reading element i of 32 different rows touch

@@ -44,9 +44,9 @@ constexpr int kDenseTileLarge = LDA_DENSE_TILE;  // most tokens per dense-word t
 #endif
 constexpr int kDenseTileLargeMin = LDA_DENSE_TILE_MIN;
 #ifndef LDA_DENSE_TILES_PER_CTA
-#define LDA_DENSE_TILES_PER_CTA 4
+#define LDA_DENSE_TILES_PER_CTA 1
 #endif
-constexpr int kLargeWarps = 8;                // warps per CTA of the large-K sampler kernels
+constexpr int kLargeWarps = 8;                // warps per CTA of the large-K sparse-word statistics
 // Tokens per dense word-topic tile: the corpus' tokens over twice the warps that fill the
 // GPU, within these bounds.  The upper one alone (16,384) left the rebuild waiting for the
 // one warp that walks the most frequent word's tile, 128 tokens per round of loads.
@@ -424,7 +424,8 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     } else {
         auto dense_bytes = [&](int ns) { return dev::dense_large_smem(T.K, T.dwarps, ns); };
         auto sparse_bytes = [&](int ns) { return dev::sparse_large_smem(T.K, T.pwarps, ns); };
-        T.dwarps = T.pwarps = kLargeWarps;
+        T.dwarps = dev::kDenseWarps;
+        T.pwarps = dev::kSparseWarps;
         while (T.dwarps > 1 && dense_bytes(1) > (size_t)max_smem) --T.dwarps;
         while (T.pwarps > 1 && sparse_bytes(1) > (size_t)max_smem) --T.pwarps;
         if (dense_bytes(1) > (size_t)max_smem || sparse_bytes(1) > (size_t)max_smem)
@@ -495,9 +496,10 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
         std::vector<int4> ct, cs;
         int64_t tile_ch = kSampleTile, tile_dense = kDenseTileLarge;
         if (T.large) {
-            // dense-word tiles: the chunk's dense tokens over kDenseTilesPerCta tiles per
-            // resident CTA.  A chunk of a smaller corpus would otherwise wait for the one
-            // CTA that holds the most frequent word's 8,192 tokens.
+            // dense-word tiles: at most the chunk's dense tokens per resident CTA.  A chunk of
+            // a smaller corpus would otherwise wait for the one CTA that holds the most
+            // frequent word's 8,192 tokens; smaller tiles form more columns (10M tokens at
+            // K=10,000: 4.54 ms per sweep; half of that size 4.64, a quarter 4.79).
             int64_t nd = 0;
             for (int64_t w = 0; w < T.Vd; ++w) nd += c->seg_cnt[(size_t)ch * V + w];
             const int64_t per = LDA_DENSE_TILES_PER_CTA * std::max<int64_t>(resident_dense, 1);
