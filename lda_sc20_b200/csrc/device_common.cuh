@@ -345,7 +345,7 @@ template <bool SLOTKEYS>
 struct ColSharedT {
     using Entry = uint32_t;  // a doc-row entry: (key << 16) | count
     // rows are loaded one ahead (row_load), which reads past their end
-    static constexpr bool kAhead = SLOTKEYS;
+    static constexpr bool kAhead = SLOTKEYS, kOwnMass = false;
     const float* col;
     __device__ __forceinline__ float operator()(int k) const { return col[col_skew(k)]; }
     __device__ __forceinline__ float row(uint32_t key) const {

@@ -622,46 +622,86 @@ k_sample_t(SampleArgs a) {
 // (sample_groups) on the same values as the per-warp column, so results are unchanged.
 // The threshold is kLargeK (sweep_body.cuh).
 
-// Sparse-word view without a column: the word's topics as a bitmap in shared memory, with
-// the number of set bits before each 32-topic word; a topic's count is read from the
-// word's row (ascending k), and phi_k is formed exactly as build_column forms it.
+// Sparse-word view without a column: beta * r_k for every topic in shared memory (the CTA's),
+// the word's topics as a bitmap with the number of them before each 32-topic word; a topic's
+// count is read from the word's row (ascending k), and phi_k is formed exactly as a column
+// forms it.  The max topic's bit is set too, so that one test finds every topic whose value
+// is not beta * r_k.
 struct ColBits {
     using Entry = uint32_t;  // a doc-row entry: (k << 16) | count
-    static constexpr bool kAhead = false;
+    static constexpr bool kAhead = false, kOwnMass = true;
     const uint32_t* bits;  // ceil(K/32) words
-    const uint16_t* pre;   // set bits before each word
+    const uint16_t* pre;   // the word's topics before each of them
     const uint32_t* ent;   // the word's row, (k << 16) | count
-    const float* r;        // reciprocals in the skewed layout: r_k at col_skew(k)
+    const float* base;     // beta * r_k in the skewed layout: at col_skew(k)
+    const float* __restrict__ recip;
     float beta;
     int maxK;
-    // Branch-free: (0 + beta) is beta exactly, so one formula gives phi_k for topics in
-    // and out of the word, and only the count's load is predicated.  The branch it replaces
-    // kept the four batched row lookups of lane_mass apart (K=10,000 corpus: samplers
-    // 115.7 -> 109.5 ms per sweep, the same topics).
+    bool extra;            // the max topic is not one of the word's
+    // phi_k of a topic with its bit set
+    __device__ __forceinline__ float marked(int k, uint32_t b) const {
+        if (k == maxK) return 0.0f;
+        uint32_t i = pre[k >> 5] + __popc(b & ((1u << (k & 31)) - 1u));
+        if (extra && (maxK >> 5) == (k >> 5) && maxK < k) --i;
+        return fmul(fadd(u2f(__ldg(ent + i) & 0xffffu), beta), __ldg(recip + k));
+    }
     __device__ __forceinline__ float operator()(int k) const {
-        const uint32_t b = bits[k >> 5], m = 1u << (k & 31);
-        const float rk = r[col_skew(k)];
-        uint32_t e = 0u;
-        if (b & m) e = __ldg(ent + pre[k >> 5] + __popc(b & (m - 1u)));
-        const float phi = fmul(fadd(u2f(e & 0xffffu), beta), rk);
-        return k == maxK ? 0.0f : phi;
+        const uint32_t b = bits[k >> 5];
+        return (b >> (k & 31)) & 1u ? marked(k, b) : base[col_skew(k)];
     }
     __device__ __forceinline__ float row(uint32_t key) const { return (*this)((int)key); }
     __device__ __forceinline__ int topic(uint32_t key) const { return (int)key; }
     __device__ __forceinline__ uint32_t key(uint32_t e) const { return e >> 16; }
     __device__ __forceinline__ float cnt(uint32_t e) const { return u2f(e & 0xffffu); }
+    // A lane's sum over a row's entries l, l + 32, ... (lane_mass): four steps' lookups first,
+    // then (seldom: a sparse word holds a few of the thousands of topics) the marked topics'
+    // values, so that no branch keeps the lookups apart.  One body for full and partial
+    // batches: with the straight-line tails of the column samplers and a lookup of marked
+    // topics in each, the kernel missed the instruction cache.
+    __device__ __forceinline__ float mass(const uint32_t* __restrict__ row, uint32_t lane, uint32_t nnz) const {
+        float acc = 0.0f;
+        for (uint32_t q = lane; q < nnz + lane; q += 128u) {
+            uint32_t e[4], hit = 0u, bw[4];
+            float ph[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) e[j] = q + 32u * j < nnz ? __ldg(row + q + 32u * j) : 0u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int k = (int)key(e[j]);
+                bw[j] = bits[k >> 5];
+                ph[j] = base[col_skew(k)];
+                hit |= ((bw[j] >> (k & 31)) & 1u) << j;
+            }
+            while (hit) {
+                const int j = __ffs(hit) - 1;
+                hit &= hit - 1u;
+                const uint32_t ej = j == 0 ? e[0] : j == 1 ? e[1] : j == 2 ? e[2] : e[3];
+                const uint32_t bj = j == 0 ? bw[0] : j == 1 ? bw[1] : j == 2 ? bw[2] : bw[3];
+                const float v = marked((int)key(ej), bj);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (i == j) ph[i] = v;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc = ffma(cnt(e[j]), ph[j], acc);
+        }
+        return acc;
+    }
 };
 
 __host__ __device__ __forceinline__ int large_bit_words(int K) { return (K + 31) >> 5; }
 __host__ __device__ __forceinline__ int large_pre_words(int K) { return ((K + 31) >> 5) + 1 & ~1; }
 
-// Shared memory of the sparse-word kernel: the reciprocals in the skewed column layout
-// (col_words(K) floats: a Q round's 32 topics k, k + 32, ... then sit in 32 banks), then
-// per warp the bitmap, then per warp the prefix counts (uint16, an even number per warp),
-// then per warp the counter row.
+// Shared memory of the sparse-word kernel: beta * r_k in the skewed column layout
+// (col_words(K) floats) and the smoothing table's round ends, then per warp the bitmap, the
+// prefix counts (uint16, an even number), the counter row, the row state and the 32 prefixes
+// of a one-round word's own Q terms.
+__host__ __device__ __forceinline__ int smooth_rounds(int K) { return (K + 31) >> 5; }
+__host__ __device__ __forceinline__ int sparse_large_warp_words(int K, int nslots) {
+    return ((large_bit_words(K) + large_pre_words(K) / 2 + C_NUM + 32 + 1) & ~1) + row_state_words(nslots);
+}
 __host__ __device__ __forceinline__ size_t sparse_large_smem(int K, int warps, int nslots) {
-    return (size_t)col_words(K) * 4 +
-           (size_t)warps * (large_bit_words(K) * 4 + large_pre_words(K) * 2 + C_NUM * 4 + row_state_words(nslots) * 4) + 8;
+    return (size_t)(col_words(K) + ((smooth_rounds(K) + 1) & ~1) + warps * sparse_large_warp_words(K, nslots)) * 4;
 }
 
 // Shared memory of the dense-word kernel: the shared column, the warps' counter rows and
@@ -704,20 +744,17 @@ __global__ void __launch_bounds__(32 * kSparseWarps, LDA_SPARSE_LARGE_MIN_BLOCKS
     extern __shared__ float smf[];
     const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int bw = large_bit_words(a.K), pw = large_pre_words(a.K);
-    float* r = smf;
-    float* rend = smf + col_words(a.K);
-    uint32_t* bits = reinterpret_cast<uint32_t*>(rend) + (size_t)bw * wid;
-    uint16_t* pre = reinterpret_cast<uint16_t*>(reinterpret_cast<uint32_t*>(rend) + (size_t)bw * warps) +
-                    (size_t)pw * wid;
-    uint32_t* ctr = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(reinterpret_cast<uint32_t*>(rend) +
-                                                                            (size_t)bw * warps) +
-                                                (size_t)pw * warps) +
-                    C_NUM * wid;
-    float* slots = reinterpret_cast<float*>(
-                       (reinterpret_cast<uintptr_t>(ctr + C_NUM * (warps - wid)) + 7) & ~(uintptr_t)7) +
-                   (size_t)row_state_words(a.nslots) * wid;
-    for (int k = threadIdx.x; k < a.K; k += blockDim.x)
-        r[col_skew(k)] = __fdiv_rn(1.0f, fadd(__int2float_rn(a.n_k[k]), a.Vbeta));
+    float* base = smf;
+    float* tend = smf + col_words(a.K);
+    const int rounds = smooth_rounds(a.K);
+    uint32_t* bits = reinterpret_cast<uint32_t*>(tend + ((rounds + 1) & ~1)) + (size_t)sparse_large_warp_words(a.K, a.nslots) * wid;
+    float* slots = reinterpret_cast<float*>(bits);
+    bits += row_state_words(a.nslots);
+    uint16_t* pre = reinterpret_cast<uint16_t*>(bits + bw);
+    uint32_t* ctr = bits + bw + pw / 2;
+    float* wp = reinterpret_cast<float*>(ctr + C_NUM);
+    for (int k = threadIdx.x; k < a.K; k += blockDim.x) base[col_skew(k)] = fmul(a.beta, __ldg(a.recip + k));
+    for (int i = threadIdx.x; i < rounds; i += blockDim.x) tend[i] = __ldg(a.smooth + min(a.K, 32 * i + 32) - 1);
     for (int i = lane; i < bw; i += 32) bits[i] = 0u;
     if (lane < C_NUM) ctr[lane] = 0u;
     __syncthreads();
@@ -745,15 +782,29 @@ __global__ void __launch_bounds__(32 * kSparseWarps, LDA_SPARSE_LARGE_MIN_BLOCKS
             if (e == 0 || (__ldg(ent + e - 1) >> 21) != (k >> 5)) pre[k >> 5] = (uint16_t)e;
         }
         __syncwarp();
+        const bool extra = !((bits[maxK >> 5] >> (maxK & 31)) & 1u);
+        __syncwarp();
         if (lane == 0) {
+            if (extra) bits[maxK >> 5] |= 1u << (maxK & 31);
             ctr[C_WNNZ] += nnz_w;
             ctr[C_TSPARSE] += 1u;
         }
         const float QP = warp_ks_scan(QL, lane);
         const float Q = __shfl_sync(FULL, QP, 31);
         __syncwarp();
-        const ColBits view{bits, pre, ent, r, a.beta, maxK};
-        SplitQ sq{ent, nnz_w, __shfl_sync(FULL, QL, 0), a.smooth, r, true};
+        const ColBits view{bits, pre, ent, base, a.recip, a.beta, maxK, extra};
+        SplitQ sq{ent, nnz_w, __shfl_sync(FULL, QL, 0), a.smooth, a.recip, false};
+        if (nnz_w <= 32u) {
+            // the one round's prefixes, for thread_split_draw
+            int key;
+            float term = 0.0f;
+            bool ok = false;
+            if ((uint32_t)lane < nnz_w) sq.slot((uint32_t)lane, maxK, a.alpha, key, term, ok);
+            wp[lane] = warp_ks_scan(term, lane);
+            sq.wp = wp;
+            sq.wok = __ballot_sync(FULL, ok);
+        }
+        sq.tend = tend;
         split_q_table(sq, maxK, a.alpha, lane);
         double ll = sample_groups<LL, QB, true>(a, (uint32_t)t.y, (uint32_t)t.z, 0u, 32u, a.iter,
                                                                     maxK, ph, QL, QP, Q, view, ctr, lane, slots,
@@ -765,6 +816,7 @@ __global__ void __launch_bounds__(32 * kSparseWarps, LDA_SPARSE_LARGE_MIN_BLOCKS
         }
         __syncwarp();
         for (uint32_t e = lane; e < nnz_w; e += 32) bits[(__ldg(ent + e) >> 16) >> 5] = 0u;
+        if (lane == 0) bits[maxK >> 5] = 0u;
         __syncwarp();
         tile = __shfl_sync(FULL, next, 0);
     }
@@ -777,6 +829,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, LDA_DENSE_LARGE_MIN_BLOCKS) 
     extern __shared__ float smf[];
     __shared__ int s_tile;
     __shared__ uint32_t s_group;  // plain sweeps: the tile's next 32-token group
+    __shared__ float s_qps[32];   // the word's Q prefixes
     const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* col = smf;
     uint32_t* ctr_all = reinterpret_cast<uint32_t*>(col + col_words(a.K));
@@ -856,11 +909,13 @@ __global__ void __launch_bounds__(32 * kDenseWarps, LDA_DENSE_LARGE_MIN_BLOCKS) 
         const float QL = __ldg(a.st_ql + (size_t)w * 32 + lane);
         const float QP = warp_ks_scan(QL, lane);
         const float Q = __shfl_sync(FULL, QP, 31);
+        if (threadIdx.x < 32) s_qps[lane] = QP;
+        __syncthreads();
         double ll = sample_groups<LL, QB, false>(a, (uint32_t)t.y, (uint32_t)t.z, 32u * wid,
                                                                      32u * warps, a.iter, maxK, ph, QL, QP, Q,
                                                                      ColShared{col}, ctr, lane, slots,
                                                                      qr ? qtab : nullptr, qr, nullptr,
-                                                                     LL ? nullptr : &s_group);
+                                                                     LL ? nullptr : &s_group, s_qps);
         if (LL) {
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) ll += __shfl_xor_sync(FULL, ll, off);

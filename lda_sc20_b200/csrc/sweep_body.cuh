@@ -589,6 +589,11 @@ struct SplitQ {
     float qcarry = 0.0f, qthr = 0.0f;
     const int* n_k = nullptr;
     float Vbeta = 0.0f;
+    // in shared memory, for thread_split_draw: the prefixes of a one-round word's terms (else
+    // null) with the entries whose term is positive, and the last entry of each of T's rounds
+    const float* wp = nullptr;
+    unsigned wok = 0u;
+    const float* tend = nullptr;
     __device__ __forceinline__ float rk(int k) const {
         return r ? r[skew ? col_skew(k) : k] : __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta));
     }
@@ -666,6 +671,58 @@ __device__ __forceinline__ int split_q_draw(const SplitQ& q, float t, int maxK, 
     const float t2 = fadd(t1, fmul(alpha, fmul(beta, q.rk(maxK))));
     const int z = warp_first_above(q.T, maxK + 1, K, t2, lane);
     return z >= 0 ? z : (maxK == K - 1 ? K - 2 : K - 1);
+}
+
+// split_q_draw thread per token (t, and whether to draw, differ by lane), with binary
+// searches in the word's prefixes and in T (its round ends first).  The searches compare
+// fewer places than split_q_draw's; places may be out of order by rounding, a prefix by
+// (1 + 2^-24)^5 (thread_crossing) and T's entries by less than 16 units of 2^-24 (a round's
+// prefixes as any, and each carry is at least every sum it is formed from but for that), so
+// a target that close to a neighbour is `unsure` and left to split_q_draw.  So is a draw from
+// the word's own topics when they take more than one round.
+__device__ __forceinline__ int thread_split_draw(const SplitQ& q, float t, int maxK, int K, float alpha, float beta,
+                                                 bool& unsure) {
+    unsure = false;
+    if (t < q.Qw) {
+        if (!q.wp) {
+            unsure = true;
+            return maxK;
+        }
+        int e = 0;
+#pragma unroll
+        for (int h = 16; h >= 1; h >>= 1)
+            if (!(t < q.wp[e + h - 1])) e += h;
+        unsure = !(t < q.wp[e]) || !((q.wok >> e) & 1u) || (e > 0 && t < fmul(q.wp[e - 1], 1.0f + 0x1p-19f));
+        return (int)(__ldg(q.ent + min((uint32_t)e, q.nnz - 1u)) >> 16);
+    }
+    const float t1 = fsub(t, q.Qw);
+    const bool left = maxK > 0 && t1 < __ldg(q.T + maxK - 1);
+    const float x = left ? t1 : fadd(t1, fmul(alpha, fmul(beta, q.rk(maxK))));
+    const int start = left ? 0 : maxK + 1;
+    int lo = 0, hi = (K + 31) >> 5;
+    const int rounds = hi;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (x < q.tend[mid]) hi = mid; else lo = mid + 1;
+    }
+    if (lo == rounds) {
+        unsure = true;
+        return maxK;
+    }
+    hi = min(K, 32 * lo + 32) - 1;  // x < T[hi], the round's end
+    lo = 32 * lo;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (x < __ldg(q.T + mid)) hi = mid; else lo = mid + 1;
+    }
+    const int k = max(lo, start);
+    if (k >= K) {
+        unsure = true;
+        return maxK;
+    }
+    unsure = !(fmul(x, 1.0f + 0x1p-20f) < __ldg(q.T + k)) ||
+             (k > start && x < fmul(__ldg(q.T + k - 1), 1.0f + 0x1p-20f));
+    return k;
 }
 
 
@@ -858,6 +915,13 @@ __device__ __forceinline__ int warp_q_draw(const View& colz, float tt, float QL,
 // thread's about 130 per group, and a fifth of the draws are from Q at these sizes; with 32
 // topics per lane the thread's search costs as much as four tokens' draws by the warp.)
 constexpr int kThreadQ = kThreadQTopics / 32;
+// Above kLargeK, fewest Q-bucket draws of a group that run thread per token (three quarters
+// of the draws are from Q there while a model is young: K=10,000, 10M tokens 4.40 ms per
+// sweep; from 8 draws on 4.45, none 4.90).
+#ifndef LDA_THREAD_Q_MIN
+#define LDA_THREAD_Q_MIN 4
+#endif
+constexpr int kThreadQMin = LDA_THREAD_Q_MIN;
 
 // Q-bucket draws of all of a group's tokens with `act` (rest tt of the target each), thread
 // per token, for K <= 32 kThreadQ: the draws of warp_q_draw.  qps holds the word's 32 Q
@@ -893,6 +957,49 @@ __device__ __forceinline__ int thread_q_draw(const View& colz, const float* qps,
     return i >= 0 ? ls + 32 * i : maxK;
 }
 
+// Q-bucket draws above kThreadQTopics with the word's Q-round table (tab, `qrounds` pairs per
+// lane slot), thread per token: the lane, then the first round whose threshold exceeds the
+// rest of the target, then the crossing among that round's 32 topics, as warp_q_draw finds
+// them; `unsure` as thread_q_draw.
+template <class View>
+__device__ __forceinline__ int thread_q_draw_table(const View& colz, const float* qps, unsigned qpos, float tt, int K,
+                                                   float alpha, const float2* tab, int qrounds, bool& unsure) {
+    int ls = 0;
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1)
+        if (!(tt < qps[ls + h - 1])) ls += h;
+    float prev = ls > 0 ? qps[ls - 1] : 0.0f;
+    unsure = !(tt < qps[ls]) || tt < fmul(prev, 1.0f + 0x1p-19f) || !((qpos >> ls) & 1u);
+    const float t2 = ls > 0 ? fsub(tt, prev) : tt;
+    const int n = (K - ls + 31) / 32;  // the lane slot's topics
+    const float2* row = tab + ls * qrounds;
+    int r = 0;
+    float carry = 0.0f;
+    for (;; ++r) {
+        if (32 * r >= n) {
+            unsure = true;
+            return 0;
+        }
+        const float2 e = row[r];
+        if (t2 < e.y) {
+            carry = e.x;
+            break;
+        }
+    }
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = 32 * r + i < n ? fmul(alpha, colz(ls + 32 * (32 * r + i))) : 0.0f;
+    thread_ks_scan(v);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = fadd(carry, v[i]);
+    int i;
+    bool sure;
+    thread_crossing(v, t2, i, prev, sure);
+    const int k = ls + 32 * (32 * r + i);
+    unsure = unsure || !sure || 32 * r + i >= n || !(colz(min(k, K - 1)) > 0.0f);
+    return k;
+}
+
 // The 32-token groups g0, g0 + gstep, ... of the token range [start, start + cnt) of one
 // word (column view colz, max topic maxK, phi4 ph, Q partials QL / QP / Q of the word), or,
 // with a shared group counter gq, the groups the warp claims from it (32 tokens at a time,
@@ -910,7 +1017,8 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
                                                 uint32_t gstep, uint32_t iter, int maxK, const float4 ph, float QL,
                                                 float QP, float Q, const View& colz, uint32_t* ctr, int lane,
                                                 float* slots, const float2* qtab = nullptr, int qrounds = 0,
-                                                const SplitQ* sq = nullptr, uint32_t* gq = nullptr) {
+                                                const SplitQ* sq = nullptr, uint32_t* gq = nullptr,
+                                                float* qps = nullptr) {
     auto claim = [&]() {
         uint32_t v = 0;
         if (lane == 0) v = atomicAdd(gq, 32u);
@@ -925,9 +1033,9 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
     const E* rows = reinterpret_cast<const E*>(a.dt_ent);
     const int nslots = a.nslots;
     uint2* list = reinterpret_cast<uint2*>(slots + slot_words(nslots));
-    float* qps = reinterpret_cast<float*>(ctr + ((C_NUM + 3) & ~3));  // QB 0: the word's Q prefixes
     const unsigned qpos = __ballot_sync(FULL, QL > 0.0f);
     if (QB == 0) {
+        qps = reinterpret_cast<float*>(ctr + ((C_NUM + 3) & ~3));  // the word's Q prefixes
         qps[lane] = QP;
         __syncwarp();
     }
@@ -1008,7 +1116,8 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
                 } else {
                     for (; i < n; ++i, out += kSlotWords) {
                         const uint2 q = list[r0 + i];
-                        *out = lane_mass(rows + q.x, (uint32_t)lane, q.y, colz);
+                        if constexpr (SPLIT && View::kOwnMass) *out = colz.mass(rows + q.x, (uint32_t)lane, q.y);
+                        else *out = lane_mass(rows + q.x, (uint32_t)lane, q.y, colz);
                     }
                 }
                 __syncwarp();
@@ -1028,6 +1137,20 @@ __device__ __forceinline__ double sample_groups(const SampleArgs& a, uint32_t st
             const int zq = thread_q_draw(colz, qps, qpos, dr.t, a.K, a.alpha, maxK, unsure);
             if (dr.kind == BR_Q) znew = zq;
             by_warp = __ballot_sync(FULL, dr.kind == BR_Q && unsure);
+        }
+        if (SPLIT && sq->tend && __popc(qm) >= kThreadQMin) {
+            bool unsure = false;
+            int zq = maxK;
+            if (dr.kind == BR_Q) zq = thread_split_draw(*sq, dr.t, maxK, a.K, a.alpha, a.beta, unsure);
+            if (dr.kind == BR_Q) znew = zq;
+            by_warp = __ballot_sync(FULL, unsure);
+        }
+        if (QB > 1 && !SPLIT && qtab && __popc(qm) >= kThreadQMin) {
+            bool unsure = false;
+            int zq = maxK;
+            if (dr.kind == BR_Q) zq = thread_q_draw_table(colz, qps, qpos, dr.t, a.K, a.alpha, qtab, qrounds, unsure);
+            if (dr.kind == BR_Q) znew = zq;
+            by_warp = __ballot_sync(FULL, unsure);
         }
         for (; by_warp; by_warp &= by_warp - 1u) {
             const int j = __ffs(by_warp) - 1;
