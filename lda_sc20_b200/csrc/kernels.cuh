@@ -534,10 +534,26 @@ __global__ void __launch_bounds__(256) k_recip_order(const int* __restrict__ n_k
         recip[k] = __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta));
         if (base) base[col_skew(k)] = v;
     }
-    const int part = (K + 7) >> 3, j0 = wid * part, j1 = min(K, j0 + part);
+    // the CTA's own topics lie in [k0, k0 + 32): before them a topic ranks above with an equal
+    // value, after them only with a larger one
+    const int part = (((K + 7) >> 3) + 3) & ~3, j0 = min(K, wid * part), j1 = min(K, j0 + part);
+    const int k0 = blockIdx.x * 32, k1 = min(K, k0 + 32);
     int n = 0;
-#pragma unroll 8
-    for (int j = j0; j < j1; ++j) n += ranks_above(smf[j], j, v, k) ? 1 : 0;
+    for (int j = max(j0, k0); j < min(j1, k1); ++j) n += ranks_above(smf[j], j, v, k) ? 1 : 0;
+    const int a1 = min(j1, k0), b0 = max(j0, k1);
+    for (int j = j0; j + 4 <= a1; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(smf + j);
+        n += (x.x >= v) + (x.y >= v) + (x.z >= v) + (x.w >= v);
+    }
+    if (a1 > j0)
+        for (int j = j0 + ((a1 - j0) & ~3); j < a1; ++j) n += smf[j] >= v;
+    int j = b0;
+    for (; j < j1 && (j & 3); ++j) n += smf[j] > v;
+    for (; j + 4 <= j1; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(smf + j);
+        n += (x.x > v) + (x.y > v) + (x.z > v) + (x.w > v);
+    }
+    for (; j < j1; ++j) n += smf[j] > v;
     atomicAdd(&above[lane], n);
     __syncthreads();
     if (wid == 0 && k < K && above[lane] < kOrderList) order[above[lane]] = k;
@@ -555,19 +571,93 @@ __global__ void __launch_bounds__(256) k_word_stats(StatsArgs a) {
         word_stats_word(a, w, col, bits, clean, none, lane);
 }
 
-// Word statistics of dense words above kLargeK topics: warp per word, phi formed on the fly
-// from the word's count row and the CTA's reciprocals (no K-wide column per warp, which
-// left 4 warps per SM at K=10,000).  Results equal k_word_stats'.
-__global__ void __launch_bounds__(256) k_word_stats_dense_rows(StatsArgs a) {
+// Word statistics of dense words above kLargeK topics: CTA per word, with the word's column
+// in shared memory (K floats), formed by all threads.  The top three are merged over the
+// warps; the serial Q sums are warp 0's while the other warps take the rounds of the Q-round
+// table.  (A warp per word read its count row three times, 313 dependent steps each at
+// K=10,000: 141 us for 1,200 words, with one such CTA of 8 words per SM.)
+//
+// The Q-round table of word w (a.qtab): for lane slot ls and round r, the Kogge-Stone total
+// and largest prefix of alpha * colz(ls + 32 * (32 r + l)), l = 0..31 (slots past the lane
+// slot's last topic add 0, colz the column with its max topic zeroed), then per lane slot the
+// carries as the fadd chain of the totals: entry (ls, r) = (carry before round r, carry + the
+// round's largest prefix).  Lane ls scans its own slot's 32 terms of a round serially in
+// Kogge-Stone order.
+__global__ void __launch_bounds__(256) k_word_stats_dense_cta(StatsArgs a) {
     extern __shared__ float smf[];
-    const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* r = smf;
-    for (int k = threadIdx.x; k < a.K; k += blockDim.x) r[k] = __ldg(a.recip + k);
-    __syncthreads();
-    for (int w = a.wlo + blockIdx.x * warps + wid; w < a.V; w += gridDim.x * warps) {
-        const DenseRowPhi phi{a.dwt + (size_t)w * a.K, r, a.beta};
-        const int k1 = word_stats_from(a, w, phi, lane);
-        if (a.qtab) word_qtab(a, w, k1, phi, lane);
+    __shared__ float sv[24];
+    __shared__ int sk[24];
+    __shared__ float2 tot[16 * 32];  // qtab_rounds(K) <= 16
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, K = a.K;
+    float* col = smf;
+    for (int w = a.wlo + blockIdx.x; w < a.V; w += gridDim.x) {
+        const int* row = a.dwt + (size_t)w * K;
+        float a1 = -1.0f, a2 = -1.0f, a3 = -1.0f;
+        int i1 = 0x7fffffff, i2 = 0x7fffffff, i3 = 0x7fffffff;
+        for (int b = threadIdx.x; b < K; b += 4 * 256) {
+            int c[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) c[j] = b + 256 * j < K ? __ldg(row + b + 256 * j) : 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int k = b + 256 * j;
+                if (k >= K) break;
+                const float x = fmul(fadd(__int2float_rn(c[j]), a.beta), __ldg(a.recip + k));
+                col[k] = x;
+                top3_insert(x, k, a1, i1, a2, i2, a3, i3);
+            }
+        }
+        float v[3];
+        int kk[3];
+        warp_top3(a1, i1, a2, i2, a3, i3, v, kk);
+        if (lane < 3) {
+            sv[3 * wid + lane] = lane == 0 ? v[0] : lane == 1 ? v[1] : v[2];
+            sk[3 * wid + lane] = lane == 0 ? kk[0] : lane == 1 ? kk[1] : kk[2];
+        }
+        __syncthreads();
+        if (wid == 0) {
+            warp_top3(lane < 24 ? sv[lane] : -1.0f, lane < 24 ? sk[lane] : 0x7fffffff, -1.0f, 0x7fffffff, -1.0f,
+                      0x7fffffff, v, kk);
+            if (lane == 0) col[kk[0]] = 0.0f;  // fmaf(alpha, 0, q) is q: the max topic adds nothing
+        }
+        __syncthreads();
+        if (wid == 0) {
+            float ql = 0.0f;
+#pragma unroll 8
+            for (int k = lane; k < K; k += 32) ql = ffma(a.alpha, col[k], ql);
+            const float Q = __shfl_sync(FULL, warp_ks_scan(ql, lane), 31);
+            a.st_ql[(size_t)w * 32 + lane] = ql;
+            if (lane == 0) {
+                a.st_top2[w] = ((uint32_t)kk[1] << 16) | (uint32_t)kk[0];
+                a.st_k3[w] = (uint32_t)kk[2];
+                a.st_phi[w] = make_float4(v[0], v[1], v[2], Q);
+            }
+        } else if (a.qtab) {
+            const uint32_t n = (uint32_t)((K - lane + 31) / 32);
+            for (int r = wid - 1; r < a.qrounds; r += 7) {
+                float t[32];
+#pragma unroll
+                for (int l = 0; l < 32; ++l) {
+                    const uint32_t i = 32u * (uint32_t)r + (uint32_t)l;
+                    t[l] = i < n ? fmul(a.alpha, col[lane + 32 * (int)i]) : 0.0f;
+                }
+                thread_ks_scan(t);
+                float mx = t[0];
+#pragma unroll
+                for (int l = 1; l < 32; ++l) mx = fmaxf(mx, t[l]);
+                tot[32 * r + lane] = make_float2(t[31], mx);
+            }
+        }
+        __syncthreads();
+        if (wid == 1 && a.qtab) {
+            float2* tab = a.qtab + ((size_t)w * 32 + lane) * a.qrounds;
+            float carry = 0.0f;
+            for (int r = 0; r < a.qrounds; ++r) {
+                const float2 x = tot[32 * r + lane];
+                tab[r] = make_float2(carry, fadd(carry, x.y));
+                carry = fadd(carry, x.x);
+            }
+        }
     }
 }
 

@@ -210,15 +210,6 @@ __device__ __forceinline__ void top3_outside(const StatsArgs& a, const int* orde
     }
 }
 
-// phi_k of dense word w formed on the fly from its count row, the value its column holds
-struct DenseRowPhi {
-    const int* row;
-    const float* r;
-    float beta;
-    __device__ __forceinline__ float operator()(int k) const {
-        return fmul(fadd(__int2float_rn(__ldg(row + k)), beta), r[k]);
-    }
-};
 struct ColumnPhi {
     const float* col;
     __device__ __forceinline__ float operator()(int k) const { return col[k]; }
@@ -364,43 +355,6 @@ __device__ __forceinline__ int word_stats_from(const StatsArgs& a, int w, const 
     }
     __syncwarp();
     return k1;
-}
-
-// The Q-round table of dense word w (max topic k1) into a.qtab: for lane slot ls and round
-// r, the Kogge-Stone total and largest prefix of alpha * colz(ls + 32 * (32 r + l)),
-// l = 0..31 (slots past the lane slot's last topic add 0, colz the column with its max
-// topic zeroed), then per lane slot the carries as the fadd chain of the totals: entry
-// (ls, r) = (carry before round r, carry + the round's largest prefix).  The values
-// k_sample_dense_large forms from its shared column with warp scans; here lane ls scans
-// its own slot's 32 terms of a round serially in the same Kogge-Stone order (element l
-// adds element l - off at each step off = 1, 2, ..., 16), so that a round's loads read
-// 1,024 consecutive topics.
-template <class Phi>
-__device__ __forceinline__ void word_qtab(const StatsArgs& a, int w, int k1, const Phi& phi, int lane) {
-    const int R = a.qrounds;
-    float2* tab = a.qtab + (size_t)w * 32 * R;
-    const int ls = lane;
-    const uint32_t n = (uint32_t)((a.K - ls + 31) / 32);
-    float carry = 0.0f;
-    for (int r = 0; r < R; ++r) {
-        float v[32];
-#pragma unroll
-        for (int l = 0; l < 32; ++l) {
-            const uint32_t i = 32u * (uint32_t)r + (uint32_t)l;
-            const int k = ls + 32 * (int)i;
-            v[l] = i < n ? fmul(a.alpha, k == k1 ? 0.0f : phi(k)) : 0.0f;
-        }
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-            for (int l = 31; l >= off; --l) v[l] = fadd(v[l], v[l - off]);
-        }
-        float mx = v[0];
-#pragma unroll
-        for (int l = 1; l < 32; ++l) mx = fmaxf(mx, v[l]);
-        tab[ls * R + r] = make_float2(carry, fadd(carry, mx));
-        carry = fadd(carry, v[31]);
-    }
 }
 
 // ---------------------------------------------------------------- DT rebuild
@@ -570,7 +524,7 @@ struct SampleArgs {
     }
     // K > kLargeK: the smoothing table of the split Q bucket (k_smooth_table)
     const float* smooth = nullptr;
-    // K > kLargeK: the dense words' Q-round tables (word_qtab), or null
+    // K > kLargeK: the dense words' Q-round tables (k_word_stats_dense_cta), or null
     const float2* qtab_g = nullptr;
 };
 

@@ -735,8 +735,8 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
             return rc;
         T.grid_dense = std::min(g0, g1);
         T.grid_sparse = std::min(g2, g3);
-        CUDA_TRY(raise_smem_limit((const void*)dev::k_word_stats_dense_rows, (size_t)T.K * 4));
-        if ((rc = occupancy_grid((const void*)dev::k_word_stats_dense_rows, 256, (size_t)T.K * 4, T.num_sms,
+        CUDA_TRY(raise_smem_limit((const void*)dev::k_word_stats_dense_cta, (size_t)T.K * 4));
+        if ((rc = occupancy_grid((const void*)dev::k_word_stats_dense_cta, 256, (size_t)T.K * 4, T.num_sms,
                                  &T.grid_stats_dense)))
             return rc;
         T.smem_stats_sparse = dev::stats_sparse_smem(T.K, kLargeWarps);
@@ -956,8 +956,8 @@ extern "C" int lda_max_topic(lda_trainer* t) {
         ad.qtab = t->qtab_g;
         ad.qrounds = t->qrounds;
         if (ad.V > ad.wlo) {
-            const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(t->grid_stats_dense, (ad.V - ad.wlo + 7) / 8));
-            dev::k_word_stats_dense_rows<<<grid, 256, (size_t)t->K * 4, t->stream>>>(ad);
+            const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(t->grid_stats_dense, ad.V - ad.wlo));
+            dev::k_word_stats_dense_cta<<<grid, 256, (size_t)t->K * 4, t->stream>>>(ad);
             CUDA_TRY(cudaGetLastError());
         }
         if (a.V > std::max(t->Vd, a.wlo)) {
