@@ -297,10 +297,10 @@ struct lda_batch {
 };
 
 // Batched sampler instantiation: thread-per-token Q draws when every model has at most
-// kThreadQTopics topics, Q-bucket rounds four per batch when some model has K > 1024.
+// kThreadQTopics topics, Q-bucket rounds two per batch when some model has K > 1024.
 using BatchKernel = void (*)(dev::BatchArgs);
 static BatchKernel batch_sample_kernel(bool ll, int Kmax) {
-    if (Kmax > 1024) return ll ? dev::kb_sample<true, 4> : dev::kb_sample<false, 4>;
+    if (Kmax > 1024) return ll ? dev::kb_sample<true, 2> : dev::kb_sample<false, 2>;
     if (Kmax > dev::kThreadQTopics) return ll ? dev::kb_sample<true, 1> : dev::kb_sample<false, 1>;
     return ll ? dev::kb_sample<true, 0> : dev::kb_sample<false, 0>;
 }

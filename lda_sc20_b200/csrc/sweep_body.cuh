@@ -688,7 +688,7 @@ enum { C_TOK, C_EA, C_FULL, C_NNZ, C_MAX, C_S, C_Q, C_WNNZ, C_TDENSE, C_TSPARSE,
 // per SM it is compiled for: the register cap is 65536 / (32 * warps * blocks) per
 // thread.  A thread holds a row's 32 lane sums, so the plain kernels take 4 CTAs (64
 // registers; 5 CTAs of 48 spill: 1.96 against 1.92 ms per sweep at K=1024, and 3 leave too
-// few warps, 2.23 ms).  The K > 1024 kernels (four Q rounds per batch) and the LL kernel up
+// few warps, 2.23 ms).  The K > 1024 kernels (several Q rounds per batch) and the LL kernel up
 // to kThreadQTopics (its FP64 products; K=64: 119 -> 109 us per sweep) take 3; above, the LL
 // kernel spills 22 bytes at 4 and is still faster (K=1024: 701 against 755 us).
 // Branch taken by a token (counters only).

@@ -28,7 +28,10 @@ namespace {
 #define LDA_SAMPLE_TILE 1024
 #endif
 constexpr int kSampleTile = LDA_SAMPLE_TILE;  // most tokens per sampler tile (a word's column is rebuilt per tile)
-constexpr int kSampleTileMin = 64;            // fewest tokens per tile that a chunk's tile size goes down to
+// Fewest tokens per tile that a chunk's tile size goes down to: one group.  A corpus of
+// 200,000 tokens then spreads over all resident warps (K=64, ten sweeps 735 us with 64, 675
+// with 32).
+constexpr int kSampleTileMin = 32;
 #ifndef LDA_TILES_PER_WARP
 #define LDA_TILES_PER_WARP 2
 #endif
@@ -318,7 +321,8 @@ static int occupancy_grid(const void* fn, int threads, size_t smem, int num_sms,
 
 // The sampler instantiation for (LL mode, K, trainer's or caller's rows): up to
 // kThreadQTopics topics the trainer's Q-bucket draws run thread per token (QB 0); for K >
-// 1024 a lane's Q-bucket topics span several rounds, which are decided four per batch.
+// 1024 a lane's Q-bucket topics span several rounds, decided two per batch up to kLargeK (all
+// there are: K=1500 545 -> 533 us per sweep against four) and four above.
 // trainer: the trainer's own rows and tables; the allocation-free entry point's rows carry
 // topics as keys.
 using SampleKernel = void (*)(dev::SampleArgs);
@@ -327,7 +331,7 @@ static SampleKernel sample_kernel(bool ll, int K, bool trainer = true) {
         if (K > 1024) return ll ? dev::k_sample_t<true, 4, false> : dev::k_sample_t<false, 4, false>;
         return ll ? dev::k_sample_t<true, 1, false> : dev::k_sample_t<false, 1, false>;
     }
-    if (K > 1024) return ll ? dev::k_sample_t<true, 4, true> : dev::k_sample_t<false, 4, true>;
+    if (K > 1024) return ll ? dev::k_sample_t<true, 2, true> : dev::k_sample_t<false, 2, true>;
     if (K > dev::kThreadQTopics) return ll ? dev::k_sample_t<true, 1, true> : dev::k_sample_t<false, 1, true>;
     return ll ? dev::k_sample_t<true, 0, true> : dev::k_sample_t<false, 0, true>;
 }
