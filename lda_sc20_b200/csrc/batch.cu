@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(256, 3) kb_sample(BatchArgs b) {
     __syncwarp();
     const uint32_t done = *b.sweeps_done - 1u;  // sweeps before this one
     int cur = -1;
-    bool clean = false;
+    int held = kHoldsNone;
     const SampleArgs* ca = nullptr;
     int i = grab(b.counters + 3, lane);
     while (i < b.n_sm) {
@@ -178,11 +178,11 @@ __global__ void __launch_bounds__(256, 3) kb_sample(BatchArgs b) {
             if (lane < C_NUM) ctr[lane] = 0u;
             cur = (int)w.x;
             ca = b.sm + cur;
-            clean = false;
+            held = kHoldsNone;
         }
         const SampleArgs& a = *ca;
         for (uint32_t t = w.y; t < w.y + w.z; ++t)
-            sample_tile<LL, QB>(a, (int)t, a.tiles[t], a.iter + done, col, slots, clean, ctr, lane);
+            sample_tile<LL, QB>(a, (int)t, a.tiles[t], a.iter + done, col, slots, held, ctr, lane);
         i = __shfl_sync(FULL, next, 0);
     }
     __syncwarp();
@@ -315,7 +315,7 @@ static int occupancy(const void* fn, int threads, size_t smem, int num_sms, int*
 }
 
 #ifndef LDA_RUN_TOKENS
-#define LDA_RUN_TOKENS 256
+#define LDA_RUN_TOKENS 512
 #endif
 #ifndef LDA_RUN_TILES
 #define LDA_RUN_TILES 16

@@ -693,11 +693,11 @@ k_sample_t(SampleArgs a) {
     uint32_t* ctr = reinterpret_cast<uint32_t*>(slots + ((row_state_words(a.nslots) + 3) & ~3));
     if (lane < C_NUM) ctr[lane] = 0u;
     __syncwarp();
-    bool clean = false;
+    int held = kHoldsNone;
     int tile = __shfl_sync(FULL, claim_warp(a.tile_counter, a.ntiles, lane), 0);
     while (tile < a.ntiles) {
         const int next = claim_warp(a.tile_counter, a.ntiles, lane);
-        sample_tile<LL, QB, SKEWKEYS>(a, tile, a.tiles[tile], a.iter, col, slots, clean, ctr, lane);
+        sample_tile<LL, QB, SKEWKEYS>(a, tile, a.tiles[tile], a.iter, col, slots, held, ctr, lane);
         tile = __shfl_sync(FULL, next, 0);
     }
     __syncwarp();

@@ -1158,15 +1158,17 @@ __host__ __device__ __forceinline__ int sample_warp_words(int K, int nslots) {
 // One sampler tile (tile index `tile` of a.tiles, content t) with the word column in the
 // warp's shared `col` (col_words(K) floats, skewed layout), its row slots and its shared
 // counter row `ctr`.  QB: Q-bucket rounds decided per batch (1 for K <= 1024, where a lane
-// has one round of topics).  `clean`: whether `col` holds the column of a word without
-// tokens (a.base); a sparse word's column is that with the word's own topics written over
-// it, and a word with few of them puts the base values back when the tile is done, so that
-// the next sparse word costs its own entries instead of K.  (Forming every tile's column
+// has one round of topics; 0 for K <= kThreadQTopics).  `held`: the dense word whose column
+// `col` holds, or kHoldsBase for the column of a word without tokens (a.base): a sparse
+// word's column is that with the word's own topics written over it, and a word with few of
+// them puts the base values back when the tile is done, so that the next sparse word costs
+// its own entries instead of K, and a dense word's next tile nothing.  (Forming every tile's column
 // anew cost 160 warp instructions at K=1024, where an average tile has 31 tokens on a
 // corpus of 14M tokens.)  Without a.base the column is formed in full from n_k.
+constexpr int kHoldsNone = -1, kHoldsBase = -2;
 template <bool LL, int QB = 1, bool SKEWKEYS = true>
 __device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const int4 t, uint32_t iter, float* col,
-                                            float* slots, bool& clean, uint32_t* ctr, int lane) {
+                                            float* slots, int& held, uint32_t* ctr, int lane) {
     using View = ColSharedT<SKEWKEYS>;
     const int w = t.x;
     const uint32_t start = (uint32_t)t.y, cnt = (uint32_t)t.z;
@@ -1181,14 +1183,16 @@ __device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const
         nnz = __ldg(a.swt_nnz + (w - a.Vd));
     }
     __syncwarp();
+    bool clean = false;
     if (!sparse) {
         const int* row = a.dwt + (size_t)w * a.K;
-        for (int k = lane; k < a.K; k += 32)
-            col[col_skew(k)] = fmul(fadd(__int2float_rn(__ldg(row + k)), a.beta), a.rk<SKEWKEYS>(k));
-        clean = false;
+        if (!SKEWKEYS || held != w)
+            for (int k = lane; k < a.K; k += 32)
+                col[col_skew(k)] = fmul(fadd(__int2float_rn(__ldg(row + k)), a.beta), a.rk<SKEWKEYS>(k));
+        held = w;
     } else {
         if (SKEWKEYS) {
-            if (!clean) {
+            if (held != kHoldsBase) {
                 const float4* src = reinterpret_cast<const float4*>(a.base);
                 for (int i = lane; i < col_words(a.K) / 4; i += 32) reinterpret_cast<float4*>(col)[i] = __ldg(src + i);
             }
@@ -1202,6 +1206,7 @@ __device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const
             col[col_skew(k)] = fmul(fadd(u2f(en & 0xffffu), a.beta), a.rk<SKEWKEYS>(k));
         }
         clean = SKEWKEYS && nnz <= (uint32_t)a.K >> 3;
+        held = clean ? kHoldsBase : kHoldsNone;
     }
     __syncwarp();
     if (lane == 0) {
@@ -1214,10 +1219,10 @@ __device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const
     __syncwarp();
     double ll;
     bool split = false;
-    if constexpr (QB > 1) split = a.K > kLargeK && sparse;
+    if constexpr (QB > 1 && !SKEWKEYS) split = a.K > kLargeK && sparse;
     if (split) {
         // a sparse word above kLargeK topics: the split Q bucket
-        if constexpr (QB > 1) {
+        if constexpr (QB > 1 && !SKEWKEYS) {
             const SplitQ sq{ent, nnz, __shfl_sync(FULL, QL, 0), a.smooth, a.recip, false, 0, 0.0f, 0.0f, a.n_k, a.Vbeta};
             ll = sample_groups<LL, QB, true>(a, start, cnt, 0u, 32u, iter, maxK, ph, QL, QP, Q, View{col}, ctr, lane,
                                              slots, nullptr, 0, &sq);
