@@ -446,7 +446,7 @@ int lda_server_get_topics(lda_server* s, uint32_t rid, uint16_t* out, int32_t le
 /* Tokens per work item (a multiple of 32, default 32): a request is split into items of
  * this many tokens, each sampled by one warp.  Only while the server is idle. */
 int lda_server_set_item_tokens(lda_server* s, int32_t n);
-/* Steps issued and fold-in kernel launches since creation. */
+/* Steps issued and fold-in (sampling) kernel launches since creation, one a step. */
 int lda_server_stats(const lda_server* s, int64_t* steps, int64_t* kernel_launches);
 /* Real-time replay on an idle server: document i (words[doc_off[i]..doc_off[i+1]))
  * arrives arrival_s[i] seconds after the start (non-decreasing) and gets request id i;

@@ -728,12 +728,18 @@ struct ColBits {
     float beta;
     int maxK;
     bool extra;            // the max topic is not one of the word's
+    bool rich;             // the word holds more than a 32nd of the topics
+    // the place in the word's row of a topic with its bit set (not the max topic unless it is
+    // one of the word's)
+    __device__ __forceinline__ uint32_t place(int k, uint32_t b) const {
+        uint32_t i = pre[k >> 5] + __popc(b & ((1u << (k & 31)) - 1u));
+        if (extra && (maxK >> 5) == (k >> 5) && maxK < k) --i;
+        return i;
+    }
     // phi_k of a topic with its bit set
     __device__ __forceinline__ float marked(int k, uint32_t b) const {
         if (k == maxK) return 0.0f;
-        uint32_t i = pre[k >> 5] + __popc(b & ((1u << (k & 31)) - 1u));
-        if (extra && (maxK >> 5) == (k >> 5) && maxK < k) --i;
-        return fmul(fadd(u2f(__ldg(ent + i) & 0xffffu), beta), __ldg(recip + k));
+        return fmul(fadd(u2f(__ldg(ent + place(k, b)) & 0xffffu), beta), __ldg(recip + k));
     }
     __device__ __forceinline__ float operator()(int k) const {
         const uint32_t b = bits[k >> 5];
@@ -744,8 +750,11 @@ struct ColBits {
     __device__ __forceinline__ uint32_t key(uint32_t e) const { return e >> 16; }
     __device__ __forceinline__ float cnt(uint32_t e) const { return u2f(e & 0xffffu); }
     // A lane's sum over a row's entries l, l + 32, ... (lane_mass): four steps' lookups first,
-    // then (seldom: a sparse word holds a few of the thousands of topics) the marked topics'
-    // values, so that no branch keeps the lookups apart.  One body for full and partial
+    // then the marked topics' values, so that no branch keeps the lookups apart: one by one
+    // when they are seldom (most sparse words hold a few of the thousands of topics), and
+    // four at a time with their loads together when the word is rich in topics (3.5M tokens
+    // of 7,000 words at K=3000, early: one by one made a sweep a quarter slower than a
+    // predicated lookup per entry).  One body for full and partial
     // batches: with the straight-line tails of the column samplers and a lookup of marked
     // topics in each, the kernel missed the instruction cache.
     __device__ __forceinline__ float mass(const uint32_t* __restrict__ row, uint32_t lane, uint32_t nnz) const {
@@ -761,6 +770,22 @@ struct ColBits {
                 bw[j] = bits[k >> 5];
                 ph[j] = base[col_skew(k)];
                 hit |= ((bw[j] >> (k & 31)) & 1u) << j;
+            }
+            if (rich && hit) {
+                uint32_t en[4];
+                float rk[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int k = (int)key(e[j]);
+                    const bool in = (hit >> j) & 1u && k != maxK;
+                    en[j] = in ? __ldg(ent + place(k, bw[j])) : 0u;
+                    rk[j] = in ? __ldg(recip + k) : 0.0f;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if ((hit >> j) & 1u)
+                        ph[j] = (int)key(e[j]) == maxK ? 0.0f : fmul(fadd(u2f(en[j] & 0xffffu), beta), rk[j]);
+                hit = 0u;
             }
             while (hit) {
                 const int j = __ffs(hit) - 1;
@@ -796,14 +821,11 @@ __host__ __device__ __forceinline__ size_t sparse_large_smem(int K, int warps, i
 
 // Shared memory of the dense-word kernel: the shared column, the warps' counter rows and
 // their LL partials (the reciprocals are formed while the column is built).
-#ifndef LDA_QTAB
-#define LDA_QTAB 1
-#endif
 // Shared memory of the dense-word sampler: the word column, the warps' counter rows, their
 // LL partials and (when qtab_rounds(K) > 0) the Q-round table of 32 x R float2.
 __host__ __device__ __forceinline__ size_t dense_large_smem(int K, int warps, int nslots) {
     return (((size_t)col_words(K) * 4 + (size_t)warps * C_NUM * 4 + 7) & ~(size_t)7) + (size_t)warps * 8 +
-           (LDA_QTAB ? (size_t)32 * qtab_rounds(K) * sizeof(float2) : 0) + (size_t)warps * row_state_words(nslots) * 4;
+           (size_t)32 * qtab_rounds(K) * sizeof(float2) + (size_t)warps * row_state_words(nslots) * 4;
 }
 
 // Warps per CTA of the two samplers and the CTAs per SM they are compiled for.  Dense: the
@@ -882,7 +904,7 @@ __global__ void __launch_bounds__(32 * kSparseWarps, LDA_SPARSE_LARGE_MIN_BLOCKS
         const float QP = warp_ks_scan(QL, lane);
         const float Q = __shfl_sync(FULL, QP, 31);
         __syncwarp();
-        const ColBits view{bits, pre, ent, base, a.recip, a.beta, maxK, extra};
+        const ColBits view{bits, pre, ent, base, a.recip, a.beta, maxK, extra, nnz_w > (uint32_t)a.K >> 5};
         SplitQ sq{ent, nnz_w, __shfl_sync(FULL, QL, 0), a.smooth, a.recip, false};
         if (nnz_w <= 32u) {
             // the one round's prefixes, for thread_split_draw
@@ -926,7 +948,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, LDA_DENSE_LARGE_MIN_BLOCKS) 
     uint32_t* ctr = ctr_all + C_NUM * wid;
     double* wll = reinterpret_cast<double*>(
         (reinterpret_cast<uintptr_t>(ctr_all + C_NUM * warps) + 7) & ~(uintptr_t)7);
-    const int qr = LDA_QTAB ? qtab_rounds(a.K) : 0;
+    const int qr = qtab_rounds(a.K);
     float2* qtab = reinterpret_cast<float2*>(wll + warps);
     float* slots = reinterpret_cast<float*>(qtab + 32 * qr) + (size_t)row_state_words(a.nslots) * wid;
     if (lane < C_NUM) ctr[lane] = 0u;
@@ -961,38 +983,10 @@ __global__ void __launch_bounds__(32 * kDenseWarps, LDA_DENSE_LARGE_MIN_BLOCKS) 
             s_group = 0u;
         }
         __syncthreads();
-        if (qr && a.qtab_g) {
+        if (qr) {
             // the word's Q-round table, built by the word statistics
             const float2* src = a.qtab_g + (size_t)w * 32 * qr;
             for (int i = threadIdx.x; i < 32 * qr; i += blockDim.x) qtab[i] = __ldg(src + i);
-            __syncthreads();
-        } else if (qr) {
-            // the Q-round table of this word: for lane slot ls and round r, the KS total and the
-            // largest KS prefix of alpha * colz(ls + 32 * (32 r + l)), l = 0..31 (slots past the
-            // lane's last topic add 0), the terms and scan of warp_level2_rounds
-            const ColShared cv{col};
-            for (int job = wid; job < 32 * qr; job += warps) {
-                const int ls = job / qr, r = job - ls * qr;
-                const uint32_t n = (uint32_t)((a.K - ls + 31) / 32), i = 32u * (uint32_t)r + (uint32_t)lane;
-                const float term = i < n ? fmul(a.alpha, cv(ls + 32 * (int)i)) : 0.0f;
-                const float ks = warp_ks_scan(term, lane);
-                float mx = ks;
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(FULL, mx, off));
-                const float tot = __shfl_sync(FULL, ks, 31);
-                if (lane == 0) qtab[job] = make_float2(tot, mx);
-            }
-            __syncthreads();
-            // per lane slot: the carry before each round (the fadd chain of the round
-            // totals) and the round's threshold carry + largest prefix
-            if (threadIdx.x < 32) {
-                float carry = 0.0f;
-                for (int r = 0; r < qr; ++r) {
-                    const float2 tm = qtab[threadIdx.x * qr + r];
-                    qtab[threadIdx.x * qr + r] = make_float2(carry, fadd(carry, tm.y));
-                    carry = fadd(carry, tm.x);
-                }
-            }
             __syncthreads();
         }
         const float4 ph = __ldg(a.st_phi + w);

@@ -481,11 +481,13 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     // sparse-word tiles, each largest first).  For K <= kLargeK a chunk's tile size is
     // its tokens / (kTilesPerWarp x the sampler's resident warps), rounded up to 32 and
     // kept within [kSampleTileMin, kSampleTile].
-    int64_t resident_warps = 0, resident_dense = 0;
+    int64_t resident_warps = 0, resident_dense = 0, resident_sparse = 0;
     if (T.large) {
         int g = 0;
         if ((orc = occupancy_grid(dense_large_kernel(false), 32 * T.dwarps, T.smem_dense, T.num_sms, &g))) return orc;
         resident_dense = g;
+        if ((orc = occupancy_grid(sparse_large_kernel(false), 32 * T.pwarps, T.smem_sparse, T.num_sms, &g))) return orc;
+        resident_sparse = (int64_t)g * T.pwarps;
     }
     if (!T.large) {
         int g = 0;
@@ -507,6 +509,13 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
             int64_t nd = 0;
             for (int64_t w = 0; w < T.Vd; ++w) nd += c->seg_cnt[(size_t)ch * V + w];
             const int64_t per = LDA_DENSE_TILES_PER_CTA * std::max<int64_t>(resident_dense, 1);
+            // sparse-word tiles: as the tiles up to kLargeK topics (a small vocabulary's sparse
+            // words are long, and one warp takes a tile: 3.5M tokens of 7,000 words at K=3000
+            // 7.6 -> 1.6 ms per sweep, 2M of 3,000 at K=2049 6.2 -> 0.95; 10M at K=10,000 4.26 ->
+            // 4.07; at least 64 tokens 2.3, 0.95 and 4.07)
+            const int64_t ns = T.chunk_tok[ch + 1] - T.chunk_tok[ch] - nd;
+            const int64_t per_s = kTilesPerWarp * std::max<int64_t>(resident_sparse, 1);
+            tile_ch = std::min<int64_t>(kSampleTile, std::max<int64_t>(kSampleTileMin, ((ns + per_s - 1) / per_s + 31) / 32 * 32));
             tile_dense = std::min<int64_t>(kDenseTileLarge,
                                            std::max<int64_t>(kDenseTileLargeMin, ((nd + per - 1) / per + 255) / 256 * 256));
         }

@@ -99,6 +99,28 @@ def test_frequent_word_over_tile_edges(K, tokens):
     assert np.array_equal(tr.topic_totals(), o.topic_totals())
 
 
+# large K: sparse words that hold many of the topics (the lookups and Q draws of topic-rich
+# words), around the 32 topics of one round and a 32nd of the topics
+@pytest.mark.parametrize("ll", [False, True])
+@pytest.mark.parametrize("K,per_word", [(2049, 20), (2049, 40), (2049, 64), (2049, 66), (2049, 600), (4096, 2000)])
+def test_topic_rich_sparse_words_at_large_k(K, per_word, ll):
+    vocab = 24
+    rng = np.random.default_rng(per_word)
+    words = np.repeat(np.arange(vocab, dtype=np.int32), per_word)
+    rng.shuffle(words)
+    off = np.unique(np.append(np.arange(0, len(words), 150), len(words))).astype(np.int64)
+    c = L.Corpus.from_docs(off, words, vocab=vocab, K=K, num_chunks=2, dense_kind=2, dense_param=2.0)
+    tr = L.Trainer(c, K=K, alpha=0.1, seed=4)
+    o = _oracle(c, tr, K)
+    z = c.topics()
+    for it in range(3):
+        st = o.iterate(z, 4, it, ll=ll)
+        tr.iterate(1, ll=ll)
+        assert np.array_equal(tr.topics(), z), f"sweep {it}"
+        if ll:
+            assert abs(tr.loglik()[0] - st.loglik) <= 1e-9 * abs(st.loglik)
+
+
 # more requests than slots and a fragmented token pool: admissions and retirements change the
 # request table at nearly every step; rows beyond the 128 entries held in registers
 @pytest.mark.parametrize("K,active", [(300, 3), (1024, 5), (1025, 2)])
