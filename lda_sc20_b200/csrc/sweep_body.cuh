@@ -469,16 +469,15 @@ __device__ __forceinline__ void dt_doc(const DtArgs& a, uint32_t d, const H& his
 // ------------------------------------------------------------------- sampler
 // Warp per (word, token range) tile.  The word's phi column (phi_max zeroed) sits in
 // warp-private shared memory.  Each 32-token group is screened thread-per-token by the
-// max-topic bound.  Tokens the bound does not settle (all tokens in LL mode) are then
-// evaluated one at a time by the whole warp, with uniform control flow:
-//   S      lane l sums the doc row's entries l, l+32, l+64, ... (coalesced loads); one
-//          Kogge-Stone scan gives the lane prefixes; a doc row is evaluated once for
-//          consecutive tokens of the same (word, doc) in the tile;
-//   bucket a ballot over the lane prefixes picks the lane of an S-bucket draw; the
-//          in-lane draw (at most ceil(nnz/32) entries) runs afterwards thread-per-token,
-//          all the group's S-bucket tokens at once;
-//   Q      a ballot over the per-word lane prefixes of Q, then one topic per lane with a
-//          scan and a ballot (topics k = l, l+32, ..., 32 per round, carried).
+// max-topic bound; the tokens the bound does not settle (all tokens in LL mode) then need
+//   S      lane l's sum over the doc row's entries l, l+32, l+64, ... (coalesced loads, the
+//          whole warp per row), a Kogge-Stone scan of the 32 lane sums; a row is summed once
+//          for consecutive tokens of the same (word, doc) in the tile;
+//   bucket the first lane prefix above the target picks the lane of an S-bucket draw, then
+//          a draw among its (at most ceil(nnz/32)) entries; scans, searches and draws run
+//          thread-per-token, all the group's tokens at once (sample_groups);
+//   Q      a lane by the per-word lane prefixes of Q, then one of its topics k = l, l+32, ...
+//          (32 per round, carried).
 // Replaces UpdateProbKernelTrainD1, LDAKernelTrainD and LDAKernelTrain
 // (EZLDA/utility.cu:2680-3312, :1625-2103, :1217-1611) in one pass, with no
 // effective-token list in global memory and no spin lock.
@@ -721,14 +720,26 @@ constexpr int kThreadQTopics = 256;
 __host__ __device__ __forceinline__ int slot_words(int nslots) { return (kSlotWords * nslots + 1) & ~1; }
 __host__ __device__ __forceinline__ int row_state_words(int nslots) { return slot_words(nslots) + 64; }
 
-// The Kogge-Stone scan of N values held by one thread: element l adds element l - off at
-// each step off = 1, 2, ..., the additions of warp_ks_scan's first N lanes.
+// Two binary32 additions in one instruction, each rounded to nearest.
+__device__ __forceinline__ void fadd2(float& a0, float& a1, float b0, float b1) {
+    uint64_t a, b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(a0), "f"(a1));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(b0), "f"(b1));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
+}
+
+// The Kogge-Stone scan of N (even) values held by one thread: element l adds element l - off
+// at each step off = 1, 2, ..., the additions of warp_ks_scan's first N lanes, from step 2 on
+// two at a time.
 template <int N>
 __device__ __forceinline__ void thread_ks_scan(float (&v)[N]) {
 #pragma unroll
-    for (int off = 1; off < N; off <<= 1) {
+    for (int l = N - 1; l >= 1; --l) v[l] = fadd(v[l], v[l - 1]);
 #pragma unroll
-        for (int l = N - 1; l >= off; --l) v[l] = fadd(v[l], v[l - off]);
+    for (int off = 2; off < N; off <<= 1) {
+#pragma unroll
+        for (int l = N - 2; l >= off; l -= 2) fadd2(v[l], v[l + 1], v[l - off], v[l - off + 1]);
     }
 }
 
