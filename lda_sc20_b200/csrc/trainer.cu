@@ -50,9 +50,11 @@ constexpr int kDenseTileLargeMin = LDA_DENSE_TILE_MIN;
 #define LDA_DENSE_TILES_PER_CTA 1
 #endif
 constexpr int kLargeWarps = 8;                // warps per CTA of the large-K sparse-word statistics
-// Tokens per dense word-topic tile: the corpus' tokens over twice the warps that fill the
-// GPU, within these bounds.  The upper one alone (16,384) left the rebuild waiting for the
-// one warp that walks the most frequent word's tile, 128 tokens per round of loads.
+// Tokens per dense word-topic tile: the corpus' tokens over half the warps that fill the GPU,
+// within these bounds.  The upper one alone (16,384) left a small corpus' rebuild waiting for
+// the one warp that walks the most frequent word's tile, 128 tokens per round of loads (K=64,
+// 200K tokens 84 -> 27 us); a quarter of that size flushes too often on a large one (48M
+// tokens at K=1024 360 against 180 us).
 constexpr int kWtTileMax = 16384;
 #ifndef LDA_WT_TILE_MIN
 #define LDA_WT_TILE_MIN 2048
@@ -345,6 +347,19 @@ static const void* sparse_large_kernel(bool ll) {
     return ll ? (const void*)dev::k_sample_sparse_large<true, 4> : (const void*)dev::k_sample_sparse_large<false, 4>;
 }
 
+// Tiles by descending tokens, equal ones in their order: a counting sort (a tile has at most
+// 65,535 tokens).
+static void largest_first(std::vector<int4>& v) {
+    int most = 0;
+    for (const int4& t : v) most = std::max(most, t.z);
+    std::vector<size_t> at((size_t)most + 2, 0);
+    for (const int4& t : v) ++at[(size_t)(most - t.z) + 1];
+    for (size_t i = 1; i < at.size(); ++i) at[i] += at[i - 1];
+    std::vector<int4> out(v.size());
+    for (const int4& t : v) out[at[(size_t)(most - t.z)]++] = t;
+    v.swap(out);
+}
+
 // The row slots per warp of a sampler whose CTA takes bytes(slots) of shared memory: as many,
 // up to a group's 32, as leave the CTAs per SM that kMinRowSlots leave (a group whose rows do
 // not fit is taken in parts, each with a whole per-token part); fewer only where the shared
@@ -497,7 +512,6 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     std::vector<int4> st;
     T.s_tile_base.assign(T.C + 1, 0);
     T.s_tile_split.assign(T.C, 0);
-    auto by_size = [](const int4& a, const int4& b) { return a.z > b.z; };
     for (int ch = 0; ch < T.C; ++ch) {
         std::vector<int4> ct, cs;
         int64_t tile_ch = kSampleTile, tile_dense = kDenseTileLarge;
@@ -533,8 +547,8 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
                 (T.large && !dense ? cs : ct).push_back(v);
             }
         }
-        std::stable_sort(ct.begin(), ct.end(), by_size);
-        std::stable_sort(cs.begin(), cs.end(), by_size);
+        largest_first(ct);
+        largest_first(cs);
         st.insert(st.end(), ct.begin(), ct.end());
         T.s_tile_split[ch] = (int)st.size();
         st.insert(st.end(), cs.begin(), cs.end());
@@ -542,7 +556,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     }
     // word-topic tiles: dense segments of every chunk, and one tile per sparse word
     const int64_t wt_tile = std::min<int64_t>(
-        kWtTileMax, std::max<int64_t>(kWtTileMin, (N / (2 * 64 * (int64_t)T.num_sms) + 127) / 128 * 128));
+        kWtTileMax, std::max<int64_t>(kWtTileMin, (N / (32 * (int64_t)T.num_sms) + 127) / 128 * 128));
     std::vector<int4> wt;
     for (int64_t w = 0; w < V; ++w) {
         if (w < T.Vd) {
@@ -555,7 +569,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
             wt.push_back(make_int4((int)w, 0, (int)c->word_count[w], 0));
         }
     }
-    std::stable_sort(wt.begin(), wt.end(), [](const int4& a, const int4& b) { return a.z > b.z; });
+    largest_first(wt);
     if (T.large && T.C <= 32) {
         // small sparse words last (stable: each part keeps largest first)
         auto big = [&](const int4& x) { return (x.w & 1) || x.z > dev::kSmallSparse; };
