@@ -80,7 +80,7 @@ struct lda_trainer {
     float* recip = nullptr;  // [K] per-sweep reciprocals
     float* base = nullptr;   // K <= kLargeK: the column of a word without tokens (SampleArgs::base)
     float* smooth = nullptr; // [K] per-sweep smoothing table of the split Q bucket (K > kLargeK)
-    int* order = nullptr;    // [dev::kOrderList] per-sweep topic order of the sparse-word statistics (K > kLargeK)
+    int* order = nullptr;    // [dev::kOrderList] per-sweep topic order of the sparse-word statistics
     // K > kLargeK: the dense words' Q-round tables, [Vd][32 * qrounds] float2, built by the
     // word statistics and read by the dense-word sampler (null when dev::qtab_rounds(K) = 0)
     float2* qtab_g = nullptr;
