@@ -279,7 +279,10 @@ int lda_max_topic(lda_trainer* t);
  * 2nd topic.  Replaces UpdateDTKernel (EZLDA/DTUpdateKernel.cuh:13). */
 int lda_update_dt(lda_trainer* t, int32_t chunk);
 /* Samples every token of one chunk (dense and sparse words, early accept and
- * full evaluation in one kernel).  Replaces UpdateProbKernelD, SampleKernelD
+ * full evaluation in one kernel).  The statistics are those of the last lda_max_topic; the
+ * word columns are formed from the counts and topic totals of the last lda_update_wt, also
+ * when no lda_max_topic followed it (above 2048 topics the dense words' totals are
+ * lda_max_topic's).  Replaces UpdateProbKernelD, SampleKernelD
  * and SampleKernel (EZLDA/SamplingKernel.cuh:10-14). */
 int lda_sample_chunk(lda_trainer* t, int32_t chunk, int32_t ll_mode);
 /* Reduces the per-tile LL partials of the sampled chunks to *ll_sum (blocks).

@@ -81,6 +81,13 @@ struct lda_trainer {
     float* base = nullptr;   // K <= kLargeK: the column of a word without tokens (SampleArgs::base)
     float* smooth = nullptr; // [K] per-sweep smoothing table of the split Q bucket (K > kLargeK)
     int* order = nullptr;    // [dev::kOrderList] per-sweep topic order of the sparse-word statistics
+    // Stage calls may sample after lda_update_wt without lda_max_topic in between: the
+    // statistics are then the earlier ones, but the word columns take the current n_k
+    // (sample_totals).  Above kLargeK only the sparse words' do (the dense words' columns and
+    // Q-round tables go together), from a table of their own.
+    bool totals_new = true;        // n_k has been rewritten since the reciprocals were formed
+    float* recip_cur = nullptr;    // K > kLargeK: that table, from the first such call on
+    bool sparse_cur = false;       // the sparse words' samplers read recip_cur
     // K > kLargeK: the dense words' Q-round tables, [Vd][32 * qrounds] float2, built by the
     // word statistics and read by the dense-word sampler (null when dev::qtab_rounds(K) = 0)
     float2* qtab_g = nullptr;
@@ -238,6 +245,7 @@ struct lda_trainer {
         cudaFreeHost(h_dtok_pos);
         cudaFreeHost(h_dtok_word);
         for (void* p : allocs) cudaFree(p);
+        if (recip_cur) cudaFree(recip_cur);
         if (w_tiles_rng) cudaFree(w_tiles_rng);
         if (ll_host) cudaFreeHost(ll_host);
         for (auto& e : pending) { cudaEventDestroy(e.a); cudaEventDestroy(e.b); }
@@ -902,6 +910,7 @@ extern "C" int lda_update_wt(lda_trainer* t) {
     if (!t) return fail(LDA_ERR_ARG, "null trainer");
     CUDA_TRY(cudaSetDevice(t->device));
     t->begin_stage(0);
+    t->totals_new = true;
     dev::WtArgs a = wt_args(t);
     if (t->w_tiles_rng) {
         // a word range: its dense rows, its sparse rows and its words' share of n_k
@@ -953,20 +962,41 @@ extern "C" int lda_update_wt(lda_trainer* t) {
     return LDA_OK;
 }
 
+// The reciprocals of the current n_k into `recip` (and base, when there is one), and the
+// topic order of the words' statistics.
+static int launch_recip(lda_trainer* t, float* recip) {
+    dev::k_recip_order<<<(t->K + 31) / 32, 256, sizeof(float) * (size_t)t->K, t->stream>>>(t->n_k, t->K, t->Vbeta, t->beta,
+                                                                                        recip, t->base, t->order);
+    CUDA_TRY(cudaGetLastError());
+    return LDA_OK;
+}
+
+// Before sampling by a call that has not run lda_max_topic itself: the reciprocals of an n_k
+// that was rewritten since they were formed.
+static int sample_totals(lda_trainer* t) {
+    if (!t->totals_new) return LDA_OK;
+    if (t->large && !t->recip_cur) CUDA_TRY(cudaMalloc(&t->recip_cur, sizeof(float) * (size_t)t->K));
+    int rc = launch_recip(t, t->large ? t->recip_cur : t->recip);
+    if (rc) return rc;
+    t->totals_new = false;
+    t->sparse_cur = t->large;
+    return LDA_OK;
+}
+
 extern "C" int lda_max_topic(lda_trainer* t) {
     if (!t) return fail(LDA_ERR_ARG, "null trainer");
     CUDA_TRY(cudaSetDevice(t->device));
     t->begin_stage(1);
+    int rc;
     dev::StatsArgs a = stats_args(t);
     if (t->w_tiles_rng) {
         // a word range: its words' statistics only
         a.wlo = t->wt_lo;
         a.V = t->wt_hi;
     }
-    // the sweep's reciprocals and the topic order of the words' statistics
-    dev::k_recip_order<<<(t->K + 31) / 32, 256, sizeof(float) * (size_t)t->K, t->stream>>>(t->n_k, t->K, t->Vbeta, t->beta,
-                                                                                        t->recip, t->base, t->order);
-    CUDA_TRY(cudaGetLastError());
+    if ((rc = launch_recip(t, t->recip))) return rc;
+    t->totals_new = false;
+    t->sparse_cur = false;
     if (!t->large) {
         if (a.V > a.wlo) {
             const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(t->grid_stats, (a.V - a.wlo + t->warps - 1) / t->warps));
@@ -1114,6 +1144,7 @@ static int sample_launch(lda_trainer* t, int chunk, int slot, int ll_mode, cudaS
         as.tile_counter = t->tile_ctr + 1 + t->C + chunk;
         ad.nslots = t->slots_dense;
         as.nslots = t->slots_sparse;
+        if (t->sparse_cur) as.recip = t->recip_cur;
         const bool ll = ll_mode != 0;
         // the sparse-word sampler on the side stream of q, so that its CTAs start as the
         // dense-word kernel's CTAs run out of tiles (both read only this chunk's doc rows)
@@ -1215,8 +1246,8 @@ extern "C" int lda_sample_chunk(lda_trainer* t, int32_t chunk, int32_t ll_mode) 
         return fail(LDA_ERR_STATE, "chunk %d is not loaded (run lda_update_dt for it first)", chunk);
     CUDA_TRY(cudaSetDevice(t->device));
     t->begin_stage(3);
-    int rc = sample_launch(t, chunk, slot, ll_mode, t->stream);
-    if (rc) return rc;
+    int rc;
+    if ((rc = sample_totals(t)) || (rc = sample_launch(t, chunk, slot, ll_mode, t->stream))) return rc;
     t->end_stage();
     return LDA_OK;
 }
@@ -1291,6 +1322,8 @@ static int sweep_async(lda_trainer* t, int ll_mode, uint16_t* zout = nullptr, bo
             return fail(LDA_ERR_STATE, "a word range is set: the caller completes the word side and calls lda_trainer_sweep_chunks");
         if ((rc = lda_update_wt(t))) return rc;
         if ((rc = lda_max_topic(t))) return rc;
+    } else if ((rc = sample_totals(t))) {
+        return rc;
     }
     // Resident sweeps without host copies take the chunk range in two groups up to kLargeK
     // topics: a group's chunks share one rebuild launch and one sampler launch, so the
@@ -1755,6 +1788,7 @@ int lda::trainer_note_sweeps(lda_trainer* t, int n, int ll_mode, double ll_sum) 
     if (!t) return fail(LDA_ERR_ARG, "null trainer");
     t->iter += (uint32_t)n;
     if (n > 0) {
+        t->totals_new = false;  // a sweep forms the reciprocals of its n_k
         for (int ch = 0; ch < t->C; ++ch) t->chunk_sampled_ll[ch] = ll_mode != 0;
         if (ll_mode) {
             t->last_ll = ll_sum;
