@@ -510,17 +510,13 @@ struct SampleArgs {
     // tok_doc / meta hold tokens [tok_base, ...) and dt_ent the doc-row entries
     // [dt_base, ...) (non-zero when the chunk is streamed into a slot buffer)
     uint32_t tok_base, dt_base;
-    // r_k = 1 / ((float)n_k + V*beta) for k < K, formed once per sweep with the word
-    // statistics, or null (then a column's r_k are formed from n_k)
+    // r_k = 1 / ((float)n_k + V*beta) for k < K, formed once per sweep or call (per column
+    // instead, an allocation-free call at K=12,000 took 1,334 us against 627)
     const float* recip = nullptr;
     // K <= kLargeK: beta * r_k in the skewed column layout, the column of a word without
     // tokens (col_words(K) floats, formed with recip)
     const float* base = nullptr;
     int nslots = 1;  // row slots per warp (sample_groups)
-    template <bool TABLE>
-    __device__ __forceinline__ float rk(int k) const {
-        return TABLE ? __ldg(recip + k) : __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta));
-    }
     // K > kLargeK: the smoothing table of the split Q bucket (k_smooth_table)
     const float* smooth = nullptr;
     // K > kLargeK: the dense words' Q-round tables (k_word_stats_dense_cta), or null
@@ -534,22 +530,18 @@ struct SplitQ {
     uint32_t nnz;
     float Qw;
     const float* T;       // the smoothing table (K entries, non-decreasing)
-    const float* r;       // r_k, at col_skew(k) when skew; null: formed from n_k
+    const float* r;       // r_k, at col_skew(k) when skew
     bool skew;
     // the Qw rounds' table, lane r holding round r's (carry before it, carry + its largest
     // KS prefix); rounds = 0 when not built (more than 32 rounds, or not wanted)
     int rounds = 0;
     float qcarry = 0.0f, qthr = 0.0f;
-    const int* n_k = nullptr;
-    float Vbeta = 0.0f;
     // in shared memory, for thread_split_draw: the prefixes of a one-round word's terms (else
     // null) with the entries whose term is positive, and the last entry of each of T's rounds
     const float* wp = nullptr;
     unsigned wok = 0u;
     const float* tend = nullptr;
-    __device__ __forceinline__ float rk(int k) const {
-        return r ? r[skew ? col_skew(k) : k] : __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta));
-    }
+    __device__ __forceinline__ float rk(int k) const { return r[skew ? col_skew(k) : k]; }
     // round slot i of the Qw search: alpha * (n_wk * r_k), the max topic's term 0
     __device__ __forceinline__ void slot(uint32_t i, int maxK, float alpha, int& key, float& term, bool& ok) const {
         const uint32_t en = __ldg(ent + i);
@@ -1199,7 +1191,7 @@ __device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const
         const int* row = a.dwt + (size_t)w * a.K;
         if (!SKEWKEYS || held != w)
             for (int k = lane; k < a.K; k += 32)
-                col[col_skew(k)] = fmul(fadd(__int2float_rn(__ldg(row + k)), a.beta), a.rk<SKEWKEYS>(k));
+                col[col_skew(k)] = fmul(fadd(__int2float_rn(__ldg(row + k)), a.beta), __ldg(a.recip + k));
         held = w;
     } else {
         if (SKEWKEYS) {
@@ -1208,13 +1200,13 @@ __device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const
                 for (int i = lane; i < col_words(a.K) / 4; i += 32) reinterpret_cast<float4*>(col)[i] = __ldg(src + i);
             }
         } else {
-            for (int k = lane; k < a.K; k += 32) col[col_skew(k)] = fmul(a.beta, a.rk<SKEWKEYS>(k));
+            for (int k = lane; k < a.K; k += 32) col[col_skew(k)] = fmul(a.beta, __ldg(a.recip + k));
         }
         __syncwarp();
         for (uint32_t e = lane; e < nnz; e += 32) {
             const uint32_t en = __ldg(ent + e);
             const int k = (int)(en >> 16);
-            col[col_skew(k)] = fmul(fadd(u2f(en & 0xffffu), a.beta), a.rk<SKEWKEYS>(k));
+            col[col_skew(k)] = fmul(fadd(u2f(en & 0xffffu), a.beta), __ldg(a.recip + k));
         }
         clean = SKEWKEYS && nnz <= (uint32_t)a.K >> 3;
         held = clean ? kHoldsBase : kHoldsNone;
@@ -1234,7 +1226,7 @@ __device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const
     if (split) {
         // a sparse word above kLargeK topics: the split Q bucket
         if constexpr (QB > 1 && !SKEWKEYS) {
-            const SplitQ sq{ent, nnz, __shfl_sync(FULL, QL, 0), a.smooth, a.recip, false, 0, 0.0f, 0.0f, a.n_k, a.Vbeta};
+            const SplitQ sq{ent, nnz, __shfl_sync(FULL, QL, 0), a.smooth, a.recip, false};
             ll = sample_groups<LL, QB, true>(a, start, cnt, 0u, 32u, iter, maxK, ph, QL, QP, Q, View{col}, ctr, lane,
                                              slots, nullptr, 0, &sq);
         }

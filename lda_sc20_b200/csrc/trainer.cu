@@ -1898,11 +1898,13 @@ extern "C" int lda_get_token_meta(lda_trainer* t, uint32_t* meta) {
 namespace {
 constexpr int kNoAllocMaxTiles = 65536;
 constexpr size_t kNoAllocHeader = 256;
-// above 2048 topics the split Q bucket's smoothing table (K floats) follows the LL partials;
-// K is bounded below this by the sampler's shared memory anyway
+// the LL partials are followed by the split Q bucket's smoothing table (above 2048 topics) and
+// the reciprocals of the call's n_k, K floats each; K is bounded below this by the rule that
+// picks the sampler's warps anyway
 constexpr int kNoAllocMaxK = 29696;
 constexpr size_t kNoAllocSmooth = kNoAllocHeader + sizeof(double) * (size_t)kNoAllocMaxTiles;
-constexpr size_t kNoAllocBytes = kNoAllocSmooth + sizeof(float) * (size_t)kNoAllocMaxK;
+constexpr size_t kNoAllocRecip = kNoAllocSmooth + sizeof(float) * (size_t)kNoAllocMaxK;  // the reciprocals
+constexpr size_t kNoAllocBytes = kNoAllocRecip + sizeof(float) * (size_t)kNoAllocMaxK;
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mu;
 unsigned char* g_noalloc_addr[kMaxDevices] = {};
@@ -1927,17 +1929,22 @@ struct IoCheck {
     int64_t N, n_dt, n_sp;
     int* status;
     unsigned* tile_counter;
+    const int* n_k;
+    float Vbeta;
+    float* recip;
 };
 }  // namespace
 
-// Range checks before an allocation-free sampling launch: warp per tile (its word, token
-// range, the word's max topic and sparse row, its tokens' doc ids), thread per doc (its
-// row's extent and topics).  A failure ORs LDA_IO_* bits into *status and moves the tile
+// What precedes an allocation-free sampling launch.  The reciprocals of the caller's n_k, and
+// the range checks: warp per tile (its word, token range, the word's max topic and sparse row,
+// its tokens' doc ids), thread per doc (its row's extent and topics).  A failure ORs LDA_IO_* bits into *status and moves the tile
 // counter past any tile index, so the sampling kernel that follows on the stream takes no
 // tile (its warps' first claim returns >= ntiles; the counter stays below 2^31).
 __global__ void __launch_bounds__(256) k_check_sample_io(IoCheck c) {
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nw = (int)((gridDim.x * blockDim.x) >> 5);
+    for (int k = (int)(blockIdx.x * blockDim.x + threadIdx.x); k < c.K; k += (int)(gridDim.x * blockDim.x))
+        c.recip[k] = __fdiv_rn(1.0f, dev::fadd(__int2float_rn(c.n_k[k]), c.Vbeta));
     int bad = 0;
     for (int t = gw; t < c.ntiles; t += nw) {
         const int4 tl = c.tiles[t];
@@ -2073,6 +2080,8 @@ extern "C" int lda_sample_chunk_noalloc(const lda_sample_io* io, int32_t device,
     chk.swt_ent = io->sparse_ent; chk.tok_doc = io->tok_doc; chk.dt_off = io->dt_off; chk.dt_nnz = io->dt_nnz;
     chk.dt_ent = io->dt_ent; chk.N = io->num_tokens; chk.n_dt = io->num_dt_entries;
     chk.n_sp = io->num_sparse_entries; chk.status = io->status; chk.tile_counter = a.tile_counter;
+    chk.n_k = io->n_k; chk.Vbeta = a.Vbeta; chk.recip = reinterpret_cast<float*>(scratch + kNoAllocRecip);
+    a.recip = chk.recip;
     k_check_sample_io<<<4 * num_sms, 256, 0, st>>>(chk);
     CUDA_TRY(cudaGetLastError());
     kfn<<<grid, 32 * warps, smem, st>>>(a);
