@@ -1,5 +1,6 @@
-"""The allocation-free entry point's tables are of each call's own topic totals: calls of
-different K and totals in turn, through the one scratch array they share."""
+"""The allocation-free entry point's tables are of each call's own topic totals, and its launch
+shape of the call's own K: calls of different K and totals in turn, through the one scratch
+array and the 16 launch shapes they share."""
 import numpy as np
 import pytest
 
@@ -9,7 +10,7 @@ from test_zz_no_alloc import LL_RTOL, _call, _device_io, _state
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("Ks", [(100, 2048, 100), (2049, 5001, 2049, 64)])
+@pytest.mark.parametrize("Ks", [(100, 2048, 100), (2049, 5001, 2049, 64), tuple(range(250, 268))])
 def test_calls_of_different_topic_counts_in_turn(Ks):
     torch = pytest.importorskip("torch")
     states = []
