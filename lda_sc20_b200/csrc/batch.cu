@@ -81,36 +81,23 @@ __global__ void __launch_bounds__(256) kb_wt(BatchArgs b) {
     }
 }
 
-// Every model's reciprocals, column of a word without tokens and topic order, as
-// k_recip_order forms them: block per model, Kmax floats of shared memory.  (The statistics
-// and the sampler each formed the reciprocals per warp whenever the warp's next item was
-// another model's.)  Also counts the sweep.
+// Every model's reciprocals, column of a word without tokens and topic order: CTA per model
+// (blockIdx.x) and 32 of its topics, Kmax floats of shared memory.  (The statistics and the
+// sampler each formed the reciprocals per warp whenever the warp's next item was another
+// model's.)  Also counts the sweep.
 struct RecipOut {
     float* recip;
     float* base;
     int* order;
 };
-__global__ void __launch_bounds__(256) kb_recip(const StatsArgs* st, const RecipOut* out, uint32_t* sweeps_done) {
+__global__ void __launch_bounds__(kRecipThreads) kb_recip(const StatsArgs* st, const RecipOut* out,
+                                                          uint32_t* sweeps_done) {
     extern __shared__ float smf[];
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *sweeps_done += 1u;
     const StatsArgs& a = st[blockIdx.x];
     const RecipOut o = out[blockIdx.x];
-    const int K = a.K;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *sweeps_done += 1u;
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const float r = __fdiv_rn(1.0f, fadd(__int2float_rn(a.n_k[k]), a.Vbeta));
-        const float v = fmul(a.beta, r);
-        smf[k] = v;
-        o.recip[k] = r;
-        o.base[col_skew(k)] = v;
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const float v = smf[k];
-        int n = 0;
-#pragma unroll 4
-        for (int j = 0; j < K; ++j) n += ranks_above(smf[j], j, v, k) ? 1 : 0;
-        if (n < kOrderList) o.order[n] = k;
-    }
+    const int k0 = (int)blockIdx.y * 32;
+    if (k0 < a.K) recip_order(a.n_k, a.K, a.Vbeta, a.beta, o.recip, o.base, o.order, k0, smf);
 }
 
 __global__ void __launch_bounds__(256) kb_stats(BatchArgs b) {
@@ -464,7 +451,7 @@ static int enqueue_sweeps(lda_batch* b, int sweeps, int ll) {
         const bool last_ll = ll && s == sweeps - 1;
         dev::kb_zero<<<std::min<int>((int)b->zero.n, 4 * b->num_sms), 256, 0, b->st>>>(b->zero.p, (int)b->zero.n, b->counters);
         dev::kb_wt<<<grid_for(b->grid_wt, a.n_wt, W), threads, b->smem_hist, b->st>>>(a);
-        dev::kb_recip<<<M, 256, sizeof(float) * (size_t)b->Kmax, b->st>>>(b->stt.p, b->rout.p, b->sweeps_done);
+        dev::kb_recip<<<dim3((unsigned)M, (unsigned)(b->Kmax + 31) / 32), dev::kRecipThreads, sizeof(float) * (size_t)b->Kmax, b->st>>>(b->stt.p, b->rout.p, b->sweeps_done);
         dev::kb_stats<<<grid_for(b->grid_stats, a.n_st, W), threads, b->smem_stats, b->st>>>(a);
         dev::kb_dt<<<grid_for(b->grid_dt, a.n_dt, W), threads, b->smem_dt, b->st>>>(a);
         const int gs = last_ll ? grid_for(b->grid_sample_ll, a.n_sm, W) : grid_for(b->grid_sample, a.n_sm, W);

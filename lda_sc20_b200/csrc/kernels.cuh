@@ -512,51 +512,12 @@ __global__ void __launch_bounds__(256, LDA_DT_SMALL_MIN_BLOCKS) k_dt_build_small
     }
 }
 
-// The sweep's reciprocals r_k = 1 / ((float)n_k + V*beta), up to kLargeK topics beta * r_k
-// in the sampler's column layout (base, else null), and the order of the topics outside a
-// word: the first kOrderList by (beta * r_k desc, k asc).  A CTA takes 32 topics.  A topic's
-// place in the order is the number of topics that rank above it, counted by the CTA's 8
-// warps against an eighth of all K each, so K^2 comparisons spread over ceil(K/32) CTAs.
-// (64 arg-max rounds of one CTA over the table took 239 us at K=10,000.)  K floats of
-// shared memory.
-__global__ void __launch_bounds__(256) k_recip_order(const int* __restrict__ n_k, int K, float Vbeta, float beta,
-                                                     float* recip, float* base, int* order) {
+// The sweep's reciprocals, base column and topic order (recip_order): CTA per 32 topics, K
+// floats of shared memory.
+__global__ void __launch_bounds__(kRecipThreads) k_recip_order(const int* __restrict__ n_k, int K, float Vbeta,
+                                                               float beta, float* recip, float* base, int* order) {
     extern __shared__ float smf[];
-    __shared__ int above[32];
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int k = threadIdx.x; k < K; k += blockDim.x)
-        smf[k] = fmul(beta, __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta)));
-    if (threadIdx.x < 32) above[threadIdx.x] = 0;
-    __syncthreads();
-    const int k = blockIdx.x * 32 + lane;
-    const float v = k < K ? smf[k] : 0.0f;
-    if (wid == 0 && k < K) {
-        recip[k] = __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta));
-        if (base) base[col_skew(k)] = v;
-    }
-    // the CTA's own topics lie in [k0, k0 + 32): before them a topic ranks above with an equal
-    // value, after them only with a larger one
-    const int part = (((K + 7) >> 3) + 3) & ~3, j0 = min(K, wid * part), j1 = min(K, j0 + part);
-    const int k0 = blockIdx.x * 32, k1 = min(K, k0 + 32);
-    int n = 0;
-    for (int j = max(j0, k0); j < min(j1, k1); ++j) n += ranks_above(smf[j], j, v, k) ? 1 : 0;
-    const int a1 = min(j1, k0), b0 = max(j0, k1);
-    for (int j = j0; j + 4 <= a1; j += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(smf + j);
-        n += (x.x >= v) + (x.y >= v) + (x.z >= v) + (x.w >= v);
-    }
-    if (a1 > j0)
-        for (int j = j0 + ((a1 - j0) & ~3); j < a1; ++j) n += smf[j] >= v;
-    int j = b0;
-    for (; j < j1 && (j & 3); ++j) n += smf[j] > v;
-    for (; j + 4 <= j1; j += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(smf + j);
-        n += (x.x > v) + (x.y > v) + (x.z > v) + (x.w > v);
-    }
-    for (; j < j1; ++j) n += smf[j] > v;
-    atomicAdd(&above[lane], n);
-    __syncthreads();
-    if (wid == 0 && k < K && above[lane] < kOrderList) order[above[lane]] = k;
+    recip_order(n_k, K, Vbeta, beta, recip, base, order, (int)blockIdx.x * 32, smf);
 }
 
 // Word statistics: warp per word.

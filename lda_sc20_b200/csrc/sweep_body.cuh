@@ -148,6 +148,53 @@ constexpr int kOrderList = 64;
 // (v, k) ranks above (a, i): larger value, ties to the lower topic.
 __device__ __forceinline__ bool ranks_above(float v, int k, float a, int i) { return v > a || (v == a && k < i); }
 
+// The reciprocals r_k = 1 / ((float)n_k + V*beta) of a CTA's 32 topics from k0 on, up to
+// kLargeK topics beta * r_k in the sampler's column layout (base, else null), and the order of
+// the topics outside a word: the first kOrderList by (beta * r_k desc, k asc).  A topic's
+// place in the order is the number of topics that rank above it, counted by the CTA's 8
+// warps against an eighth of all K each, so K^2 comparisons spread over ceil(K/32) CTAs.
+// (64 arg-max rounds of one CTA over the table took 239 us at K=10,000; one CTA per model of a
+// batch for all of its K^2 comparisons 200 us at K=2048, now 8.5.)  smf: K floats.
+constexpr int kRecipThreads = 256;
+__device__ __forceinline__ void recip_order(const int* __restrict__ n_k, int K, float Vbeta, float beta, float* recip,
+                                            float* base, int* order, int k0, float* smf) {
+    __shared__ int above[32];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int k = threadIdx.x; k < K; k += blockDim.x)
+        smf[k] = fmul(beta, __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta)));
+    if (threadIdx.x < 32) above[threadIdx.x] = 0;
+    __syncthreads();
+    const int k = k0 + lane;
+    const float v = k < K ? smf[k] : 0.0f;
+    if (wid == 0 && k < K) {
+        recip[k] = __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(n_k + k)), Vbeta));
+        if (base) base[col_skew(k)] = v;
+    }
+    // the CTA's own topics lie in [k0, k0 + 32): before them a topic ranks above with an equal
+    // value, after them only with a larger one
+    const int part = (((K + 7) >> 3) + 3) & ~3, j0 = min(K, wid * part), j1 = min(K, j0 + part);
+    const int k1 = min(K, k0 + 32);
+    int n = 0;
+    for (int j = max(j0, k0); j < min(j1, k1); ++j) n += ranks_above(smf[j], j, v, k) ? 1 : 0;
+    const int a1 = min(j1, k0), b0 = max(j0, k1);
+    for (int j = j0; j + 4 <= a1; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(smf + j);
+        n += (x.x >= v) + (x.y >= v) + (x.z >= v) + (x.w >= v);
+    }
+    if (a1 > j0)
+        for (int j = j0 + ((a1 - j0) & ~3); j < a1; ++j) n += smf[j] >= v;
+    int j = b0;
+    for (; j < j1 && (j & 3); ++j) n += smf[j] > v;
+    for (; j + 4 <= j1; j += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(smf + j);
+        n += (x.x > v) + (x.y > v) + (x.z > v) + (x.w > v);
+    }
+    for (; j < j1; ++j) n += smf[j] > v;
+    atomicAdd(&above[lane], n);
+    __syncthreads();
+    if (wid == 0 && k < K && above[lane] < kOrderList) order[above[lane]] = k;
+}
+
 __device__ __forceinline__ void top3_insert(float v, int k, float& a1, int& i1, float& a2, int& i2, float& a3, int& i3) {
     if (ranks_above(v, k, a1, i1)) {
         a3 = a2; i3 = i2;

@@ -965,7 +965,7 @@ extern "C" int lda_update_wt(lda_trainer* t) {
 // The reciprocals of the current n_k into `recip` (and base, when there is one), and the
 // topic order of the words' statistics.
 static int launch_recip(lda_trainer* t, float* recip) {
-    dev::k_recip_order<<<(t->K + 31) / 32, 256, sizeof(float) * (size_t)t->K, t->stream>>>(t->n_k, t->K, t->Vbeta, t->beta,
+    dev::k_recip_order<<<(t->K + 31) / 32, dev::kRecipThreads, sizeof(float) * (size_t)t->K, t->stream>>>(t->n_k, t->K, t->Vbeta, t->beta,
                                                                                         recip, t->base, t->order);
     CUDA_TRY(cudaGetLastError());
     return LDA_OK;
