@@ -25,6 +25,15 @@ __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float ffma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float u2f(uint32_t x) { return __uint2float_rn(x); }
 
+// Two binary32 additions in one instruction, each rounded to nearest.
+__device__ __forceinline__ void fadd2(float& a0, float& a1, float b0, float b1) {
+    uint64_t a, b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(a0), "f"(a1));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(b0), "f"(b1));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
+}
+
 // Inclusive Kogge-Stone scan over the warp: round `off` adds lane l-off into lane l.
 __device__ __forceinline__ float warp_ks_scan(float v, int lane) {
 #pragma unroll
