@@ -44,8 +44,11 @@ struct BatchArgs {
     unsigned* counters;    // [4] work counters of the stages, zeroed at the start of a sweep
     const uint32_t* sweeps_done;  // sweeps this batch has begun: with a model's base iteration, its iteration
     int Kmax;
-    int nslots;            // row slots per warp of the sampler
 };
+
+// Row slots per warp of the batched sampler: a whole group's.  (16, which leave room for more
+// CTAs at large K, measured the same above 512 topics and 1% slower in batches up to K=256.)
+constexpr int kBatchSlots = 32;
 
 __device__ __forceinline__ int grab(unsigned* counter, int lane) {
     int i = 0;
@@ -144,9 +147,9 @@ template <bool LL, int QB>
 __global__ void __launch_bounds__(256, 3) kb_sample(BatchArgs b) {
     extern __shared__ float smf[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* col = smf + (size_t)sample_warp_words(b.Kmax, b.nslots) * wid;
+    float* col = smf + (size_t)sample_warp_words(b.Kmax, kBatchSlots) * wid;
     float* slots = col + col_words(b.Kmax);
-    uint32_t* ctr = reinterpret_cast<uint32_t*>(slots + ((row_state_words(b.nslots) + 3) & ~3));
+    uint32_t* ctr = reinterpret_cast<uint32_t*>(slots + ((row_state_words(kBatchSlots) + 3) & ~3));
     if (lane < C_NUM) ctr[lane] = 0u;
     __syncwarp();
     const uint32_t done = *b.sweeps_done - 1u;  // sweeps before this one
@@ -264,7 +267,6 @@ struct lda_batch {
     uint32_t host_sweeps = 0;
     // launch shapes
     size_t smem_hist = 0, smem_stats = 0, smem_sample = 0, smem_dt = 0;
-    int nslots = 1;
     int grid_wt = 0, grid_stats = 0, grid_dt = 0, grid_sample = 0, grid_sample_ll = 0;
     // cached graph of (sweeps, ll)
     cudaGraphExec_t graph = nullptr;
@@ -301,14 +303,10 @@ static int occupancy(const void* fn, int threads, size_t smem, int num_sms, int*
     return LDA_OK;
 }
 
-#ifndef LDA_RUN_TOKENS
-#define LDA_RUN_TOKENS 512
-#endif
-#ifndef LDA_RUN_TILES
-#define LDA_RUN_TILES 16
-#endif
-constexpr int kRunTokens = LDA_RUN_TOKENS;  // most tokens of a run of small tiles
-constexpr int kRunTiles = LDA_RUN_TILES;    // most tiles of a run
+// Most tokens and tiles of a run of small tiles.  Sweeps of 48 to 512 models up to K=256 are
+// within 1.5% of each other with 256 to 1,024 tokens and with 8 to 32 tiles.
+constexpr int kRunTokens = 512;
+constexpr int kRunTiles = 16;
 
 // Builds the tables, work lists and launch shapes for the current tuning.
 static int batch_build(lda_batch* b) {
@@ -319,7 +317,6 @@ static int batch_build(lda_batch* b) {
     std::vector<dev::DtArgs> dt(M);
     std::vector<dev::SampleArgs> sm(M);
     std::vector<dev::RecipOut> rout(M);
-    const int nslots = b->Kmax <= 512 ? 32 : 16;
     std::vector<dev::ZeroSeg> zero;
     std::vector<int*> errs;
     std::vector<int4> sub;
@@ -346,7 +343,7 @@ static int batch_build(lda_batch* b) {
         sm[m].tiles = b->sub_tiles.p + sub_base[m];
         sm[m].ntiles = (int)(sub_base[m + 1] - sub_base[m]);
         sm[m].tile_ll = b->sub_ll.p + sub_base[m];
-        sm[m].nslots = nslots;
+        sm[m].nslots = dev::kBatchSlots;
         zero.push_back({v.n_k, (long long)v.K});
         if (v.dwt_count > 0) zero.push_back({v.dwt, (long long)v.dwt_count});
         errs.push_back(v.wt.err);
@@ -360,8 +357,11 @@ static int batch_build(lda_batch* b) {
     std::vector<uint4> wt_work, sm_work;
     std::vector<uint4> st_work, dt_work;
     std::vector<int> wt_cnt, sm_cnt;
-    // Runs are as long as leave about eight items per resident warp, up to those limits: a
-    // batch of 1.4M tokens in all has too few tiles to join (1.25 against 1.63 ms).
+    // Runs are as long as leave about eight items per resident warp (24 an SM: the sampler's
+    // three CTAs of 8), up to those limits: a batch of 1.4M tokens in all has too few tiles to
+    // join (1.25 against 1.63 ms).  Sixteen items per warp are up to 13% slower (24 models up
+    // to K=2048), four 6% faster there, 1% slower with 24 up to K=1024 and the same with 48
+    // up to K=256.
     int64_t all_tokens = 0;
     for (const TrainerView& v : b->views) all_tokens += v.N;
     const int64_t share = 8 * 24 * (int64_t)b->num_sms;  // items wanted
@@ -407,8 +407,7 @@ static int batch_build(lda_batch* b) {
     const int threads = 32 * tu.warps;
     b->smem_hist = (size_t)tu.warps * (b->Kmax + (b->Kmax + 31) / 32) * 4;
     b->smem_stats = (size_t)tu.warps * dev::stats_warp_words(b->Kmax) * 4;
-    b->smem_sample = (size_t)tu.warps * dev::sample_warp_words(b->Kmax, nslots) * 4;
-    b->nslots = nslots;
+    b->smem_sample = (size_t)tu.warps * dev::sample_warp_words(b->Kmax, dev::kBatchSlots) * 4;
     b->smem_dt = (size_t)tu.warps * (b->Kmax + (b->Kmax + 31) / 32) * 4;
     if ((rc = occupancy((const void*)dev::kb_wt, threads, b->smem_hist, b->num_sms, &b->grid_wt)) ||
         (rc = occupancy((const void*)dev::kb_stats, threads, b->smem_stats, b->num_sms, &b->grid_stats)) ||
@@ -434,7 +433,6 @@ static dev::BatchArgs batch_args(const lda_batch* b) {
     a.counters = b->counters;
     a.sweeps_done = b->sweeps_done;
     a.Kmax = b->Kmax;
-    a.nslots = b->nslots;
     return a;
 }
 
