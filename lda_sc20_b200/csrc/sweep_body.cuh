@@ -268,6 +268,11 @@ struct ColumnPhi {
 template <class Phi>
 __device__ __forceinline__ int word_stats_from(const StatsArgs& a, int w, const Phi& phi, int lane);
 
+// Whether a sparse word of nnz topics puts the base values back into a column kept for the next
+// sparse word: up to an eighth of the topics (a sixteenth and a quarter measure the same, in the
+// statistics and in the samplers, K=64 to 1500).
+__device__ __forceinline__ bool put_back(uint32_t nnz, int K) { return nnz <= (uint32_t)K >> 3; }
+
 // Words of shared memory a warp of the K <= kLargeK statistics uses: a word column (plain
 // layout) and a topic bitmap, a multiple of 4.
 __host__ __device__ __forceinline__ int stats_warp_words(int K) { return ((K + 3) & ~3) + ((((K + 31) >> 5) + 3) & ~3); }
@@ -355,7 +360,7 @@ __device__ __forceinline__ void word_stats_word(const StatsArgs& a, int w, float
         none.ql = ql;
     }
     __syncwarp();
-    clean = nnz <= (uint32_t)K >> 2;
+    clean = put_back(nnz, K);
     if (clean) {
         for (uint32_t e = lane; e < nnz; e += 32) {
             const int k = (int)(__ldg(ent + e) >> 16);
@@ -1072,7 +1077,7 @@ __device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const
             const int k = (int)(en >> 16);
             col[col_skew(k)] = fmul(fadd(u2f(en & 0xffffu), a.beta), __ldg(a.recip + k));
         }
-        clean = SKEWKEYS && nnz <= (uint32_t)a.K >> 3;
+        clean = SKEWKEYS && put_back(nnz, a.K);
         held = clean ? kHoldsBase : kHoldsNone;
     }
     __syncwarp();
