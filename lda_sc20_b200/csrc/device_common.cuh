@@ -279,10 +279,11 @@ __device__ __forceinline__ int warp_level2_rounds(uint32_t n, float t2, int fall
     return last >= 0 ? last : fallback;
 }
 
-// First k in [lo, hi) with x < T[k] for a non-decreasing table T in global memory, else
+// First k in [lo, hi) with x < T[k] for an ascending table T in global memory, else
 // -1; uniform across the warp.  A 32-way search: each round the lanes probe the ends of 32
 // equal segments of the range, and a ballot keeps the first segment whose end exceeds x
-// (the answer lies in it, since every entry before its start is <= x).
+// (the answer lies in it, since every entry before its start is <= x).  Where rounding leaves
+// T's neighbours out of order, the answer is the one this search finds, here and in the oracle.
 __device__ __forceinline__ int warp_first_above(const float* __restrict__ T, int lo, int hi, float x, int lane) {
     if (lo >= hi || !(x < __ldg(T + hi - 1))) return -1;
     while (hi - lo > 32) {

@@ -641,11 +641,11 @@ __global__ void __launch_bounds__(256) k_dt_build(DtArgs a) {
 
 // Sampler: warp per tile, tiles taken from an atomic counter (the next one is claimed when a
 // tile starts, so that the claim's round trip overlaps the tile's work).  SKEWKEYS: the doc
-// rows' keys are word-column slot indices and a.recip / a.base are there (the trainer's rows
+// rows' keys are byte offsets of word-column slots and a.base is there (the trainer's rows
 // and tables up to kLargeK topics).
 template <bool LL, int QB = 1, bool SKEWKEYS = true>
 __global__ void __launch_bounds__(32 * kSampleWarps, QB > 1 ? LDA_SAMPLE_QB_MIN_BLOCKS
-                                                       : (!LL ? LDA_SAMPLE_MIN_BLOCKS : QB == 0 ? LDA_SAMPLE_LL0_MIN_BLOCKS : LDA_SAMPLE_LL_MIN_BLOCKS))
+                                                       : (!LL ? LDA_SAMPLE_MIN_BLOCKS : QB == 0 ? kSampleLL0MinBlocks : LDA_SAMPLE_LL_MIN_BLOCKS))
 k_sample_t(SampleArgs a) {
     extern __shared__ float smf[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -780,8 +780,6 @@ __host__ __device__ __forceinline__ size_t sparse_large_smem(int K, int warps, i
     return (size_t)(col_words(K) + ((smooth_rounds(K) + 1) & ~1) + warps * sparse_large_warp_words(K, nslots)) * 4;
 }
 
-// Shared memory of the dense-word kernel: the shared column, the warps' counter rows and
-// their LL partials (the reciprocals are formed while the column is built).
 // Shared memory of the dense-word sampler: the word column, the warps' counter rows, their
 // LL partials and (when qtab_rounds(K) > 0) the Q-round table of 32 x R float2.
 __host__ __device__ __forceinline__ size_t dense_large_smem(int K, int warps, int nslots) {
@@ -796,19 +794,13 @@ __host__ __device__ __forceinline__ size_t dense_large_smem(int K, int warps, in
 // three of 8).  Sparse: the reciprocals (41 KB at K=10,000) are the CTA's, so two CTAs of 12
 // warps hold as many warps as three of 8, and 80 registers a thread avoid 130 bytes of
 // spills (5.40 -> 4.79 ms with the dense kernel as it is; 16 warps at 64 registers 5.6).
-#ifndef LDA_DENSE_WARPS
-#define LDA_DENSE_WARPS 8
-#endif
 #ifndef LDA_DENSE_LARGE_MIN_BLOCKS
 #define LDA_DENSE_LARGE_MIN_BLOCKS 4
-#endif
-#ifndef LDA_SPARSE_WARPS
-#define LDA_SPARSE_WARPS 12
 #endif
 #ifndef LDA_SPARSE_LARGE_MIN_BLOCKS
 #define LDA_SPARSE_LARGE_MIN_BLOCKS 2
 #endif
-constexpr int kDenseWarps = LDA_DENSE_WARPS, kSparseWarps = LDA_SPARSE_WARPS;
+constexpr int kDenseWarps = 8, kSparseWarps = 12;
 
 // The sparse-word sampler keeps each word's Qw rounds' table in registers (lane r: round
 // r), so a Q draw evaluates the one round that holds its target instead of walking them.
@@ -866,7 +858,7 @@ __global__ void __launch_bounds__(32 * kSparseWarps, LDA_SPARSE_LARGE_MIN_BLOCKS
         const float Q = __shfl_sync(FULL, QP, 31);
         __syncwarp();
         const ColBits view{bits, pre, ent, base, a.recip, a.beta, maxK, extra, nnz_w > (uint32_t)a.K >> 5};
-        SplitQ sq{ent, nnz_w, __shfl_sync(FULL, QL, 0), a.smooth, a.recip, false};
+        SplitQ sq{ent, nnz_w, __shfl_sync(FULL, QL, 0), a.smooth, a.recip};
         if (nnz_w <= 32u) {
             // the one round's prefixes, for thread_split_draw
             int key;
@@ -932,7 +924,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, LDA_DENSE_LARGE_MIN_BLOCKS) 
         // (that corpus: samplers 116.1 -> 115.6 ms per sweep)
         const uint64_t spol = l2_stream_policy();
         for (int k = threadIdx.x; k < a.K; k += blockDim.x) {
-            const float rk = a.recip ? __ldg(a.recip + k) : __fdiv_rn(1.0f, fadd(__int2float_rn(__ldg(a.n_k + k)), a.Vbeta));
+            const float rk = __ldg(a.recip + k);
             const int c = ldg_hint(wrow + k, spol);
             col[col_skew(k)] = fmul(fadd(__int2float_rn(c), a.beta), rk);
         }
@@ -982,7 +974,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, LDA_DENSE_LARGE_MIN_BLOCKS) 
 // statistics need no column: the top three come from its own topics and the first three
 // other topics of the CTA's list of topics in decreasing beta * r_k (ties to the lower k),
 // and its split Q from its own entries and the smoothing table (Qw in st_ql slot 0, Qs in
-// slot 1).  Dense words keep k_word_stats.
+// slot 1).  Dense words take k_word_stats_dense_cta.
 // Shared memory of the sparse-word statistics: the order list, then per warp the bitmap.
 // The reciprocals are read from the global table (k_recip_order), so that the CTA does not
 // hold K of them and eight CTAs fit per SM.
@@ -1050,7 +1042,7 @@ __global__ void __launch_bounds__(256) k_word_stats_sparse_large(StatsArgs a) {
 
 // The smoothing table of the split Q bucket (K > kLargeK): T[k] = carry + Kogge-Stone scan
 // of sm_k = alpha * (beta * r_k) over rounds of 32 topics, the carry being the previous
-// round's last prefix, so T is non-decreasing and T[K-1] is the total.  r_k is formed from
+// round's last prefix, so T ascends but for rounding and T[K-1] is the total.  r_k is formed from
 // n_k as k_recip_order forms it.  One CTA: its warps scan the rounds in parallel (the scan of
 // a round does not depend on the carry), one thread chains the carries, then every T[k] is
 // one addition.  T holds each round's scan until the carries are known.

@@ -138,7 +138,7 @@ struct StatsArgs {
     const float* recip = nullptr;   // r_k = 1 / ((float)n_k + V*beta) (k_recip_order)
     const int* order = nullptr;     // the sparse words' topic order (k_recip_order)
     // K > kLargeK: the dense words' Q-round tables (32 lane slots x qrounds float2 per word,
-    // the table k_sample_dense_large would build per tile), or null
+    // read by k_sample_dense_large), or null
     float2* qtab = nullptr;
     int qrounds = 0;
 };
@@ -258,15 +258,43 @@ __device__ __forceinline__ void top3_outside(const StatsArgs& a, const int* orde
     }
 }
 
-struct ColumnPhi {
-    const float* col;
-    __device__ __forceinline__ float operator()(int k) const { return col[k]; }
-};
-
-// The statistics of word w from phi(k), k < K: top three, the lane partials of Q (the
+// The statistics of word w from its column of phi: top three, the lane partials of Q (the
 // max topic excluded) and Q.
-template <class Phi>
-__device__ __forceinline__ int word_stats_from(const StatsArgs& a, int w, const Phi& phi, int lane);
+__device__ __forceinline__ void word_stats_column(const StatsArgs& a, int w, const float* col, int lane) {
+    // the lane's top three by (phi desc, k asc) in one pass (k ascends, so a strictly larger
+    // value is needed to displace), then three warp-wide pops of the lanes' heads
+    float a1 = -1.0f, a2 = -1.0f, a3 = -1.0f;
+    int i1 = 0x7fffffff, i2 = 0x7fffffff, i3 = 0x7fffffff;
+    for (int k = lane; k < a.K; k += 32) {
+        const float x = col[k];
+        if (x > a1) {
+            a3 = a2; i3 = i2;
+            a2 = a1; i2 = i1;
+            a1 = x; i1 = k;
+        } else if (x > a2) {
+            a3 = a2; i3 = i2;
+            a2 = x; i2 = k;
+        } else if (x > a3) {
+            a3 = x; i3 = k;
+        }
+    }
+    float v[3];
+    int kk[3];
+    warp_top3(a1, i1, a2, i2, a3, i3, v, kk);
+    const float v1 = v[0], v2 = v[1], v3 = v[2];
+    const int k1 = kk[0], k2 = kk[1], k3 = kk[2];
+    float ql = 0.0f;
+    for (int k = lane; k < a.K; k += 32) if (k != k1) ql = ffma(a.alpha, col[k], ql);
+    const float qp = warp_ks_scan(ql, lane);
+    const float Q = __shfl_sync(FULL, qp, 31);
+    a.st_ql[(size_t)w * 32 + lane] = ql;
+    if (lane == 0) {
+        a.st_top2[w] = ((uint32_t)k2 << 16) | (uint32_t)k1;
+        a.st_k3[w] = (uint32_t)k3;
+        a.st_phi[w] = make_float4(v1, v2, v3, Q);
+    }
+    __syncwarp();
+}
 
 // Whether a sparse word of nnz topics puts the base values back into a column kept for the next
 // sparse word: up to an eighth of the topics (a sixteenth and a quarter measure the same, in the
@@ -302,7 +330,7 @@ __device__ __forceinline__ void word_stats_word(const StatsArgs& a, int w, float
         for (int k = lane; k < K; k += 32)
             col[k] = fmul(fadd(__int2float_rn(__ldg(row + k)), a.beta), __ldg(a.recip + k));
         __syncwarp();
-        word_stats_from(a, w, ColumnPhi{col}, lane);
+        word_stats_column(a, w, col, lane);
         clean = false;
         return;
     }
@@ -370,44 +398,6 @@ __device__ __forceinline__ void word_stats_word(const StatsArgs& a, int w, float
         if (lane == 0) col[k1] = fmul(a.beta, __ldg(a.recip + k1));
         __syncwarp();
     }
-}
-
-template <class Phi>
-__device__ __forceinline__ int word_stats_from(const StatsArgs& a, int w, const Phi& phi, int lane) {
-    // the lane's top three by (phi desc, k asc) in one pass (k ascends, so a strictly larger
-    // value is needed to displace), then three warp-wide pops of the lanes' heads
-    float a1 = -1.0f, a2 = -1.0f, a3 = -1.0f;
-    int i1 = 0x7fffffff, i2 = 0x7fffffff, i3 = 0x7fffffff;
-    for (int k = lane; k < a.K; k += 32) {
-        const float x = phi(k);
-        if (x > a1) {
-            a3 = a2; i3 = i2;
-            a2 = a1; i2 = i1;
-            a1 = x; i1 = k;
-        } else if (x > a2) {
-            a3 = a2; i3 = i2;
-            a2 = x; i2 = k;
-        } else if (x > a3) {
-            a3 = x; i3 = k;
-        }
-    }
-    float v[3];
-    int kk[3];
-    warp_top3(a1, i1, a2, i2, a3, i3, v, kk);
-    const float v1 = v[0], v2 = v[1], v3 = v[2];
-    const int k1 = kk[0], k2 = kk[1], k3 = kk[2];
-    float ql = 0.0f;
-    for (int k = lane; k < a.K; k += 32) if (k != k1) ql = ffma(a.alpha, phi(k), ql);
-    const float qp = warp_ks_scan(ql, lane);
-    const float Q = __shfl_sync(FULL, qp, 31);
-    a.st_ql[(size_t)w * 32 + lane] = ql;
-    if (lane == 0) {
-        a.st_top2[w] = ((uint32_t)k2 << 16) | (uint32_t)k1;
-        a.st_k3[w] = (uint32_t)k3;
-        a.st_phi[w] = make_float4(v1, v2, v3, Q);
-    }
-    __syncwarp();
-    return k1;
 }
 
 // ---------------------------------------------------------------- DT rebuild
@@ -582,9 +572,8 @@ struct SplitQ {
     const uint32_t* ent;  // the word's row (k << 16 | count), ascending k
     uint32_t nnz;
     float Qw;
-    const float* T;       // the smoothing table (K entries, non-decreasing)
-    const float* r;       // r_k, at col_skew(k) when skew
-    bool skew;
+    const float* T;       // the smoothing table (K entries, ascending but for rounding)
+    const float* r;       // r_k
     // the Qw rounds' table, lane r holding round r's (carry before it, carry + its largest
     // KS prefix); rounds = 0 when not built (more than 32 rounds, or not wanted)
     int rounds = 0;
@@ -594,7 +583,7 @@ struct SplitQ {
     const float* wp = nullptr;
     unsigned wok = 0u;
     const float* tend = nullptr;
-    __device__ __forceinline__ float rk(int k) const { return r[skew ? col_skew(k) : k]; }
+    __device__ __forceinline__ float rk(int k) const { return __ldg(r + k); }
     // round slot i of the Qw search: alpha * (n_wk * r_k), the max topic's term 0
     __device__ __forceinline__ void slot(uint32_t i, int maxK, float alpha, int& key, float& term, bool& ok) const {
         const uint32_t en = __ldg(ent + i);
@@ -683,9 +672,7 @@ enum { C_TOK, C_EA, C_FULL, C_NNZ, C_MAX, C_S, C_Q, C_WNNZ, C_TDENSE, C_TSPARSE,
 // registers; 5 CTAs of 48 spill: 1.96 against 1.92 ms per sweep at K=1024, and 3 leave too
 // few warps, 2.23 ms).  The K > 1024 kernels (several Q rounds per batch) and the LL kernel up
 // to kThreadQTopics (its FP64 products; K=64: 119 -> 109 us per sweep) take 3; above, the LL
-// kernel spills 22 bytes at 4 and is still faster (K=1024: 701 against 755 us).
-// Branch taken by a token (counters only).
-enum { BR_NONE = 0, BR_MAX = 1, BR_S = 2, BR_Q = 3 };
+// kernel spills 44 bytes at 4 and is still faster (K=1024: 701 against 755 us).
 
 #ifndef LDA_SAMPLE_WARPS
 #define LDA_SAMPLE_WARPS 8
@@ -700,9 +687,7 @@ constexpr int kSampleWarps = LDA_SAMPLE_WARPS;
 #ifndef LDA_SAMPLE_LL_MIN_BLOCKS
 #define LDA_SAMPLE_LL_MIN_BLOCKS 4
 #endif
-#ifndef LDA_SAMPLE_LL0_MIN_BLOCKS
-#define LDA_SAMPLE_LL0_MIN_BLOCKS 3
-#endif
+constexpr int kSampleLL0MinBlocks = 3;
 
 // The slots in which a warp keeps doc rows' lane sums: row slot s holds the 32 sums of one
 // row at [33 s, 33 s + 32), so that 32 threads reading element i of 32 different rows touch
@@ -711,6 +696,9 @@ constexpr int kSlotWords = 33;
 // Words of a warp's row slots, even (the rows' list, 32 x {offset, length}, follows them).
 __host__ __device__ __forceinline__ int slot_words(int nslots) { return (kSlotWords * nslots + 1) & ~1; }
 __host__ __device__ __forceinline__ int row_state_words(int nslots) { return slot_words(nslots) + 64; }
+
+// The branch that a token's draw takes: early accepts and tokens without a draw have none.
+enum { BR_NONE = 0, BR_MAX = 1, BR_S = 2, BR_Q = 3 };
 
 // What a group's tokens drew so far: the branch, and for the S bucket the lane and the rest
 // of the target inside it, for the Q bucket the rest of the target.
@@ -722,11 +710,9 @@ struct Draw {
 };
 
 // Fewest tokens that decide_tokens takes thread per token: below, the whole warp decides
-// them one by one (about 45 warp instructions each against 280).
-#ifndef LDA_DECIDE_MIN
-#define LDA_DECIDE_MIN 3
-#endif
-constexpr int kDecideMin = LDA_DECIDE_MIN;
+// them one by one (about 45 warp instructions each against 280; from 7 tokens on instead, 1.96
+// against 1.92 ms per sweep at K=1024).
+constexpr int kDecideMin = 3;
 
 // The tokens (lane = token, those with `act`) whose doc row's lane sums sit in slot my_s of
 // `slots`: S from the row's 32 sums, the branch, and for an S-bucket draw the lane: the
@@ -821,10 +807,7 @@ __device__ __forceinline__ int warp_q_draw(const View& colz, float tt, float QL,
 // Above kLargeK, fewest Q-bucket draws of a group that run thread per token (three quarters
 // of the draws are from Q there while a model is young: K=10,000, 10M tokens 4.40 ms per
 // sweep; from 8 draws on 4.45, none 4.90).
-#ifndef LDA_THREAD_Q_MIN
-#define LDA_THREAD_Q_MIN 4
-#endif
-constexpr int kThreadQMin = LDA_THREAD_Q_MIN;
+constexpr int kThreadQMin = 4;
 
 // The 32-token groups g0, g0 + gstep, ... of the token range [start, start + cnt) of one
 // word (column view colz, max topic maxK, phi4 ph, Q partials QL / QP / Q of the word), or,
@@ -1095,7 +1078,7 @@ __device__ __forceinline__ void sample_tile(const SampleArgs& a, int tile, const
     if (split) {
         // a sparse word above kLargeK topics: the split Q bucket
         if constexpr (QB > 1 && !SKEWKEYS) {
-            const SplitQ sq{ent, nnz, __shfl_sync(FULL, QL, 0), a.smooth, a.recip, false};
+            const SplitQ sq{ent, nnz, __shfl_sync(FULL, QL, 0), a.smooth, a.recip};
             ll = sample_groups<LL, QB, true>(a, start, cnt, 0u, 32u, iter, maxK, ph, QL, QP, Q, View{col}, ctr, lane,
                                              slots, nullptr, 0, &sq);
         }

@@ -42,24 +42,18 @@ constexpr int kTilesPerWarp = LDA_TILES_PER_WARP;
 #define LDA_DENSE_TILE 8192
 #endif
 constexpr int kDenseTileLarge = LDA_DENSE_TILE;  // most tokens per dense-word tile above kLargeK topics (one CTA per tile)
-#ifndef LDA_DENSE_TILE_MIN
-#define LDA_DENSE_TILE_MIN 512
-#endif
-constexpr int kDenseTileLargeMin = LDA_DENSE_TILE_MIN;
-#ifndef LDA_DENSE_TILES_PER_CTA
-#define LDA_DENSE_TILES_PER_CTA 1
-#endif
+// Fewest: 256 are the same at K=4096 and 10,000 (a shorter tile does not pay for its column),
+// 1,024 cost 3% at K=4096 in chunks of 0.5M tokens.
+constexpr int kDenseTileLargeMin = 512;
 constexpr int kLargeWarps = 8;                // warps per CTA of the large-K sparse-word statistics
 // Tokens per dense word-topic tile: the corpus' tokens over half the warps that fill the GPU,
 // within these bounds.  The upper one alone (16,384) left a small corpus' rebuild waiting for
 // the one warp that walks the most frequent word's tile, 128 tokens per round of loads (K=64,
-// 200K tokens 84 -> 27 us); a quarter of that size flushes too often on a large one (48M
-// tokens at K=1024 360 against 180 us).
+// 200K tokens 103 -> 20 us); a quarter of that size flushes too often on a large one (48M
+// tokens at K=1024 360 against 180 us).  The lower one: ten sweeps of 200K tokens at K=64 take
+// 782 us with 4,096, 678 with 2,048, 618 with 1,024.
 constexpr int kWtTileMax = 16384;
-#ifndef LDA_WT_TILE_MIN
-#define LDA_WT_TILE_MIN 2048
-#endif
-constexpr int kWtTileMin = LDA_WT_TILE_MIN;
+constexpr int kWtTileMin = 2048;
 constexpr int kCounters = 16;
 
 struct EventPair {
@@ -371,11 +365,9 @@ static void largest_first(std::vector<int4>& v) {
 // The row slots per warp of a sampler whose CTA takes bytes(slots) of shared memory: as many,
 // up to a group's 32, as leave the CTAs per SM that kMinRowSlots leave (a group whose rows do
 // not fit is taken in parts, each with a whole per-token part); fewer only where the shared
-// memory of one CTA asks for it.
-#ifndef LDA_MIN_ROW_SLOTS
-#define LDA_MIN_ROW_SLOTS 8
-#endif
-constexpr int kMinRowSlots = LDA_MIN_ROW_SLOTS;
+// memory of one CTA asks for it.  With 16 K=10,000 loses a CTA per SM (4.32 against 4.03 ms per
+// sweep of 10M tokens); 4 measure the same there and at K=64 to 1500.
+constexpr int kMinRowSlots = 8;
 template <class Bytes>
 static int pick_slots(const void* fn, int threads, int max_smem, const Bytes& bytes, int* slots, size_t* smem) {
     int least = kMinRowSlots;
@@ -435,10 +427,12 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
     T.budget = cfg->device_budget;
     T.chunk_tok = c->chunk_tok;
     T.chunk_doc = c->chunk_doc;
-    // warps per CTA: (warps + 1) K-wide shared rows must fit
+    // Warps per CTA of the K <= kLargeK statistics, and the limit on K: twice K floats must fit
+    // in a CTA's shared memory (28,736 topics).  The kernels above kLargeK need less, 1.6 K floats
+    // for the count rebuilds; the limit on K is kept.
     const int64_t row = (int64_t)T.K * 4;
     T.warps = (int)std::min<int64_t>(8, ((int64_t)max_smem - 2048) / (row + 256) - 1);
-    if (T.warps < 1) return fail(LDA_ERR_ARG, "K=%d needs %lld bytes of shared memory per warp (max %d)", T.K, (long long)(2 * row), max_smem);
+    if (T.warps < 1) return fail(LDA_ERR_ARG, "K=%d is above the limit of %lld topics", T.K, (long long)(((int64_t)max_smem - 2048) / 2 - 256) / 4);
     T.large = T.K > dev::kLargeK;
     int orc;
     if (!T.large) {
@@ -530,7 +524,7 @@ extern "C" int lda_trainer_create(const lda_corpus* c, const lda_train_config* c
             // K=10,000: 4.54 ms per sweep; half of that size 4.64, a quarter 4.79).
             int64_t nd = 0;
             for (int64_t w = 0; w < T.Vd; ++w) nd += c->seg_cnt[(size_t)ch * V + w];
-            const int64_t per = LDA_DENSE_TILES_PER_CTA * std::max<int64_t>(resident_dense, 1);
+            const int64_t per = std::max<int64_t>(resident_dense, 1);
             // sparse-word tiles: as the tiles up to kLargeK topics (a small vocabulary's sparse
             // words are long, and one warp takes a tile: 3.5M tokens of 7,000 words at K=3000
             // 7.6 -> 1.6 ms per sweep, 2M of 3,000 at K=2049 6.2 -> 0.95; 10M at K=10,000 4.26 ->
