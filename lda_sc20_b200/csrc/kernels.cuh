@@ -807,7 +807,7 @@ constexpr int kDenseWarps = 8, kSparseWarps = 12;
 template <bool LL, int QB>
 __global__ void __launch_bounds__(32 * kSparseWarps, LDA_SPARSE_LARGE_MIN_BLOCKS) k_sample_sparse_large(SampleArgs a) {
     extern __shared__ float smf[];
-    const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int bw = large_bit_words(a.K), pw = large_pre_words(a.K);
     float* base = smf;
     float* tend = smf + col_words(a.K);
