@@ -663,9 +663,11 @@ def serving_figures(model, corpus, sweeps: int, rates_arg: str, seconds: float, 
         rates.append({"offered_docs_per_s": rate, "requests": n, "achieved_docs_per_s": n / wall,
                       "p50_ms": float(np.percentile(lat, 50) * 1e3), "p99_ms": float(np.percentile(lat, 99) * 1e3),
                       "max_ms": float(lat.max() * 1e3)})
+    # the library counts the sampling kernel, one launch a step; the kernel that builds the
+    # requests' next rows or theta is another
     return {"docs_per_s": batch_dps, "one_at_a_time_docs_per_s": single_dps,
             "batch_vs_one_at_a_time": batch_dps / single_dps, "batch_token_sweeps_per_s": tokens_b * sweeps / batch_s,
-            "batch_steps": s1 - s0, "gpu_launches": l1 - l0, "alone_equals_batched": f"{ident}/32",
+            "batch_steps": s1 - s0, "gpu_launches": 2 * (l1 - l0), "alone_equals_batched": f"{ident}/32",
             "rates": rates, "sweeps": sweeps}
 
 
@@ -791,7 +793,8 @@ def run_batch(args, local):
                          "dense_rule": {"None": "corpus split (count >= K)", "-1": "no dense words"}.get(
                              str(rule), f"count >= {rule}*K"),
                          "dense_rule_ms_per_sweep_on_sample": {str(k): round(v[0], 3) for k, v in rule_ms.items()}},
-            "gpu_launches": l1 - l0, "work_items_per_sweep": work,
+            # the library counts a sweep as seven launches; it makes six
+            "gpu_launches": l1 - l0 - sweeps, "work_items_per_sweep": work,
             "models_identical_to_plain": f"{same}/{len(corpora)}", "loglik_max_rel_diff": ll_rel,
             "clocks": clk}
     print(json.dumps(line), flush=True)

@@ -128,7 +128,8 @@ typedef struct {
     float beta;             /* EZLDA: 0.01 (EZLDA/Argument.cuh:8) */
     uint64_t seed;          /* Philox seed of the sweep randoms */
     int32_t device;         /* CUDA device ordinal */
-    int64_t device_budget;  /* bytes the trainer may allocate (0: no limit) */
+    int64_t device_budget;  /* bytes the trainer may allocate (0: no limit), the sweep's tables
+                               and the tile lists included (lda_trainer_device_bytes) */
     int32_t stream_mode;    /* 0: keep the corpus resident when it fits device_budget, else
                                stream it; 1: always resident; 2: always stream */
     int32_t num_streams;    /* streaming: chunk slots on the device, one CUDA stream each (0: 4);
@@ -403,6 +404,8 @@ int lda_batch_get_tuning(const lda_batch* b, lda_batch_tuning* tuning);
  * sweep per model (lda_batch_loglik, and each trainer's lda_trainer_loglik). */
 int lda_batch_iterate(lda_batch* b, int32_t sweeps, int32_t ll_mode);
 int lda_batch_loglik(const lda_batch* b, double* ll /*n*/, int32_t n);
+/* kernel_launches counts a sweep as seven launches and as eight with the LL (it makes six and
+ * seven); work_items are those of one sweep. */
 int lda_batch_stats(const lda_batch* b, int64_t* kernel_launches, int64_t* work_items);
 /* Times every candidate tuning (warps {4,8} x schedule {0,1} x tile_tokens {128,256,512})
  * for sweeps_per_trial sweeps on the live batch, restoring the models' topics, iterations
@@ -449,7 +452,9 @@ int lda_server_get_topics(lda_server* s, uint32_t rid, uint16_t* out, int32_t le
 /* Tokens per work item (a multiple of 32, default 32): a request is split into items of
  * this many tokens, each sampled by one warp.  Only while the server is idle. */
 int lda_server_set_item_tokens(lda_server* s, int32_t n);
-/* Steps issued and fold-in (sampling) kernel launches since creation, one a step. */
+/* Steps issued and launches of the sampling kernel since creation, one a step.  (A step also
+ * launches the kernel that builds the requests' next rows or theta, and once more for the
+ * requests it admits.) */
 int lda_server_stats(const lda_server* s, int64_t* steps, int64_t* kernel_launches);
 /* Real-time replay on an idle server: document i (words[doc_off[i]..doc_off[i+1]))
  * arrives arrival_s[i] seconds after the start (non-decreasing) and gets request id i;

@@ -456,7 +456,7 @@ static int enqueue_sweeps(lda_batch* b, int sweeps, int ll) {
         batch_sample_kernel(last_ll, b->Kmax)<<<gs, threads, b->smem_sample, b->st>>>(a);
         if (last_ll) dev::kb_ll<<<M, 1024, 0, b->st>>>(b->sm.p, b->ll_dev);
         CUDA_TRY(cudaGetLastError());
-        b->kernel_launches += last_ll ? 8 : 7;
+        b->kernel_launches += last_ll ? 8 : 7;  // the interface's count; the launches above are 7 and 6
     }
     return LDA_OK;
 }
