@@ -969,7 +969,16 @@ static int launch_recip(lda_trainer* t, float* recip) {
 // that was rewritten since they were formed.
 static int sample_totals(lda_trainer* t) {
     if (!t->totals_new) return LDA_OK;
-    if (t->large && !t->recip_cur) CUDA_TRY(cudaMalloc(&t->recip_cur, sizeof(float) * (size_t)t->K));
+    if (t->large && !t->recip_cur) {
+        // outside the budget: a call that fitted without the table is not refused for it
+        const size_t n = sizeof(float) * (size_t)t->K;
+        const cudaError_t e = cudaMalloc(&t->recip_cur, n);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return fail(LDA_ERR_DEVICE_MEM, "cudaMalloc of %zu bytes failed: %s", n, cudaGetErrorString(e));
+        }
+        t->bytes += (int64_t)n;
+    }
     int rc = launch_recip(t, t->large ? t->recip_cur : t->recip);
     if (rc) return rc;
     t->totals_new = false;
