@@ -530,10 +530,9 @@ struct SampleArgs {
     unsigned* tile_counter;
     double* tile_ll;
     int K, Vd, ll_mode;
-    float alpha, beta, Vbeta;
+    float alpha, beta;
     double den_add;  // (double)K * (double)alpha
     uint32_t seed_lo, seed_hi, iter;
-    const int* n_k;
     const int* dwt;
     const uint32_t* swt_off;
     const uint32_t* swt_nnz;

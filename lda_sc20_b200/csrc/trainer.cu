@@ -1116,10 +1116,10 @@ static dev::SampleArgs sample_args(const lda_trainer* t, int chunk, int slot, in
     dev::SampleArgs a;
     a.tiles = t->s_tiles + base; a.ntiles = n; a.tile_counter = t->tile_ctr + 1 + chunk; a.tile_ll = t->tile_ll + base;
     a.K = t->K; a.Vd = t->Vd; a.ll_mode = ll_mode ? 1 : 0;
-    a.alpha = t->alpha; a.beta = t->beta; a.Vbeta = t->Vbeta;
+    a.alpha = t->alpha; a.beta = t->beta;
     a.den_add = (double)t->K * (double)t->alpha;
     a.seed_lo = (uint32_t)t->seed; a.seed_hi = (uint32_t)(t->seed >> 32); a.iter = t->iter;
-    a.n_k = t->n_k; a.dwt = t->dwt; a.swt_off = t->swt_off; a.swt_nnz = t->swt_nnz; a.swt_ent = t->swt_ent;
+    a.dwt = t->dwt; a.swt_off = t->swt_off; a.swt_nnz = t->swt_nnz; a.swt_ent = t->swt_ent;
     a.st_top2 = t->st_top2; a.st_phi = t->st_phi; a.st_ql = t->st_ql;
     a.tok_doc = b.tok_doc; a.meta = b.meta; a.z = t->z; a.doc_len = t->doc_len;
     a.dt_off = t->dt_off; a.dt_nnz = t->dt_nnz; a.dt_ent = b.dt_ent; a.ctr = t->ctr;
@@ -2090,10 +2090,11 @@ extern "C" int lda_sample_chunk_noalloc(const lda_sample_io* io, int32_t device,
     a.tile_counter = reinterpret_cast<unsigned*>(scratch);
     a.tile_ll = reinterpret_cast<double*>(scratch + kNoAllocHeader);
     a.K = io->K; a.Vd = io->num_dense; a.ll_mode = io->ll_mode ? 1 : 0;
-    a.alpha = io->alpha; a.beta = io->beta; a.Vbeta = (float)io->vocab * io->beta;
+    const float Vbeta = (float)io->vocab * io->beta;
+    a.alpha = io->alpha; a.beta = io->beta;
     a.den_add = (double)io->K * (double)io->alpha;
     a.seed_lo = (uint32_t)io->seed; a.seed_hi = (uint32_t)(io->seed >> 32); a.iter = io->iter;
-    a.n_k = io->n_k; a.dwt = io->dense_wt;
+    a.dwt = io->dense_wt;
     a.swt_off = io->sparse_off; a.swt_nnz = io->sparse_nnz; a.swt_ent = io->sparse_ent;
     a.st_top2 = io->top2; a.st_phi = reinterpret_cast<const float4*>(io->phi4); a.st_ql = io->ql;
     a.tok_doc = io->tok_doc; a.meta = io->meta; a.z = io->topics; a.doc_len = io->doc_len;
@@ -2104,7 +2105,7 @@ extern "C" int lda_sample_chunk_noalloc(const lda_sample_io* io, int32_t device,
     a.nslots = sh.nslots;
     if (io->K > dev::kLargeK) {
         a.smooth = reinterpret_cast<const float*>(scratch + kNoAllocSmooth);
-        dev::k_smooth_table<<<1, 1024, 0, st>>>(io->n_k, io->K, a.Vbeta, io->alpha, io->beta,
+        dev::k_smooth_table<<<1, 1024, 0, st>>>(io->n_k, io->K, Vbeta, io->alpha, io->beta,
                                               reinterpret_cast<float*>(scratch + kNoAllocSmooth));
         CUDA_TRY(cudaGetLastError());
     }
@@ -2114,7 +2115,7 @@ extern "C" int lda_sample_chunk_noalloc(const lda_sample_io* io, int32_t device,
     chk.swt_ent = io->sparse_ent; chk.tok_doc = io->tok_doc; chk.dt_off = io->dt_off; chk.dt_nnz = io->dt_nnz;
     chk.dt_ent = io->dt_ent; chk.N = io->num_tokens; chk.n_dt = io->num_dt_entries;
     chk.n_sp = io->num_sparse_entries; chk.status = io->status; chk.tile_counter = a.tile_counter;
-    chk.n_k = io->n_k; chk.Vbeta = a.Vbeta; chk.recip = reinterpret_cast<float*>(scratch + kNoAllocRecip);
+    chk.n_k = io->n_k; chk.Vbeta = Vbeta; chk.recip = reinterpret_cast<float*>(scratch + kNoAllocRecip);
     a.recip = chk.recip;
     k_check_sample_io<<<4 * sh.num_sms, 256, 0, st>>>(chk);
     CUDA_TRY(cudaGetLastError());
